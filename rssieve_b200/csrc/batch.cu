@@ -12,12 +12,11 @@
 //   k_mr_batch_sprp, k_mr_batch_lucas  Baillie-PSW over the survivors of every
 //                    range at once (base 2, then Lucas over the passers)
 //   k_setup_*<true>  per-prime set-up over the primes of every range at once
-//   k_batch_group_prefix  every (geometry, product) group's prefix sums of its
-//                    ranges' prime counts, in one launch
-//   per group, on its own branch (fork/join through events): one persistent
-//   k_bsgs<..., true> over all primes of the group's ranges (each prime carries
-//   its job index and loads that job's arguments); the branches overlap, so one
-//   group's last wave does not idle the device
+//   per group (CTA size x step kind), on its own branch (fork/join through
+//   events): one persistent k_bsgs<..., true> over the group's primes, which the
+//   set-up has put on lists by class (each prime carries its job index and loads
+//   that job's arguments); the branches overlap, so one group's last wave does
+//   not idle the device
 //   k_batch_account  primes tested per range, unfinished-range count
 //
 // so the host only waits once per round, to read the error word and whether
@@ -35,8 +34,8 @@
 // between rounds -- their tables are written to device memory that the
 // captured round reads -- and a finished job's slots are released for the
 // next one, so the batch also serves a stream of arriving work units.  The
-// ten BSGS groups (geometry x product) cover every range slot and count only
-// the slots currently in them, so the captured round never changes.  A job's
+// six BSGS groups take whatever the set-up put on their lists, so the captured
+// round never changes.  A job's
 // bitmap and factor list come from the batch's own stream-ordered memory pool,
 // which keeps freed blocks mapped and can be grown ahead of time
 // (rs_batch_reserve): admitting or releasing a job neither
@@ -67,8 +66,6 @@ struct BJob {
     std::vector<u32> ranges;
 };
 
-constexpr int NGROUP = 3 * NGEOM;  // BSGS groups: g = 3*geometry + step kind (2 FP64, 1 Shoup, 0 Montgomery)
-
 __global__ void k_batch_account(const BatchRange *ranges, const u32 *ctrs, u32 rcap, u32 nranges, u64 *range_primes,
                                 u64 *stats, u32 *unfinished)
 {
@@ -98,8 +95,7 @@ struct rs_batch {
     u32 *d_win = nullptr;
     u32 *d_prefix_c = nullptr, *d_prefix_p = nullptr;   // prefix sums over all ranges: survivors, primes
     u32 *h_win_pin = nullptr;
-    u32 *d_gprefix = nullptr;              // NGROUP x (nranges + 1) prefix sums of the groups' prime counts
-    u32 *d_gwork = nullptr;                // NGROUP work counters of the groups' BSGS launches
+    BsgsLists lists = {nullptr, 0, nullptr};   // the round's records by group and class
     cudaStream_t side[NGROUP] = {};        // one branch per group: the groups' launches overlap
     cudaEvent_t fork = nullptr, join[NGROUP] = {};
     // device tables
@@ -164,7 +160,7 @@ extern "C" void rs_batch_destroy(rs_batch *b)
     void *ptrs[] = {b->d_sp, b->d_jobs, b->d_geoms, b->d_args, b->d_fctrs, b->d_ranges, b->d_wins, b->d_ctrs,
                     b->d_range_primes, b->d_cands, b->d_primes, b->d_hdr, b->d_aux, b->d_tabs, b->d_tgt, b->d_meta,
                     b->d_err, b->d_stats, b->d_unfinished, b->d_win, b->d_prefix_c, b->d_prefix_p,
-                    b->d_gprefix, b->d_gwork, b->d_mid, b->d_mid_r, b->d_mid_ctr, b->d_rec_of};
+                    b->lists.list, b->lists.ctl, b->d_mid, b->d_mid_r, b->d_mid_ctr, b->d_rec_of};
     for (void *p : ptrs) cudaFree(p);
     if (b->h_pin) cudaFreeHost(b->h_pin);
     if (b->h_win_pin) cudaFreeHost(b->h_win_pin);
@@ -255,8 +251,10 @@ extern "C" int rs_batch_create(int device, uint32_t max_jobs, uint32_t range_slo
         if (cudaMemPoolSetAttribute(b->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
             return fail(RS_ECUDA);
     }
-    if (!alloc((void **)&b->d_gprefix, (size_t)NGROUP * (R + 1) * 4) || !alloc((void **)&b->d_gwork, NGROUP * 4)) {
-        rs_set_error("cannot allocate the BSGS group tables");
+    b->lists.stride = R * RCAP;
+    if (!alloc((void **)&b->lists.list, (size_t)NGROUP * NCLASS * R * RCAP * 4) ||
+        !alloc((void **)&b->lists.ctl, (size_t)NGROUP * 2 * NCLASS * 4)) {
+        rs_set_error("cannot allocate the BSGS group lists");
         return fail(RS_ENOMEM);
     }
     if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess) return fail(RS_ECUDA);
@@ -493,23 +491,23 @@ static int batch_round(rs_batch *b)
     BCU(launch_mr_batch2(b->d_cands, CCAP, b->d_primes, RCAP, b->d_ctrs, R, b->d_prefix_c, b->d_mid, b->d_mid_r,
                          R * CCAP, b->d_mid_ctr, b->d_err, b->sms, st));
     BCU(launch_batch_prefix_all(b->d_ranges, R, 1, RCAP, b->d_ctrs, b->d_prefix_p, st));
+    BCU(cudaMemsetAsync(b->lists.ctl, 0, (size_t)NGROUP * 2 * NCLASS * 4, st));
     BCU(launch_setup_batch(b->d_jobs, b->d_geoms, b->d_ranges, b->d_primes, RCAP, b->d_prefix_p, R, b->d_hdr,
-                           b->d_aux, b->d_tabs, b->d_tgt, b->d_meta, b->d_stats, b->d_err, b->d_rec_of, b->sms,
-                           st));
+                           b->d_aux, b->d_tabs, b->d_tgt, b->d_meta, b->lists, b->d_stats, b->d_err, b->d_rec_of,
+                           b->sms, st));
     BsgsArgs a;
     memset(&a, 0, sizeof a);
     a.stats = b->d_stats;
     a.err = b->d_err;
-    // the groups' prefix sums in one launch, then one persistent BSGS launch per
-    // group on its own branch (fork/join through events, so a captured round is
-    // a graph with parallel branches): one group's last wave overlaps the others
-    BCU(launch_batch_group_prefix(b->d_ranges, R, b->d_ctrs, RCAP, b->d_gprefix, b->d_gwork, st));
+    // one persistent BSGS launch per group on its own branch (fork/join through
+    // events, so a captured round is a graph with parallel branches): one
+    // group's last wave overlaps the others
     BCU(cudaEventRecord(b->fork, st));
     for (int g = 0; g < NGROUP; ++g) {
         BCU(cudaStreamWaitEvent(b->side[g], b->fork, 0));
-        BCU(launch_bsgs_batch(a, b->d_args, b->d_hdr, b->d_tabs, b->d_tgt, b->d_meta, R,
-                              b->d_gprefix + (size_t)g * (R + 1), RCAP, b->d_gwork + g, g % 3, g / 3, b->sms,
-                              b->side[g]));
+        const BsgsLists L = {b->lists.list + (size_t)g * NCLASS * b->lists.stride, b->lists.stride,
+                             b->lists.ctl + g * 2 * NCLASS};
+        BCU(launch_bsgs_batch(a, b->d_args, b->d_hdr, b->d_tabs, b->d_tgt, b->d_meta, L, g, b->sms, b->side[g]));
         BCU(cudaEventRecord(b->join[g], b->side[g]));
         BCU(cudaStreamWaitEvent(st, b->join[g], 0));
     }

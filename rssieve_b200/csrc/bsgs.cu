@@ -1,37 +1,51 @@
-// bsgs.cu -- baby-step giant-step search, one prime per CTA at a time.
+// bsgs.cu -- baby-step giant-step search, a group of 32 to 1024 threads per prime.
 //
 // Replaces the reference's giantfull/giantparity kernels (kernels/giant.cl:77-323).
-// For one prime p with per-prime record (see setup.cu):
-//   baby phase   y_j = s^j for j in [0,Q'), Q' = TPB*cp with cp = C, C/2 or
-//                C/4 chosen per prime by the set-up: thread t computes
-//                y_{t*cp..t*cp+cp-1} from its start A[t%32]*B[t/32] with cheap
-//                steps (doublings when b^e is 2 or 4, else one modular
-//                product), checks y_j == 1 to detect ord(s) < Q'
-//                (giant.cl:123-134), then inserts j < ord into a shared-memory
-//                hash table.
-//   giant phase  gamma = T_i * S^q for q in [0,Mg): thread (i,g) walks q in
-//                [g*Lc, (g+1)*Lc) from T_i * S^(g*Lc) as two interleaved
-//                chains, one modular product (Shoup's for p < 2^63, else
-//                Montgomery) and one table probe per step (giant.cl:170-192).  A match
-//                s^j == gamma gives n = nmin + off_i + e*((q+1)*Q' - 1 - j),
-//                where s = b^e and off_i is target i's class of n mod e
-//                (setup.cu; e = 2 is the reference's parity split).
-//   small order  ord(s) < Q': each target is looked up once and every n in
+// For one prime p with per-prime record (see setup.cu), searched by a group of
+// GS = 32 << c threads (class c, chosen per prime by the set-up):
+//   baby phase   y_j = s^j for j in [0,Q'), Q' = 16*GS: thread t forms
+//                y_{16t..16t+15} from its start A[t%32]*B[t/32] as two chains
+//                (doublings when b^e is 2 or 4, else one modular product per
+//                step) and enters each into the group's filter.  y_j = 1 for
+//                some 0 < j <= Q' detects ord(s) <= Q' (giant.cl:123-134).
+//   giant phase  gamma = T_i * S^q for q in [0,Mg): item (i,g) walks q in
+//                [g*Lc, (g+1)*Lc) from T_i * S^(g*Lc); a thread runs two items
+//                at a time, one modular product and one filter probe per step
+//                (giant.cl:170-192).  s^j == gamma gives n = nmin + off_i +
+//                e*((q+1)*Q' - 1 - j), where s = b^e and off_i is target i's
+//                class of n mod e (setup.cu; e = 2 is the reference's parity
+//                split).
+//   small order  ord(s) <= Q': each target is looked up once and every n in
 //                range with the same residue mod e*ord is claimed (giant.cl:146-168).
 //   claims       atomicAnd on the term's bitmap bit; the first claimer appends
 //                {p, n, seq} to the factor buffer (giant.cl:21-39,158-162).
 //
-// Hash table: NB buckets in shared memory.  Bucket b is 16 bytes of
-// fingerprints -- seven 16-bit slots and an eighth halfword that is 0x8000
-// when the bucket overflowed, i.e. later values continued into the next bucket
-// (linear probing) -- plus seven 16-bit baby indices j in a separate array and
-// a 16-bit fill count in a third (two per word, so that the counts' atomics
-// spread over all shared-memory banks).  Every halfword has one writer or
-// writers of one value, so all table writes are plain 16-bit stores.
-// A fingerprint match is verified exactly by recomputing y_j from its
-// thread's start value, so the search is exact for every 64-bit value (the
-// reference's split lo32/hi32 table cannot find values whose low 32 bits are
-// zero, giant.cl:46,63).
+// The filter holds the baby values as a blocked Bloom filter in shared memory:
+// 48 words per thread, i.e. three words per baby value; a value sets three bits
+// of one word (one atomicOr without a result) and a probe tests them (one
+// 4-byte load).  It never misses a value; about one probe in 2000 passes for a
+// value that is not there.  Passing probes go on a queue and are checked exactly
+// once the giant steps are done, 16 lanes each: with anchors x_t = s^(16t), t =
+// 0..GS, in an index that then takes the filter's place, gamma = s^j for some j = 16t -
+// l, 0 <= l < 16, exactly when gamma * s^l is an anchor, so lane l forms gamma *
+// s^l and looks it up.  The search is exact for every 64-bit value (the reference's split lo32/hi32
+// table cannot find values whose low 32 bits are zero, giant.cl:46,63).
+//
+// What bounds it: issue.  A random 4-byte shared-memory access of a warp, load or
+// atomic, takes 3.55 cycles of the SM's shared-memory pipe, a 16-byte one 10.2,
+// and the ALU and FP64 pipes take two cycles per warp instruction (measured).
+// A step is about 8 FP64, 8 ALU and 3 IMAD instructions and one such access,
+// 14 to 16 cycles of an SM quarter on each of these resources, and its 22 issue
+// slots come first.  100 sequences, n-range 6*10^6, p near 2^50: 18.3 ns per
+// prime (28.1 with an exact table of 16-byte buckets of fingerprints, whose
+// probes and three-store inserts took 5600 shared-memory cycles per prime
+// against 2200 now, and with one group size for all primes of a job); p near
+// 2^58, 61 sequences: 20.5 (26.8); 68 sequences over an n-range of 10^5: 2.4
+// (4.0).  Three bits per value and three words per value: with two bits a pass
+// comes four times as often and costs more than the third bit's two
+// instructions; the filter fills what two CTAs of 512 threads have of shared
+// memory.  A group of Q'/16 threads per prime instead of the whole CTA keeps 16
+// baby and about as many giant steps per thread whatever the prime's work.
 #include "mont.cuh"
 #include "rs_internal.h"
 
@@ -40,76 +54,16 @@
 namespace rs {
 
 constexpr u32 HMUL = 0x9E3779B1u;
+constexpr u32 FILTER_WPT = 48;         // filter words per thread of the group
 
-// Table hash of a 64-bit residue: h = (lo32 ^ hi32) * 0x9E3779B1.  The bucket
-// is floor(h * NB / 2^32), i.e. the top bits of h; the fingerprint comes from
-// the low 16 bits of h with bit 14 cleared and bit 10 set, which makes it the
-// bit pattern of a normal (finite, nonzero) fp16 number.  Both words of the
-// residue are folded in because the baby chain for small bases is a run of
-// doublings whose low bits alone repeat shifted patterns.
-template <u32 NB>
-__device__ __forceinline__ void tab_hash(u64 val, u32 &bucket, u32 &fp)
+// Hash of a residue's 64 bits: word of an nw-word filter (top bits of h) and
+// the three bits it sets there (from the low bits of h; they may coincide).
+// Both halves are folded in because the baby chain for small bases is a run of
+// doublings that repeat shifted patterns (as doubles: one mantissa).
+__device__ __forceinline__ u32 val_hash(u64 v) { return ((u32)v ^ (u32)(v >> 32)) * HMUL; }
+__device__ __forceinline__ u32 filter_mask(u32 h)
 {
-    const u32 h = ((u32)val ^ (u32)(val >> 32)) * HMUL;
-    bucket = __umulhi(h, NB);
-    fp = (h & 0xBFFFu) | 0x0400u;
-}
-
-// Lane-wise fp16 equality of two packed pairs: 0xFFFF per equal half.  For
-// normal fp16 patterns equality of values is equality of bits, and an empty
-// slot (+0) never equals a fingerprint, so this is an exact 16-bit compare
-// that covers two slots per instruction.
-__device__ __forceinline__ u32 heq2(u32 a, u32 b)
-{
-    u32 d;
-    asm("set.eq.u32.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-
-struct Table {
-    uint4 *fpb;                // NB buckets of fingerprints + overflow flag
-    unsigned short *jt;        // j of slot k of bucket b at jt[8*b + k]
-    u32 *cnt;                  // fill count of bucket b in half (b & 1) of cnt[b >> 1]
-};
-
-constexpr u32 OVF_FLAG = 0x80000000u;   // bit 31 of a bucket's last word: halfword 7 = 0x8000
-
-// Slot claim in bucket b: the count's atomicAdd hands out the slot.
-__device__ __forceinline__ u32 tab_claim(const Table &T, u32 b)
-{
-    const u32 sh = (b & 1u) << 4;
-    return (atomicAdd(&T.cnt[b >> 1], 1u << sh) >> sh) & 0xFFFFu;
-}
-
-// Fills slot `slot` of bucket b, or flags b as overflowed when slot > 6.
-// Returns whether the value was placed.
-__device__ __forceinline__ bool tab_fill(const Table &T, u32 b, u32 slot, u32 fp, u32 j)
-{
-    unsigned short *h = reinterpret_cast<unsigned short *>(&T.fpb[b]);
-    if (slot < 7) {
-        h[slot] = (unsigned short)fp;
-        T.jt[8 * b + slot] = (unsigned short)j;
-        return true;
-    }
-    h[7] = 0x8000u;
-    return false;
-}
-
-// One insertion attempt into bucket b; on a full bucket, b advances and false
-// is returned.
-template <u32 NB>
-__device__ __forceinline__ bool tab_try(const Table &T, u32 &b, u32 fp, u32 j)
-{
-    if (tab_fill(T, b, tab_claim(T, b), fp, j)) return true;
-    b = (b + 1 == NB) ? 0u : b + 1;
-    return false;
-}
-
-// halfword k (0..6) of a bucket
-__device__ __forceinline__ u32 slot_fp(const uint4 &bv, int k)
-{
-    const u32 w = (k < 2) ? bv.x : (k < 4) ? bv.y : (k < 6) ? bv.z : bv.w;
-    return (k & 1) ? (w >> 16) : (w & 0xFFFFu);
+    return (1u << (h & 31)) | (1u << ((h >> 5) & 31)) | (1u << ((h >> 10) & 31));
 }
 
 // y -> y*s: doubling/quadrupling for b = 2 (the common case), additions for
@@ -121,14 +75,47 @@ __device__ __forceinline__ u64 dbl63(u64 x, u64 p)
     return (x >= p) ? x - p : x;
 }
 
-__device__ __forceinline__ u64 baby_step(u64 x, u32 smul, u64 s, u64 p, u64 q)
-{
-    if (smul == 2) return madd(x, x, p);
-    if (smul == 4) { x = madd(x, x, p); return madd(x, x, p); }
-    return smul ? mul_small(x, smul, p) : mmul(x, s, p, q);
-}
+// ---- arithmetic by step kind (MODE) ----
+// V: a residue as the chains hold it; Fix: a fixed multiplier.  MODE 2 (p below
+// FP_BOUND = 2^51): plain residues, exact in doubles.  MODE 1 (p < 2^63):
+// Montgomery form, products by a fixed multiplier by Shoup's method.  MODE 0:
+// Montgomery throughout.
+template <int MODE>
+struct Ring {
+    typedef u64 V;
+    u64 p, q;
+    struct Fix { u64 w, wq; };
+    __device__ __forceinline__ explicit Ring(const PrimeHdr &h) : p(h.p), q(h.q) {}
+    static __device__ __forceinline__ V val(u64 b) { return b; }
+    static __device__ __forceinline__ u64 bits(V v) { return v; }
+    static __device__ __forceinline__ V one(const PrimeHdr &h) { return h.one; }
+    static __device__ __forceinline__ Fix baby(const PrimeHdr &h) { return MODE == 1 ? Fix{h.sp, h.sw} : Fix{h.s, 0}; }
+    static __device__ __forceinline__ Fix giant(const PrimeHdr &h) { return MODE == 1 ? Fix{h.Sp, h.Sw} : Fix{h.S, 0}; }
+    __device__ __forceinline__ V mul(V a, V b) const { return mmul(a, b, p, q); }
+    __device__ __forceinline__ V step(V x, const Fix &f) const
+    {
+        return MODE == 1 ? shoup_mul(x, f.w, f.wq, p) : mmul(x, f.w, p, q);
+    }
+    __device__ __forceinline__ V dbl(V x) const { return MODE == 1 ? dbl63(x, p) : madd(x, x, p); }
+};
+template <>
+struct Ring<2> {
+    typedef double V;
+    double p, pinv;
+    struct Fix { double w, wq; };
+    __device__ __forceinline__ explicit Ring(const PrimeHdr &h)
+        : p(fp_exact(h.p)), pinv(bits_double(h.q)) {}
+    static __device__ __forceinline__ V val(u64 b) { return bits_double(b); }
+    static __device__ __forceinline__ u64 bits(V v) { return double_bits(v); }
+    static __device__ __forceinline__ V one(const PrimeHdr &) { return 1.0; }
+    static __device__ __forceinline__ Fix baby(const PrimeHdr &h) { return Fix{val(h.s), val(h.sw)}; }
+    static __device__ __forceinline__ Fix giant(const PrimeHdr &h) { return Fix{val(h.S), val(h.Sw)}; }
+    __device__ __forceinline__ V mul(V a, V b) const { return fp_mul(a, b, p, pinv); }
+    __device__ __forceinline__ V step(V x, const Fix &f) const { return fp_mulfix(x, f.w, f.wq, p); }
+    __device__ __forceinline__ V dbl(V x) const { return fp_dbl(x, p); }
+};
 
-// ---- TMA 1D bulk copies and mbarriers (record prefetch) ----
+// ---- TMA 1D bulk copies and mbarriers (record header prefetch) ----
 __device__ __forceinline__ u32 smem_u32(const void *p) { return (u32)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(u64 *bar, u32 count)
@@ -150,6 +137,11 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, u32 bytes,
                  : "memory");
 }
 
+__device__ __forceinline__ void l2_prefetch(const void *src, u32 bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(u64 *bar, u32 parity)
 {
     u32 ok;
@@ -163,65 +155,57 @@ __device__ __forceinline__ bool mbar_try_wait(u64 *bar, u32 parity)
     return ok != 0;
 }
 
-// One prime's record as the setup kernels lay it out, staged in shared memory.
-struct RecBuf {
-    PrimeHdr hdr;
-    u64 tabs[TABS];                 // A[32] B[32] Z1[32] Z2[32]
-    u64 tgt[KSTRIDE];
-    unsigned short meta[KSTRIDE];   // sequence | offset << 7
-};
-static_assert(sizeof(RecBuf) % 16 == 0, "bulk copies move 16-byte units");
+// Barrier of group gid of the CTA: a warp by itself, else a named barrier over
+// its gs threads (1 to 15; barrier 0 is the whole CTA's, so groups of 64 need a
+// CTA of at most 960 threads).
+__device__ __forceinline__ void group_sync(u32 gid, u32 gs)
+{
+    if (gs == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(gid + 1), "r"(gs) : "memory");
+}
 
 constexpr u32 WAIT_BOUND = 1u << 24;   // default try_wait rounds before a copy is declared lost
+constexpr u32 NONE = 0xFFFFFFFFu;
 
-// ---- per-CTA state in shared memory, read by the out-of-line rare paths ----
-// The hot loops stay small (and in the instruction cache) because matches,
-// overflowed buckets, small orders and claims run in __noinline__ functions
-// that take a few scalars and find everything else here.
-struct PrimeCtx {
-    u64 p, q, s;         // the prime, p^-1 mod 2^64, Montgomery b^e
-    u32 smul, e;         // baby-step multiplier when additions suffice; split modulus
-    u32 cp, qp;          // baby steps per thread and per prime (qp = TPB * cp)
-    u32 fp;              // FP64 steps (MODE 2): table and giant values are the bits of doubles
+// ---- a group's slice of the CTA's dynamic shared memory ----
+// Slice | anchors start[GS + 1] (+1 pad) | filter words | queue of GS/4 filter
+// passes.  The index of the anchors takes the filter's place once the giant
+// steps are done.
+// The rare paths are __noinline__ functions that take the slice and a few
+// scalars, so the hot loops stay small.
+struct Slice {
+    PrimeHdr hdr[2];             // this prime's header and the next one's
+    u32 idx[2];                  // their record indices (NONE: no more primes)
+    u32 claim;                   // the prime after them, claimed ahead
+    u32 order;                   // ord(s) when it is at most Q', else NONE
+    u32 abort;                   // a record wait gave up
+    u32 nq;                      // filter passes put on the queue
+    u32 pad_[2];
+    u64 pw[16];                  // s^l, l < 16
 };
+static_assert(sizeof(Slice) % 16 == 0, "slices start on 16-byte boundaries");
+__device__ __forceinline__ u64 *slice_start(Slice *s) { return reinterpret_cast<u64 *>(s + 1); }
+__device__ __forceinline__ u32 *slice_filter(Slice *s, u32 gs) { return reinterpret_cast<u32 *>(slice_start(s) + gs + 2); }
+constexpr u32 INDEX_PT = 16;           // index slots per anchor
+static_assert(INDEX_PT <= FILTER_WPT, "the index lies in the filter's words");
+// queue of filter passes: {value bits, item, giant step}
+__device__ __forceinline__ uint4 *slice_queue(Slice *s, u32 gs) { return reinterpret_cast<uint4 *>(slice_filter(s, gs) + FILTER_WPT * gs); }
+__host__ __device__ constexpr size_t slice_bytes(u32 gs)
+{
+    return sizeof(Slice) + (gs + 2) * 8 + (size_t)FILTER_WPT * gs * 4 + gs / 4 * 16;
+}
+static_assert(slice_bytes(32) % 16 == 0, "slices start on 16-byte boundaries");
+// the slices of TPB/gs groups take the most room for gs = 32
+template <int TPB>
+constexpr size_t smem_bytes() { return slice_bytes(32) * (TPB / 32); }
+
 extern __shared__ __align__(128) unsigned char smem_raw[];
-__shared__ BsgsArgs s_args;
-__shared__ BsgsArgs s_args_next;                         // batch launches: the job arguments of the next prime
-__shared__ PrimeCtx s_ctx;
 __shared__ unsigned long long s_cands, s_dups, s_facs;   // per-CTA totals
-__shared__ unsigned long long s_baby, s_giant, s_small;  // per-CTA totals kept by thread 0
-__shared__ u32 s_nsol, s_sol_i[KMAX], s_sol_u0[KMAX];   // small-order solutions
-
-// A residue's table value: the residue itself, or with FP64 steps (MODE 2) the
-// bit pattern of the double that holds it exactly (every step of that mode
-// yields canonical residues, so equal residues have equal bits).
-__device__ __forceinline__ u64 fp_val(u64 v) { return (u64)__double_as_longlong(fp_exact(v)); }
-__device__ __forceinline__ u64 fp_res(u64 bits) { return (u64)__longlong_as_double((long long)bits); }
-__device__ __forceinline__ u64 to_val(u64 v) { return s_ctx.fp ? fp_val(v) : v; }
-__device__ __forceinline__ u64 to_res(u64 val) { return s_ctx.fp ? fp_res(val) : val; }
-
-// Dynamic shared memory: fingerprints | indices | counts | start values | giant
-// start powers | two record staging buffers.
-template <int TPB, int NB>
-struct Smem {
-    static __device__ __forceinline__ Table table()
-    {
-        Table T;
-        T.fpb = reinterpret_cast<uint4 *>(smem_raw);
-        T.jt = reinterpret_cast<unsigned short *>(T.fpb + NB);
-        T.cnt = reinterpret_cast<u32 *>(T.jt + 8 * NB);
-        return T;
-    }
-    static __device__ __forceinline__ u64 *start() { return reinterpret_cast<u64 *>(table().cnt + NB / 2); }
-    static __device__ __forceinline__ u64 *zs() { return start() + TPB; }
-    static __device__ __forceinline__ RecBuf *rec() { return reinterpret_cast<RecBuf *>(zs() + TPB); }
-    static constexpr size_t bytes() { return (size_t)NB * 16 + (size_t)NB * 16 + (size_t)NB * 2 + (size_t)TPB * 16 + 2 * sizeof(RecBuf); }
-};
+__shared__ unsigned long long s_baby, s_giant, s_small;
 
 // First claimer of term (seq, n) clears its bitmap bit and appends the factor.
-__device__ __forceinline__ void claim(u64 p, u32 seq, u32 n)
+__device__ __forceinline__ void claim(const BsgsArgs &a, u64 p, u32 seq, u32 n)
 {
-    const BsgsArgs &a = s_args;
     const u32 o = n - a.nmin;
     u32 *w = a.bitmap + (size_t)seq * a.words + (o >> 5);
     const u32 mask = 1u << (o & 31);
@@ -241,444 +225,434 @@ __device__ __forceinline__ void claim(u64 p, u32 seq, u32 n)
     }
 }
 
-// exact check of a fingerprint match: y_j == val ?  (y_j from its thread's
-// start, by integer steps on the residues whatever the launch's step kind)
-__device__ __forceinline__ bool verify(const u64 *s_start, u32 j, u64 val)
+// Builds the group's index of anchors (open addressing over 16 GS slots, t + 1
+// in a slot, 0: empty) in the filter's place, and pw[l] = s^l for l < 16.
+// Called by the whole group after the last use of the filter; the checks below
+// follow it.
+template <int MODE>
+__device__ __noinline__ void build_index(Slice *sl, const PrimeHdr *H, u32 gid, u32 gs, u32 gt)
 {
-    const PrimeCtx c = s_ctx;
-    if (j >= c.qp) return false;
-    u64 y = to_res(s_start[j / c.cp]);
-    for (u32 r = j % c.cp; r; --r) y = baby_step(y, c.smul, c.s, c.p, c.q);
-    return y == to_res(val);
+    typedef typename Ring<MODE>::V V;
+    u32 *idx = slice_filter(sl, gs);
+    u64 *start = slice_start(sl);
+    for (u32 i = gt; i < INDEX_PT / 4 * gs; i += gs) reinterpret_cast<uint4 *>(idx)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (gt < 16) {
+        const Ring<MODE> R(*H);
+        V x = Ring<MODE>::val(H->s), r = (gt & 1) ? x : Ring<MODE>::one(*H);
+        for (u32 k = 1; k < 4; ++k) {
+            x = R.mul(x, x);
+            const V t = R.mul(r, x);
+            r = ((gt >> k) & 1) ? t : r;
+        }
+        sl->pw[gt] = Ring<MODE>::bits(r);
+    }
+    group_sync(gid, gs);
+    // anchors t = gt, and by the first thread the one past the end, s^Q'; at most
+    // GS + 1 entries, so the walks end
+    for (u32 t = gt; t < gs + 1; t += gs) {
+        const u64 v = (t == gs) ? H->S : start[t];
+        if (t == gs) start[gs] = v;
+        u32 k = __umulhi(val_hash(v), INDEX_PT * gs);
+        while (atomicCAS(&idx[k], 0u, t + 1) != 0u) k = (k + 1) & (INDEX_PT * gs - 1);
+    }
+    group_sync(gid, gs);
 }
 
-// Giant-step match or overflowed bucket: check every matching slot of the
-// chain starting at bucket b exactly and claim n = nmin + off + e*((q+1)Q'-1-j).
-template <int TPB, int C, int NB>
-__device__ __noinline__ void giant_slow(u64 gamma, u32 b, u32 fp, u32 qq, u32 meta)
+// The anchor equal to v, or NONE.
+__device__ __forceinline__ u32 anchor_find(const u32 *idx, const u64 *start, u32 gs, u64 v)
 {
-    const u32 Q = s_ctx.qp;
-    const Table T = Smem<TPB, NB>::table();
-    const u64 *st = Smem<TPB, NB>::start();
-    for (int pr = 0; pr < BSGS_MAXPROBE; ++pr) {
-        const uint4 bv = T.fpb[b];
-#pragma unroll
-        for (int k = 0; k < 7; ++k) {
-            if (slot_fp(bv, k) != fp) continue;
-            atomicAdd(&s_cands, 1ull);
-            const u32 j = T.jt[8 * b + k];
-            if (!verify(st, j, gamma)) continue;
-            const u64 u = (u64)(qq + 1) * Q - 1 - j;
-            const u64 n = (u64)s_args.nmin + (meta >> 7) + (u64)s_ctx.e * u;
-            if (n <= s_args.nmax) claim(s_ctx.p, meta & 0x7Fu, (u32)n);
-        }
-        if (!(bv.w & OVF_FLAG)) break;
-        b = (b + 1 == NB) ? 0u : b + 1;
+    u32 k = __umulhi(val_hash(v), INDEX_PT * gs);
+    for (u32 n = 0; n < INDEX_PT * gs; ++n) {
+        const u32 e = idx[k];
+        if (e == 0) return NONE;
+        if (start[e - 1] == v) return e - 1;
+        k = (k + 1) & (INDEX_PT * gs - 1);
+    }
+    return NONE;
+}
+
+// Exact discrete logarithm of gamma (uniform over the warp) to the base s among
+// the group's anchors: lane l < 16 looks gamma * s^l up.  Returns 16t - l, in
+// (-16, Q'], of the first lane that finds an anchor t, or NO_LOG.  When ord(s) >
+// Q' the anchors differ, and gamma = s^j with 0 <= j < Q' is found as exactly
+// that j.  Called by a whole warp.
+constexpr int NO_LOG = -1000;
+template <int MODE>
+__device__ __forceinline__ int warp_find(const Ring<MODE> &R, Slice *sl, u32 gs, typename Ring<MODE>::V gamma)
+{
+    const u32 lane = threadIdx.x & 31;
+    u32 t = NONE;
+    if (lane < 16)
+        t = anchor_find(slice_filter(sl, gs), slice_start(sl), gs,
+                        Ring<MODE>::bits(R.mul(gamma, Ring<MODE>::val(sl->pw[lane]))));
+    const u32 found = __ballot_sync(0xFFFFFFFFu, t != NONE);
+    if (!found) return NO_LOG;
+    const u32 src = __ffs((int)found) - 1;
+    return (int)(16 * __shfl_sync(0xFFFFFFFFu, t, src)) - (int)src;
+}
+
+// Item w of a prime's giant phase: chunk g of target i, w = g*numk + i, by the
+// float reciprocal in the header: (w + 1/2)/numk lies at least 1/(2 numk) from
+// an integer and errs by under 2^-21 of itself (w < 2^17).
+__device__ __forceinline__ void item_of(u32 w, const PrimeHdr *H, u32 &g, u32 &i)
+{
+    g = (u32)(((float)w + 0.5f) * H->rk);
+    i = w - g * H->numk;
+}
+
+// Lane l < 16's share of a filter pass's exact check: if gamma * s^l is anchor t,
+// gamma = s^j with j = 16t - l, and for 0 <= j < Q' the step (item w, giant step
+// t of its chunk) claims n = nmin + off + e*((q+1)Q'-1-j).
+template <int MODE>
+__device__ __forceinline__ void check_pass(const Ring<MODE> &R, Slice *sl, const PrimeHdr *H, u32 gs, u64 gamma, u32 w,
+                                           u32 t, u32 l, const BsgsArgs *args, const unsigned short *meta)
+{
+    const u32 a = anchor_find(slice_filter(sl, gs), slice_start(sl), gs,
+                              Ring<MODE>::bits(R.mul(Ring<MODE>::val(gamma), Ring<MODE>::val(sl->pw[l]))));
+    if (a == NONE) return;
+    const int Q = 16 * (int)gs, j = 16 * (int)a - (int)l;
+    if (j < 0 || j >= Q) return;
+    u32 g, i;
+    item_of(w, H, g, i);
+    const u32 m = meta[i];
+    const u64 u = (u64)(g * H->Lc + t + 1) * (u32)Q - 1 - (u32)j;
+    const u64 n = (u64)args->nmin + (m >> 7) + (u64)H->e * u;
+    if (n <= args->nmax) claim(*args, H->p, m & 0x7Fu, (u32)n);
+}
+
+// Start value of item w: T_i * S^(g*Lc).
+template <int MODE>
+__device__ __forceinline__ typename Ring<MODE>::V item_start(const Ring<MODE> &R, u32 w, const PrimeHdr *H, const u64 *tb,
+                                                             const u64 *tg)
+{
+    typedef typename Ring<MODE>::V V;
+    u32 g, i;
+    item_of(w, H, g, i);
+    V z = Ring<MODE>::val(tb[64 + (g & 31)]);
+    if (H->G > 32) z = R.mul(z, Ring<MODE>::val(tb[96 + (g >> 5)]));
+    return R.mul(Ring<MODE>::val(tg[i]), z);
+}
+
+// More filter passes than the queue holds (p not far above Q', where most are
+// true): the giant steps of items [w0, w1) again, one item per thread, each
+// value checked by its own thread.
+template <int MODE>
+__device__ __noinline__ void giant_unqueued(Slice *sl, const PrimeHdr *H, u32 gs, u32 gt, u32 w0, u32 w1, const u64 *tb,
+                                            const u64 *tg, const BsgsArgs *args, const unsigned short *meta)
+{
+    typedef typename Ring<MODE>::V V;
+    const Ring<MODE> R(*H);
+    const typename Ring<MODE>::Fix f = Ring<MODE>::giant(*H);
+    for (u32 w = w0 + gt; w < w1; w += gs) {
+        V g = item_start<MODE>(R, w, H, tb, tg);
+        for (u32 t = 0; t < H->Lc; ++t, g = R.step(g, f))
+            for (u32 l = 0; l < 16; ++l) check_pass<MODE>(R, sl, H, gs, Ring<MODE>::bits(g), w, t, l, args, meta);
     }
 }
 
-// The giant step's table probe: one 128-bit load, four paired fp16 compares
-// and one branch in the common case.  The flag half of the last word (0 or
-// 0x8000, i.e. +-0 as fp16) never equals a fingerprint, so all eight halves
-// are compared without masking.
-template <int TPB, int C, int NB>
-__device__ __forceinline__ void giant_probe(const Table &T, u64 g, u32 qq, u32 meta)
+// ord(s) <= Q': each target is looked up once; every n in range with the same
+// residue mod e*ord is claimed (giant.cl:146-168).  Warps of the group take
+// targets in turn.  Called by whole warps.
+template <int MODE>
+__device__ __noinline__ void small_order_search(Slice *sl, const PrimeHdr *H, const BsgsArgs *args, u32 gs, u32 gt,
+                                                const u64 *__restrict__ tgt, const unsigned short *__restrict__ meta)
 {
-    u32 b, fp;
-    tab_hash<NB>(g, b, fp);
-    const u32 kk = fp * 0x10001u;
-    const uint4 bv = T.fpb[b];
-    const u32 m = heq2(bv.x, kk) | heq2(bv.y, kk) | heq2(bv.z, kk) | heq2(bv.w, kk);
-    if (__builtin_expect((m | (bv.w & OVF_FLAG)) != 0, 0)) {
-        // about 1% of buckets overflowed: with no match here, the next bucket
-        // is checked inline, and only matches or longer chains go out of line
-        bool slow = (m != 0);
-        if (!slow) {
-            const uint4 bn = T.fpb[(b + 1 == NB) ? 0u : b + 1];
-            slow = ((heq2(bn.x, kk) | heq2(bn.y, kk) | heq2(bn.z, kk) | heq2(bn.w, kk)) | (bn.w & OVF_FLAG)) != 0;
-        }
-        if (slow) giant_slow<TPB, C, NB>(g, b, fp, qq, meta);
-    }
-}
-
-// Continues an insertion whose home bucket was full; returns 1 if the walk
-// gave up after maxprobe buckets.
-template <int NB>
-__device__ __noinline__ u32 insert_walk(u32 b, u32 fp, u32 j, int maxprobe)
-{
-    const Table T = Smem<0, NB>::table();
-    b = (b + 1 == NB) ? 0u : b + 1;
-    for (int pr = 1; pr < maxprobe; ++pr)
-        if (tab_try<NB>(T, b, fp, j)) return 0;
-    return 1;
-}
-
-__device__ __forceinline__ void clear_table(const Table &T, u32 nb)
-{
-    for (u32 i = threadIdx.x; i < nb; i += blockDim.x) T.fpb[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (u32 i = threadIdx.x; i < nb / 8; i += blockDim.x) reinterpret_cast<uint4 *>(T.cnt)[i] = make_uint4(0u, 0u, 0u, 0u);
-}
-
-// ord(s) < Q': rebuild the table from the distinct values j < ord (the
-// speculative one may hold repeats).  Called by the whole CTA.
-template <int TPB, int C, int NB>
-__device__ __noinline__ void rebuild_table(u32 order)
-{
-    const Table T = Smem<TPB, NB>::table();
-    const u64 *st = Smem<TPB, NB>::start();
-    const PrimeCtx c = s_ctx;
-    clear_table(T, NB);
-    __syncthreads();
-    u64 y = to_res(st[threadIdx.x]);
-    u32 pend = 0;
-    for (u32 i = 0; i < c.cp; ++i) {
-        const u32 j = threadIdx.x * c.cp + i;
-        if (j < order) {
-            u32 b, fpv;
-            tab_hash<NB>(to_val(y), b, fpv);
-            int pr = 0;
-            while (pr < BSGS_MAXPROBE && !tab_try<NB>(T, b, fpv, j)) ++pr;
-            if (pr >= BSGS_MAXPROBE) pend = 1;
-        }
-        y = baby_step(y, c.smul, c.s, c.p, c.q);
-    }
-    if (pend) atomicOr(s_args.err, ERR_HASH_OVERFLOW);
-    __syncthreads();
-}
-
-// ord(s) < Q': each target is looked up once; every n in range with the same
-// residue mod e*ord is claimed (giant.cl:146-168).  Called by the whole CTA.
-template <int TPB, int C, int NB>
-__device__ __noinline__ void small_order_search(const RecBuf *R, u32 order)
-{
-    const u32 Q = s_ctx.qp;
-    const Table T = Smem<TPB, NB>::table();
-    const u64 *st = Smem<TPB, NB>::start();
-    const u32 tid = threadIdx.x;
-    if (tid < R->hdr.numk) {
-        // FP64 launches' tables carry R^2: the target T*R times R^2 mod p
-        // (the header's ssw there) by one Montgomery product
-        const u64 Tv = to_val(s_ctx.fp ? mmul(R->tgt[tid], R->hdr.ssw, s_ctx.p, s_ctx.q) : R->tgt[tid]);
-        u32 b, fp;
-        tab_hash<NB>(Tv, b, fp);
-        for (int pr = 0; pr < BSGS_MAXPROBE; ++pr) {
-            const uint4 bv = T.fpb[b];
-            for (int k = 0; k < 7; ++k) {
-                if (slot_fp(bv, k) != fp) continue;
-                atomicAdd(&s_cands, 1ull);
-                const u32 j = T.jt[8 * b + k];
-                if (j >= order || !verify(st, j, Tv)) continue;
-                const u32 ks = atomicAdd(&s_nsol, 1u);
-                s_sol_i[ks] = tid;
-                s_sol_u0[ks] = (Q - 1 - j) % order;
-            }
-            if (!(bv.w & OVF_FLAG)) break;
-            b = (b + 1 == NB) ? 0u : b + 1;
-        }
-    }
-    __syncthreads();
-    const u32 nsol = s_nsol;
-    const u32 e = s_ctx.e;
-    for (u32 k = 0; k < nsol; ++k) {
-        const u32 m = R->meta[s_sol_i[k]];
-        const u32 seq = m & 0x7Fu, off = m >> 7;
-        for (u64 u = s_sol_u0[k] + (u64)tid * order;; u += (u64)TPB * order) {
-            const u64 n = (u64)s_args.nmin + off + (u64)e * u;
-            if (n > s_args.nmax) break;
-            claim(s_ctx.p, seq, (u32)n);
+    const Ring<MODE> R(*H);
+    const u32 lane = gt & 31;
+    const u32 Q = 16 * gs, order = sl->order;
+    for (u32 i = gt >> 5; i < H->numk; i += gs >> 5) {
+        const int j = warp_find<MODE>(R, sl, gs, Ring<MODE>::val(tgt[i]));
+        if (j == NO_LOG) continue;
+        if (lane == 0) atomicAdd(&s_cands, 1ull);
+        const u32 u0 = (u32)((int)(Q - 1 + order) - j) % order;
+        const u32 m = meta[i];
+        for (u64 u = u0 + (u64)lane * order;; u += 32ull * order) {
+            const u64 n = (u64)args->nmin + (m >> 7) + (u64)H->e * u;
+            if (n > args->nmax) break;
+            claim(*args, H->p, m & 0x7Fu, (u32)n);
         }
     }
 }
 
-// Work item i of a batch launch: range slot k contributes prefix[k+1]-prefix[k]
-// primes (0 when it is not in the launch's group), in record slots
-// k*rcap + (0, 1, ...).
-__device__ __forceinline__ u32 batch_slot(u32 i, u32 nr, const u32 *prefix, u32 rcap)
+// The least j in (0, Q'] with y_j = 1 among this thread's chain, merged into
+// the group's order (only called when some value's hash equals that of 1).
+template <int MODE>
+__device__ __noinline__ void order_check(Slice *sl, const PrimeHdr *H, u32 j0, u64 x0)
 {
-    const u32 k = prefix_find(prefix, nr, i);
-    return k * rcap + (i - prefix[k]);
+    const Ring<MODE> R(*H);
+    const typename Ring<MODE>::V s = Ring<MODE>::val(H->s);
+    const u64 one = Ring<MODE>::bits(Ring<MODE>::one(*H));
+    typename Ring<MODE>::V x = Ring<MODE>::val(x0);
+    for (u32 j = j0 + 1; j <= j0 + 16; ++j) {
+        x = R.mul(x, s);
+        if (Ring<MODE>::bits(x) == one) {
+            atomicMin(&sl->order, j);
+            return;
+        }
+    }
 }
 
-// MODE: 2 = every prime below FP_BOUND = 2^51 (FP64 baby and giant steps,
-// fp_mulfix), 1 = every prime below 2^63 (Shoup steps), 0 = every prime at or
-// above 2^63 (Montgomery giant steps).  1024 / TPB CTAs share an SM, so the
-// bound keeps each thread at 64 registers.  BATCH: the primes of several
-// ranges (jobs) in one launch -- work item i maps to a record slot through the
-// group's prefix sums, and each prime's job arguments come from job_args.
-template <int TPB, int C, int NB, int MODE, bool BATCH>
-__global__ void __launch_bounds__(TPB, 1024 / TPB) k_bsgs(BsgsArgs a, const PrimeHdr *__restrict__ hdr,
-                                                 const u64 *__restrict__ tabs, const u64 *__restrict__ tgt,
-                                                 const unsigned short *__restrict__ meta, u32 count, u32 *work_ctr,
-                                                 const BsgsArgs *__restrict__ job_args, u32 nr,
-                                                 const u32 *__restrict__ prefix, u32 rcap)
+// The primes of one launch, sorted by class into lists of record indices
+// (setup.cu): count[c] primes of class c at lists + c*stride.  CTAs of TPB
+// threads work through the classes from the largest down; a class of GS
+// threads per prime runs TPB/GS groups side by side, each claiming the next
+// prime of the class when it finishes one.  taken[c] starts at zero.
+// MODE: 2 = every prime below FP_BOUND = 2^51 (FP64 steps), 1 = every prime
+// below 2^63 (Shoup steps), 0 = every prime at or above 2^63 (Montgomery
+// steps).  1024 / TPB CTAs share an SM, so the bound keeps each thread at 64
+// registers.  BATCH: the primes of several jobs; each prime's job arguments
+// come from job_args.
+template <int TPB, int MODE, bool BATCH>
+__global__ void __launch_bounds__(TPB, 1024 / TPB)
+    k_bsgs(BsgsArgs a, const PrimeHdr *__restrict__ hdr, const u64 *__restrict__ tabs, const u64 *__restrict__ tgt,
+           const unsigned short *__restrict__ meta, const u32 *__restrict__ lists, u32 stride,
+           const u32 *__restrict__ count, u32 *taken, const BsgsArgs *__restrict__ job_args)
 {
-    constexpr u32 NONE = 0xFFFFFFFFu;
-    if (BATCH) count = prefix[nr];
-    auto slot_of = [&](u32 i) -> u32 {
-        if (i >= count) return NONE;
-        return BATCH ? batch_slot(i, nr, prefix, rcap) : i;
-    };
-    constexpr u32 Q = TPB * C;
-    static_assert(Q <= 65536, "baby indices are stored in 16 bits");
-    static_assert(NB <= 65536, "bucket indices are packed into 16 bits");
-    constexpr int IBMAX = 8;                                      // values inserted per round (two chains)
-    static_assert(C >= IBMAX, "cp in {C, C/2, C/4} splits into rounds of IBMAX/2, IBMAX/4 or IBMAX/8 per chain");
-    const Table T = Smem<TPB, NB>::table();
-    u64 *s_start = Smem<TPB, NB>::start();
-    u64 *s_Z = Smem<TPB, NB>::zs();
-    RecBuf *rec = Smem<TPB, NB>::rec();                           // two staging buffers
-    __shared__ __align__(8) u64 s_bar[3];                        // [2]: never completed (failure test)
-    __shared__ u32 s_idx[2], s_order, s_spill, s_abort, s_claim;
+    typedef Ring<MODE> RM;
+    typedef typename RM::V V;
+    // (the integer products' longer code runs slower unrolled further: 8% at p
+    // near 2^64)
+    constexpr int BABY_UNROLL = MODE == 2 ? 8 : 2, GIANT_UNROLL = MODE == 2 ? 4 : 2;
+    __shared__ __align__(8) u64 s_bar[TPB / 32][2];               // record copies of each group (by its first warp)
+    __shared__ __align__(8) u64 s_dead;                           // never completed (failure test)
+    __shared__ u32 s_par[TPB / 32][2];                            // parity of each barrier's next phase
+    __shared__ BsgsArgs s_args;
+    __shared__ u32 s_abort;
     const u32 wait_bound = a.wait_bound ? a.wait_bound : WAIT_BOUND;
-    u32 pend_buf = 0, pend_par = 0;                               // the copy waited for when aborting
-
     const u32 tid = threadIdx.x;
-    auto fetch = [&](u32 buf, u32 idx) {                          // thread 0 only
-        RecBuf *r = &rec[buf];
-        mbar_expect_tx(&s_bar[buf], (u32)sizeof(RecBuf));
-        bulk_load(&r->hdr, hdr + idx, (u32)sizeof(PrimeHdr), &s_bar[buf]);
-        bulk_load(r->tabs, tabs + (size_t)idx * TABS, TABS * 8, &s_bar[buf]);
-        bulk_load(r->tgt, tgt + (size_t)idx * KSTRIDE, KSTRIDE * 8, &s_bar[buf]);
-        bulk_load(r->meta, meta + (size_t)idx * KSTRIDE, KSTRIDE * 2, &s_bar[buf]);
-    };
+    if ((tid & 31) == 0) {
+        mbar_init(&s_bar[tid >> 5][0], 1);
+        mbar_init(&s_bar[tid >> 5][1], 1);
+        s_par[tid >> 5][0] = s_par[tid >> 5][1] = 0;
+    }
     if (tid == 0) {
-        mbar_init(&s_bar[0], 1);
-        mbar_init(&s_bar[1], 1);
-        mbar_init(&s_bar[2], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_init(&s_dead, 1);
         s_args = a;
         s_abort = 0;
-        s_cands = 0;
-        s_dups = 0;
-        s_facs = 0;
-        s_baby = 0;
-        s_giant = 0;
-        s_small = 0;
-        const u32 i0 = slot_of(atomicAdd(work_ctr, 1u));
-        s_idx[0] = i0;
-        if (i0 != NONE) fetch(0, i0);
-        s_claim = slot_of(atomicAdd(work_ctr, 1u));              // the prime after it, resolved ahead
-        if (BATCH && i0 != NONE) s_args_next = job_args[hdr[i0].job];
+        s_cands = s_dups = s_facs = 0;
+        s_baby = s_giant = s_small = 0;
     }
-    __syncthreads();
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 
-    for (u32 it = 0;; ++it) {
-        const u32 buf = it & 1;
-        const u32 idx = s_idx[buf];
-        if (idx == NONE) break;
-        // this prime's record was fetched one prime ago; the wait is bounded.
-        // A failure test sends the first wait to s_bar[2], which no copy or
-        // arrival ever completes, so the bound runs out.
-        pend_buf = buf;
-        pend_par = (it >> 1) & 1;
-        {
-            const bool dead = (a.test_stall != 0) && (it == 0);
-            u64 *bar = dead ? &s_bar[2] : &s_bar[buf];
-            const u32 par = dead ? 0u : pend_par;
-            u32 n = 0;
-            while (!mbar_try_wait(bar, par)) {
-                if (++n > wait_bound) { atomicOr(&s_abort, 1u); break; }
-            }
-        }
-        const RecBuf &R = rec[buf];
-        const bool live = (R.hdr.p != 0);
-        const u64 p = R.hdr.p, q = R.hdr.q, s = R.hdr.s;
-        const u32 e = R.hdr.e, smul = R.hdr.smul;
-        const u32 cp = R.hdr.cp;                                  // baby steps per thread for this prime
-        // The next prime's index (and, for a batch, its job's arguments) were
-        // claimed and resolved during the previous prime, off the barriers'
-        // critical path: thread 0 only copies them here.
-        if (tid == 0) {
-            s_order = 0xFFFFFFFFu;
-            s_nsol = 0;
-            s_spill = 0;
-            s_ctx.p = p; s_ctx.q = q; s_ctx.s = s; s_ctx.smul = smul; s_ctx.e = e;
-            s_ctx.cp = cp; s_ctx.qp = TPB * cp; s_ctx.fp = (MODE == 2);
-            if (BATCH) s_args = s_args_next;
-        }
-        if (live) clear_table(T, NB);
-        __syncthreads();
-        if (s_abort) break;
-        if (tid == 0) {
-            const u32 nxt = s_claim;
-            s_idx[buf ^ 1] = nxt;
-            if (nxt != NONE) {                                    // rec[buf^1] was last read before the previous barrier
+    for (int c = NCLASS - 1; c >= 0; --c) {
+        const u32 gs = 32u << c;
+        const u32 n = count[c];
+        if (gs > TPB || n == 0) continue;
+        __syncthreads();                                          // slices of the previous class are free
+        const bool stop = s_abort != 0;
+        __syncthreads();                                          // (the flag is read before any group can set it again)
+        if (stop) break;
+        const u32 gid = tid / gs, gt = tid & (gs - 1), w0 = gid * (gs >> 5);
+        const u32 ngroups = gridDim.x * (TPB / gs);
+        Slice *sl = reinterpret_cast<Slice *>(smem_raw + gid * slice_bytes(gs));
+        u64 *start = slice_start(sl);
+        u32 *filt = slice_filter(sl, gs);
+        const u32 nw = FILTER_WPT * gs;
+        const u32 *list = lists + (size_t)c * stride;
+        auto fetch = [&](u32 buf, u32 r) {                        // group's first thread only
+            mbar_expect_tx(&s_bar[w0][buf], (u32)sizeof(PrimeHdr));
+            bulk_load(&sl->hdr[buf], hdr + r, (u32)sizeof(PrimeHdr), &s_bar[w0][buf]);
+            l2_prefetch(tabs + (size_t)r * TABS, TABS * 8);
+            l2_prefetch(tgt + (size_t)r * KSTRIDE, KSTRIDE * 8);
+            l2_prefetch(meta + (size_t)r * KSTRIDE, KSTRIDE * 2);
+        };
+        // the first prime of each group is fixed, the others are claimed in order
+        // (past the end there is nothing: NONE)
+        auto claimed = [&](u32 k) -> u32 { return k < n ? list[k] : NONE; };
+        if (gt == 0) {
+            const u32 r = claimed(blockIdx.x + gid * gridDim.x);
+            sl->idx[0] = r;
+            sl->claim = NONE;
+            sl->abort = 0;
+            if (r != NONE) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                fetch(buf ^ 1, nxt);
+                fetch(0, r);
+                sl->claim = claimed(ngroups + atomicAdd(&taken[c], 1u));
             }
         }
-        // MODE 2: start values by FP64 products x*y mod p (1/p in the header's
-        // Sw), the set-up having stored Z2, s^(cp/2) and S^(Lc/2) plain: baby and
-        // giant values carry R^2 (the header's ssw) where the integer modes'
-        // Montgomery products leave R
-        const double pd = fp_exact(p), pinv = __longlong_as_double((long long)R.hdr.Sw);
-        if (live) {
-            if (tid < R.hdr.G) {
-                const u64 z1 = R.tabs[64 + (tid & 31)], z2 = R.tabs[96 + (tid >> 5)];
-                s_Z[tid] = (MODE == 2) ? (u64)__double_as_longlong(fp_mul(fp_exact(z1), fp_exact(z2), pd, pinv))
-                                       : mmul(z1, z2, p, q);
-            }
-            // ---- baby steps y_j = s^j, j < Q' = TPB*cp, inserted as they are produced ----
-            // Speculative: ord(s) < Q' is only known after the barrier; then the
-            // table (which may hold repeats) is rebuilt from j < ord.
-            const u64 ta = R.tabs[tid & 31], tb = R.tabs[32 + (tid >> 5)];
-            // s^(cp*tid); MODE 2: table values are the bits of the doubles holding the residues
-            const u64 x0 = (MODE == 2) ? (u64)__double_as_longlong(fp_mul(fp_exact(ta), fp_exact(tb), pd, pinv))
-                                       : mmul(ta, tb, p, q);
-            const u64 one = (MODE == 2) ? fp_val(R.hdr.ssw) : R.hdr.one;
-            s_start[tid] = x0;
-            u32 spill = 0;
-            // Two chains per thread, j in [tid*cp, tid*cp + cp/2) and the next
-            // cp/2 (started from s^(cp/2) further), so the two products of a step
-            // are independent.  The step kind is uniform per prime (b^e = 2, 4 or
-            // other) and is chosen once, so the loop body carries no dispatch;
-            // the least j > 0 with y_j = 1 is kept per thread and merged with one
-            // atomicMin.  Other multipliers take Shoup's product by the plain s
-            // below 2^63 (the same residues as the Montgomery product verify()
-            // uses).
-            u32 minj = 0xFFFFFFFFu;
-            const u64 ssw = R.hdr.ssw;
-            const u64 sp = R.hdr.sp;
-            const u32 half = cp >> 1;
-            u64 xa = x0, xb;
-            if (MODE == 2)
-                xb = (u64)__double_as_longlong(fp_mul(__longlong_as_double((long long)x0), fp_exact(R.hdr.u2), pd, pinv));
-            else
-                xb = mmul(x0, R.hdr.u2, p, q);
-            const double sd = fp_exact(sp), sq = __longlong_as_double((long long)R.hdr.S);
-            // IB2 values of each chain are hashed and stepped, then inserted, per
-            // round (IB2 = IBMAX/2, or cp/2 when it is smaller)
-            auto babies = [&](auto kind, auto ibc) {
-                constexpr int K = decltype(kind)::value;          // 2, 4: doublings; 1: Shoup; 0: baby_step
-                constexpr int IB2 = decltype(ibc)::value;
-                auto step = [&](u64 v) -> u64 {
-                    if (MODE == 2) {
-                        double x = __longlong_as_double((long long)v);
-                        if (K == 1) x = fp_mulfix(x, sd, sq, pd);
-                        else { x = fp_dbl(x, pd); if (K == 4) x = fp_dbl(x, pd); }
-                        return (u64)__double_as_longlong(x);
-                    }
-                    if (K == 0) return baby_step(v, smul, s, p, q);
-                    if (K == 1) return shoup_mul(v, sp, ssw, p);
-                    if (MODE == 1) { v = dbl63(v, p); return (K == 4) ? dbl63(v, p) : v; }
-                    v = madd(v, v, p);
-                    return (K == 4) ? madd(v, v, p) : v;
-                };
-#pragma unroll 1
-                for (u32 h0 = 0; h0 < half; h0 += IB2) {
-                    u32 bf[2 * IB2], old[2 * IB2];                // bucket << 16 | fingerprint; claimed slot
+        group_sync(gid, gs);
+
+        // one pass of the loop per prime, or per segment seg of a prime with a long
+        // giant phase (every segment fills the filter again)
+        for (u32 it = 0, seg = 0;;) {
+            const u32 buf = it & 1;
+            const u32 r = sl->idx[buf];
+            if (r == NONE) break;
+            // the starts' table entries, and an empty filter while they arrive
+            const u64 *tb = tabs + (size_t)r * TABS;
+            const u64 ta = tb[gt & 31], tB = tb[32 + (gt >> 5)];
+            {
+                uint4 *z = reinterpret_cast<uint4 *>(filt);
+                const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-                    for (int i = 0; i < IB2; ++i) {
-                        const u32 ja = tid * cp + h0 + i, jb = ja + half;
-                        if (ja != 0 && xa == one) minj = min(minj, ja);
-                        if (xb == one) minj = min(minj, jb);
-                        u32 bk, fp;
-                        tab_hash<NB>(xa, bk, fp);
-                        bf[2 * i] = (bk << 16) | fp;
-                        tab_hash<NB>(xb, bk, fp);
-                        bf[2 * i + 1] = (bk << 16) | fp;
+                for (u32 i = 0; i < FILTER_WPT / 4; ++i) z[i * gs + gt] = zero;
+            }
+            // this prime's header was fetched one prime ago; the wait is bounded.
+            // A failure test sends the first wait to s_dead, which no copy or
+            // arrival ever completes, so the bound runs out.
+            if (seg == 0) {
+                const bool dead = (a.test_stall != 0) && (it == 0);
+                u64 *bar = dead ? &s_dead : &s_bar[w0][buf];
+                const u32 want = dead ? 0u : s_par[w0][buf];
+                u32 tries = 0;
+                while (!mbar_try_wait(bar, want)) {
+                    if (++tries > wait_bound) { sl->abort = 1; break; }
+                }
+            }
+            if (gt == 0) {
+                sl->order = NONE;
+                sl->nq = 0;
+            }
+            group_sync(gid, gs);
+            if (sl->abort) {
+                // The group stops before fetching another record, so the only copy
+                // that can still be in flight is the one waited for: report, then
+                // let it land (bounded by the default) before the CTA's shared
+                // memory is released.
+                if (gt == 0) {
+                    atomicOr(a.err, ERR_TMA_TIMEOUT);
+                    s_abort = 1;
+                    u32 tries = 0;
+                    while (tries < WAIT_BOUND && !mbar_try_wait(&s_bar[w0][buf], s_par[w0][buf])) ++tries;
+                }
+                break;
+            }
+            if (gt == 0 && seg == 0) {
+                s_par[w0][buf] ^= 1;
+                const u32 nxt = sl->claim;
+                sl->idx[buf ^ 1] = nxt;
+                if (nxt != NONE) {                                // hdr[buf^1] was last read before the barrier
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    fetch(buf ^ 1, nxt);
+                }
+            }
+            const PrimeHdr *H = &sl->hdr[buf];
+            const RM R(*H);
+            // The last thread claims the prime after next.  The claim, issued here,
+            // and the load of its record index, issued after the baby steps, are
+            // taken up a phase later, so no warp waits for them.
+            const bool claimer = (gt == gs - 1) && seg == 0;
+            u32 ahead = NONE;
+            if (claimer) ahead = ngroups + atomicAdd(&taken[c], 1u);
+            // ---- baby steps y_j = s^j, j < Q' = 16 GS, entered as they are produced ----
+            {
+                const V x0 = R.mul(RM::val(ta), RM::val(tB));     // s^(16 gt)
+                start[gt] = RM::bits(x0);
+                // two chains, j in [16 gt, 16 gt + 8) and the next 8, so that the
+                // two products of a step are independent; the step kind is uniform
+                // per prime and chosen once.  A value whose hash equals that of 1
+                // is a candidate for y_j = 1, j > 0: the values after each step,
+                // j = 16 gt + 1 .. 16 gt + 16, are compared.
+                const typename RM::Fix f = RM::baby(*H);
+                const u32 h1 = val_hash(RM::bits(RM::one(*H)));
+                V xa = x0, xb = R.mul(x0, RM::val(H->u8));
+                bool unit = false;
+                auto babies = [&](auto kind) {
+                    constexpr int K = decltype(kind)::value;      // 2, 4: doublings; 1: product by s
+                    auto step = [&](V v) -> V {
+                        if (K == 1) return R.step(v, f);
+                        v = R.dbl(v);
+                        return (K == 4) ? R.dbl(v) : v;
+                    };
+                    u32 ha = val_hash(RM::bits(xa)), hb = val_hash(RM::bits(xb));
+#pragma unroll BABY_UNROLL
+                    for (int i = 0; i < 8; ++i) {
+                        atomicOr(&filt[__umulhi(ha, nw)], filter_mask(ha));
+                        atomicOr(&filt[__umulhi(hb, nw)], filter_mask(hb));
                         xa = step(xa);
                         xb = step(xb);
+                        ha = val_hash(RM::bits(xa));
+                        hb = val_hash(RM::bits(xb));
+                        unit |= (ha == h1) | (hb == h1);
                     }
-#pragma unroll
-                    for (int i = 0; i < 2 * IB2; ++i) old[i] = tab_claim(T, bf[i] >> 16);
-#pragma unroll
-                    for (int i = 0; i < 2 * IB2; ++i) {
-                        const u32 j = tid * cp + h0 + (i >> 1) + ((i & 1) ? half : 0u);
-                        const u32 bk = bf[i] >> 16, fp = bf[i] & 0xFFFFu;
-                        if (!tab_fill(T, bk, old[i], fp, j)) spill |= insert_walk<NB>(bk, fp, j, BSGS_SPEC_PROBE);
-                    }
-                }
-            };
-            // (FP64 steps keep three double constants live: rounds of two
-            // values per chain keep the loop within 64 registers)
-            auto babies_cp = [&](auto kind) {
-                if (MODE != 2 && half >= IBMAX / 2) babies(kind, std::integral_constant<int, IBMAX / 2>{});
-                else if (half >= IBMAX / 4) babies(kind, std::integral_constant<int, IBMAX / 4>{});
-                else babies(kind, std::integral_constant<int, IBMAX / 8>{});
-            };
-            if (smul == 2) babies_cp(std::integral_constant<int, 2>{});
-            else if (smul == 4) babies_cp(std::integral_constant<int, 4>{});
-            else if constexpr (MODE >= 1) babies_cp(std::integral_constant<int, 1>{});
-            else babies_cp(std::integral_constant<int, 0>{});
-            if (minj != 0xFFFFFFFFu) atomicMin(&s_order, minj);
-            if (spill) s_spill = 1;
-        }
-        __syncthreads();
-        // the last thread (idle in the giant phase unless every thread has a
-        // chunk) claims the prime after next and loads the next prime's job
-        // arguments; both are read after this prime's last barrier
-        if (tid == TPB - 1) {
-            s_claim = slot_of(atomicAdd(work_ctr, 1u));
-            const u32 nx = s_idx[buf ^ 1];
-            if (BATCH && nx != NONE) s_args_next = job_args[hdr[nx].job];
-        }
-        const u32 order = s_order;
-        const u32 Mg = R.hdr.Mg;
-        if (live) {
-            if (order != 0xFFFFFFFFu) rebuild_table<TPB, C, NB>(order);
-            else if (tid == 0 && s_spill) atomicOr(a.err, ERR_HASH_OVERFLOW);
-
-            if (order == 0xFFFFFFFFu) {
-                // ---- giant steps: two independent chains per thread ----
-                // chain A walks q in [q0, q0+h), chain B q in [q0+h, q1), h = Lc/2;
-                // B starts from A's start times S^h (Sh), so the two products of
-                // a step are independent and overlap in the pipeline.  Below
-                // 2^63 the step is Shoup's product by the fixed s^Q' (Sw is its
-                // quotient constant), else the Montgomery product by S.
-                const u32 numk = R.hdr.numk, G = R.hdr.G, Lc = R.hdr.Lc;
-                const u64 S = R.hdr.S, Sw = R.hdr.Sw, Sp = R.hdr.Sp;
-                const double Sd = fp_exact(Sp), Sqd = __longlong_as_double((long long)R.hdr.Sq);
-                if (tid < numk * G) {
-                    // i = tid / G by a float reciprocal: (tid + 1/2) / G lies at
-                    // least 1/(2G) from an integer, and the two roundings err by
-                    // under 2^-22 relative (below 2^-12 * (1024/G) absolute)
-                    const u32 i = (u32)(((float)tid + 0.5f) * __frcp_rn((float)G)), g = tid - i * G;
-                    const u32 q0 = g * Lc;
-                    const u32 q1 = min(q0 + Lc, Mg);
-                    const u32 h = Lc >> 1;
-                    const u32 nA = min(h, q1 - q0), nB = (q1 - q0) - nA;
-                    const u32 m = R.meta[i];
-                    u64 gA, gB;
-                    if (MODE == 2) {
-                        const double a0 = fp_mul(fp_exact(R.tgt[i]), __longlong_as_double((long long)s_Z[g]), pd, pinv);
-                        gA = (u64)__double_as_longlong(a0);
-                        gB = (u64)__double_as_longlong(fp_mul(a0, fp_exact(R.hdr.Sh), pd, pinv));
-                    } else {
-                        gA = mmul(R.tgt[i], s_Z[g], p, q);
-                        gB = mmul(gA, R.hdr.Sh, p, q);
-                    }
-                    auto gstep = [&](u64 v) -> u64 {
-                        if (MODE == 2)
-                            return (u64)__double_as_longlong(fp_mulfix(__longlong_as_double((long long)v), Sd, Sqd, pd));
-                        if (MODE == 1) return shoup_mul(v, Sp, Sw, p);
-                        return mmul(v, S, p, q);
-                    };
-                    // chain B has nA or nA+1 steps, except in a target's last,
-                    // shorter chunk, where it may have fewer or none
-                    const u32 nt = max(nA, nB);
-                    for (u32 t = 0; t < nt; ++t) {
-                        if (t < nA) {
-                            giant_probe<TPB, C, NB>(T, gA, q0 + t, m);
-                            gA = gstep(gA);
+                };
+                const u32 smul = H->smul;
+                if (smul == 2) babies(std::integral_constant<int, 2>{});
+                else if (smul == 4) babies(std::integral_constant<int, 4>{});
+                else babies(std::integral_constant<int, 1>{});
+                if (unit) order_check<MODE>(sl, H, 16 * gt, start[gt]);
+            }
+            if (claimer) ahead = claimed(ahead);
+            group_sync(gid, gs);
+            const u64 *tg = tgt + (size_t)r * KSTRIDE;
+            const u32 order = sl->order;                          // (the first thread resets it for the next pass)
+            if (order == NONE) {
+                // ---- giant steps: items (target i, chunk g), two per thread at a time ----
+                const u32 nitems = H->numk * H->G;
+                const u32 wend = min((seg + 1) * H->rounds * 2 * gs, nitems);
+                const typename RM::Fix f = RM::giant(*H);
+                // a filter pass of giant step t of item w goes on the queue (a lane
+                // past the last item repeats it, and its passes are that item's own)
+                auto pass = [&](V g, u32 w, u32 t) {
+                    if (w >= nitems) return;
+                    const u64 v = RM::bits(g);
+                    const u32 k = atomicAdd(&sl->nq, 1u);
+                    if (k < gs / 4) slice_queue(sl, gs)[k] = make_uint4((u32)v, (u32)(v >> 32), w, t);
+                };
+                for (u32 w = seg * H->rounds * 2 * gs + gt; (w & ~31u) < wend; w += 2 * gs) {
+                    V gA = item_start<MODE>(R, min(w, nitems - 1), H, tb, tg);
+                    const u32 Lc = H->Lc;
+                    if ((w & ~31u) + gs < nitems) {
+                        V gB = item_start<MODE>(R, min(w + gs, nitems - 1), H, tb, tg);
+#pragma unroll GIANT_UNROLL
+                        for (u32 t = 0; t < Lc; ++t) {
+                            const u32 ha = val_hash(RM::bits(gA)), hb = val_hash(RM::bits(gB));
+                            const u32 fa = filt[__umulhi(ha, nw)], fb = filt[__umulhi(hb, nw)];
+                            const V nA = R.step(gA, f), nB = R.step(gB, f);
+                            const bool hitA = (filter_mask(ha) & ~fa) == 0, hitB = (filter_mask(hb) & ~fb) == 0;
+                            if (__any_sync(0xFFFFFFFFu, hitA | hitB)) {
+                                if (hitA) pass(gA, w, t);
+                                if (hitB) pass(gB, w + gs, t);
+                            }
+                            gA = nA;
+                            gB = nB;
                         }
-                        if (t < nB) {
-                            giant_probe<TPB, C, NB>(T, gB, q0 + h + t, m);
-                            gB = gstep(gB);
+                    } else {
+                        for (u32 t = 0; t < Lc; ++t) {
+                            const u32 ha = val_hash(RM::bits(gA));
+                            const u32 fa = filt[__umulhi(ha, nw)];
+                            const V nA = R.step(gA, f);
+                            if ((filter_mask(ha) & ~fa) == 0) pass(gA, w, t);
+                            gA = nA;
                         }
                     }
                 }
             } else {
-                small_order_search<TPB, C, NB>(&R, order);
+                build_index<MODE>(sl, H, gid, gs, gt);
+                small_order_search<MODE>(sl, H, BATCH ? job_args + H->job : &s_args, gs, gt, tg,
+                                         meta + (size_t)r * KSTRIDE);
             }
-            if (tid == 0) {
-                s_baby += min(order, TPB * cp);
-                if (order == 0xFFFFFFFFu) s_giant += (u64)R.hdr.numk * Mg;
-                else s_small += 1;
+            if (claimer) sl->claim = ahead;
+            group_sync(gid, gs);
+            // the queued filter passes, 16 lanes each
+            const u32 nq = sl->nq;
+            if (nq) {
+                build_index<MODE>(sl, H, gid, gs, gt);
+                const BsgsArgs *args = BATCH ? job_args + H->job : &s_args;
+                const unsigned short *mt = meta + (size_t)r * KSTRIDE;
+                if (nq <= gs / 4) {
+                    for (u32 k = gt >> 4; k < nq; k += gs >> 4) {
+                        const uint4 x = slice_queue(sl, gs)[k];
+                        check_pass<MODE>(RM(*H), sl, H, gs, ((u64)x.y << 32) | x.x, x.z, x.w, gt & 15, args, mt);
+                    }
+                } else {
+                    const u32 per = H->rounds * 2 * gs;
+                    giant_unqueued<MODE>(sl, H, gs, gt, seg * per, min((seg + 1) * per, H->numk * H->G), tb, tg, args, mt);
+                }
+                if (gt == 0) atomicAdd(&s_cands, (unsigned long long)nq);
+                group_sync(gid, gs);
             }
+            if (++seg < H->nseg && order == NONE) continue;
+            if (gt == 0) {
+                atomicAdd(&s_baby, (unsigned long long)min(order, 16 * gs));
+                if (order == NONE) atomicAdd(&s_giant, (unsigned long long)H->numk * H->Mg);
+                else atomicAdd(&s_small, 1ull);
+            }
+            seg = 0;
+            ++it;
         }
-        __syncthreads();
     }
+    __syncthreads();
     if (tid == 0) {
         atomicAdd(&a.stats[ST_BABY], s_baby);
         atomicAdd(&a.stats[ST_GIANT], s_giant);
@@ -688,118 +662,82 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB) k_bsgs(BsgsArgs a, const Prim
         atomicAdd(&a.stats[ST_FACTORS], s_facs);
         atomicAdd(&a.stats[ST_HITS], s_dups + s_facs);
     }
-    if (s_abort && tid == 0) {
-        // A record wait gave up.  The CTA stopped before fetching another record,
-        // so the only copy that can still be in flight is the one waited for:
-        // report, then let it land (bounded by the default) before the CTA's
-        // shared memory is released.
-        atomicOr(a.err, ERR_TMA_TIMEOUT);
-        u32 n = 0;
-        while (n < WAIT_BOUND && !mbar_try_wait(&s_bar[pend_buf], pend_par)) ++n;
-    }
 }
 
-template <int G, int MODE, bool BATCH = false>
-static cudaError_t launch_geom(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,
-                              const unsigned short *meta, u32 count, u32 *work_ctr, int sms, cudaStream_t st,
-                              const BsgsArgs *job_args = nullptr, u32 nr = 0, const u32 *prefix = nullptr,
-                              u32 rcap = 0)
+template <int TPB, int MODE, bool BATCH>
+static cudaError_t launch_shape(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,
+                               const unsigned short *meta, const BsgsLists &L, int sms, cudaStream_t st,
+                               const BsgsArgs *job_args)
 {
-    constexpr BsgsGeom g = BSGS_GEOMS[G];
-    auto kern = k_bsgs<g.tpb, g.c, g.nb, MODE, BATCH>;
-    const size_t smem = Smem<g.tpb, g.nb>::bytes();
-    static thread_local int per_sm[32] = {0};            // resident CTAs per SM, per device
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int &occ = per_sm[dev & 31];
-    if (occ == 0) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, g.tpb, smem);
-        if (e != cudaSuccess) return e;
-        if (occ < 1) return cudaErrorInvalidConfiguration;
-    }
-    const u64 want = (u64)sms * (u64)occ;
-    const unsigned grid = (unsigned)((BATCH || want < count) ? want : count);
-    kern<<<grid, g.tpb, smem, st>>>(a, hdr, tabs, tgt, meta, count, work_ctr, job_args, nr, prefix, rcap);
+    auto kern = k_bsgs<TPB, MODE, BATCH>;
+    kern<<<(unsigned)(sms * (1024 / TPB)), TPB, smem_bytes<TPB>(), st>>>(a, hdr, tabs, tgt, meta, L.list, L.stride,
+                                                                        L.ctl, L.ctl + NCLASS, job_args);
     return cudaGetLastError();
 }
 
-template <int G, int MODE>
-static cudaError_t set_smem()
+template <bool BATCH>
+static cudaError_t launch_any(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,
+                              const unsigned short *meta, const BsgsLists &L, int mode, u32 tpb, int sms,
+                              cudaStream_t st, const BsgsArgs *job_args)
 {
-    constexpr BsgsGeom g = BSGS_GEOMS[G];
-    cudaError_t e = cudaFuncSetAttribute(k_bsgs<g.tpb, g.c, g.nb, MODE, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<g.tpb, g.nb>::bytes());
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_bsgs<g.tpb, g.c, g.nb, MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)Smem<g.tpb, g.nb>::bytes());
+    if (tpb == 1024)
+        return mode == 2 ? launch_shape<1024, 2, BATCH>(a, hdr, tabs, tgt, meta, L, sms, st, job_args)
+             : mode == 1 ? launch_shape<1024, 1, BATCH>(a, hdr, tabs, tgt, meta, L, sms, st, job_args)
+                         : launch_shape<1024, 0, BATCH>(a, hdr, tabs, tgt, meta, L, sms, st, job_args);
+    return mode == 2 ? launch_shape<512, 2, BATCH>(a, hdr, tabs, tgt, meta, L, sms, st, job_args)
+         : mode == 1 ? launch_shape<512, 1, BATCH>(a, hdr, tabs, tgt, meta, L, sms, st, job_args)
+                     : launch_shape<512, 0, BATCH>(a, hdr, tabs, tgt, meta, L, sms, st, job_args);
 }
 
-template <int G>
-static size_t smem_of() { return Smem<BSGS_GEOMS[G].tpb, BSGS_GEOMS[G].nb>::bytes(); }
-
-size_t bsgs_smem_bytes(int geom)
-{
-    switch (geom) {
-    case 0: return smem_of<0>();
-    case 1: return smem_of<1>();
-    case 2: return smem_of<2>();
-    case 3: return smem_of<3>();
-    default: return smem_of<4>();
-    }
-}
+size_t bsgs_smem_bytes() { return smem_bytes<1024>(); }
 
 cudaError_t bsgs_prepare()
 {
     cudaError_t e = cudaSuccess;
-    auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-    chk(set_smem<0, 0>()); chk(set_smem<0, 1>()); chk(set_smem<0, 2>());
-    chk(set_smem<1, 0>()); chk(set_smem<1, 1>()); chk(set_smem<1, 2>());
-    chk(set_smem<2, 0>()); chk(set_smem<2, 1>()); chk(set_smem<2, 2>());
-    chk(set_smem<3, 0>()); chk(set_smem<3, 1>()); chk(set_smem<3, 2>());
-    chk(set_smem<4, 0>()); chk(set_smem<4, 1>()); chk(set_smem<4, 2>());
+    auto set = [&](const void *k, size_t bytes) {
+        const cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess) e = r;
+    };
+#define RS_BSGS_SET(TPB, MODE)                                                  \
+    set((const void *)k_bsgs<TPB, MODE, false>, smem_bytes<TPB>());             \
+    set((const void *)k_bsgs<TPB, MODE, true>, smem_bytes<TPB>());
+    RS_BSGS_SET(512, 0) RS_BSGS_SET(512, 1) RS_BSGS_SET(512, 2)
+    RS_BSGS_SET(1024, 0) RS_BSGS_SET(1024, 1) RS_BSGS_SET(1024, 2)
+#undef RS_BSGS_SET
     return e;
 }
 
 cudaError_t launch_bsgs(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,
-                        const unsigned short *meta, u32 count, u32 *work_ctr, u64 pmin, u64 pmax, int geom, int sms,
+                        const unsigned short *meta, const BsgsLists &L, u64 pmin, u64 pmax, int geom, int sms,
                         cudaStream_t st)
 {
-    if (count == 0) return cudaSuccess;
     const u64 TOP = 1ull << 63;
     if (pmin < TOP && pmax > TOP) return cudaErrorInvalidValue;   // the caller splits launches at 2^63
     if (pmin < FP_BOUND && pmax > FP_BOUND) return cudaErrorInvalidValue;   // and at FP_BOUND
+    if (geom < 0 || geom >= NGEOM) return cudaErrorInvalidValue;
     const int mode = (pmax <= FP_BOUND) ? 2 : (pmax <= TOP) ? 1 : 0;
-#define RS_BSGS_CASE(G)                                                                                  \
-    case G:                                                                                              \
-        return mode == 2 ? launch_geom<G, 2>(a, hdr, tabs, tgt, meta, count, work_ctr, sms, st)          \
-             : mode == 1 ? launch_geom<G, 1>(a, hdr, tabs, tgt, meta, count, work_ctr, sms, st)          \
-                         : launch_geom<G, 0>(a, hdr, tabs, tgt, meta, count, work_ctr, sms, st);
-    switch (geom) {
-        RS_BSGS_CASE(0)
-        RS_BSGS_CASE(1)
-        RS_BSGS_CASE(2)
-        RS_BSGS_CASE(3)
-        RS_BSGS_CASE(4)
-    default: return cudaErrorInvalidValue;
-    }
-#undef RS_BSGS_CASE
+    return launch_any<false>(a, hdr, tabs, tgt, meta, L, mode, BSGS_GEOMS[geom].tpb, sms, st, nullptr);
+}
+
+cudaError_t launch_bsgs_batch(const BsgsArgs &a, const BsgsArgs *job_args, const PrimeHdr *hdr, const u64 *tabs,
+                              const u64 *tgt, const unsigned short *meta, const BsgsLists &L, int group, int sms,
+                              cudaStream_t st)
+{
+    return launch_any<true>(a, hdr, tabs, tgt, meta, L, group % 3, group >= 3 ? 1024 : 512, sms, st, job_args);
 }
 
 // prefix[0] = 0, prefix[k+1] = prefix[k] + counter `which` of range slot k
-// (capped at rcap) when it is active and in the (geom, shoup) group -- or, for
-// geom < 0, when it is active -- else + 0.  One block of 256 threads: each
+// (capped at rcap) when it is active, else + 0.  One block of 256 threads: each
 // sums a contiguous run of slots, a block scan offsets the runs.
-__global__ void __launch_bounds__(256) k_batch_prefix(const BatchRange *ranges, u32 nr, int geom, int mode,
-                                                      const u32 *ctrs, u32 rcap, u32 *prefix, int which)
+__global__ void __launch_bounds__(256) k_batch_prefix(const BatchRange *ranges, u32 nr, const u32 *ctrs, u32 rcap,
+                                                      u32 *prefix, int which)
 {
     __shared__ u32 part[256];
     const u32 t = threadIdx.x;
     const u32 per = (nr + 255) / 256;
     const u32 k0 = t * per, k1 = min(k0 + per, nr);
     auto cnt = [&](u32 k) -> u32 {
-        const BatchRange R = ranges[k];
-        const bool in = R.active && (geom < 0 || (R.geom == geom && R.mode == mode));
-        return in ? min(ctrs[k * BR_CTRS + which], rcap) : 0u;
+        return ranges[k].active ? min(ctrs[k * BR_CTRS + which], rcap) : 0u;
     };
     u32 sum = 0;
     for (u32 k = k0; k < k1; ++k) sum += cnt(k);
@@ -819,78 +757,11 @@ __global__ void __launch_bounds__(256) k_batch_prefix(const BatchRange *ranges, 
     }
 }
 
-// Every BSGS group's prefix sums in one launch: block g computes those of
-// group g = 3*geometry + step kind (BatchRange::mode) into prefix + g*(nr+1) and
-// clears the group's work counter.
-__global__ void __launch_bounds__(256) k_batch_group_prefix(const BatchRange *ranges, u32 nr, const u32 *ctrs,
-                                                            u32 rcap, u32 *prefix, u32 *work)
-{
-    __shared__ u32 part[256];
-    const u32 g = blockIdx.x;
-    const int geom = (int)(g / 3), mode = (int)(g % 3);
-    u32 *pf = prefix + (size_t)g * (nr + 1);
-    const u32 t = threadIdx.x;
-    if (t == 0) work[g] = 0;
-    const u32 per = (nr + 255) / 256;
-    const u32 k0 = t * per, k1 = min(k0 + per, nr);
-    auto cnt = [&](u32 k) -> u32 {
-        const BatchRange R = ranges[k];
-        const bool in = R.active && R.geom == geom && R.mode == mode;
-        return in ? min(ctrs[k * BR_CTRS + 1], rcap) : 0u;
-    };
-    u32 sum = 0;
-    for (u32 k = k0; k < k1; ++k) sum += cnt(k);
-    part[t] = sum;
-    __syncthreads();
-    for (u32 o = 1; o < 256; o <<= 1) {
-        const u32 v = (t >= o) ? part[t - o] : 0u;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    u32 acc = part[t] - sum;
-    if (t == 0) pf[0] = 0;
-    for (u32 k = k0; k < k1; ++k) {
-        acc += cnt(k);
-        pf[k + 1] = acc;
-    }
-}
-
-cudaError_t launch_batch_group_prefix(const BatchRange *ranges, u32 nr, const u32 *ctrs, u32 rcap, u32 *prefix,
-                                      u32 *work, cudaStream_t st)
-{
-    k_batch_group_prefix<<<3 * NGEOM, 256, 0, st>>>(ranges, nr, ctrs, rcap, prefix, work);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_batch_prefix_all(const BatchRange *ranges, u32 nr, int which, u32 cap, const u32 *ctrs,
                                     u32 *prefix, cudaStream_t st)
 {
-    k_batch_prefix<<<1, 256, 0, st>>>(ranges, nr, -1, 0, ctrs, cap, prefix, which);
+    k_batch_prefix<<<1, 256, 0, st>>>(ranges, nr, ctrs, cap, prefix, which);
     return cudaGetLastError();
-}
-
-cudaError_t launch_bsgs_batch(const BsgsArgs &a, const BsgsArgs *job_args, const PrimeHdr *hdr, const u64 *tabs,
-                              const u64 *tgt, const unsigned short *meta, u32 nr, const u32 *prefix, u32 rcap,
-                              u32 *work_ctr, int mode, int geom, int sms, cudaStream_t st)
-{
-#define RS_BSGS_BCASE(G)                                                                                           \
-    case G:                                                                                                        \
-        return mode == 2 ? launch_geom<G, 2, true>(a, hdr, tabs, tgt, meta, 0, work_ctr, sms, st, job_args, nr, prefix, \
-                                                   rcap)                                                           \
-             : mode == 1 ? launch_geom<G, 1, true>(a, hdr, tabs, tgt, meta, 0, work_ctr, sms, st, job_args, nr, prefix, \
-                                                   rcap)                                                           \
-                         : launch_geom<G, 0, true>(a, hdr, tabs, tgt, meta, 0, work_ctr, sms, st, job_args, nr, prefix, \
-                                                   rcap);
-    switch (geom) {
-        RS_BSGS_BCASE(0)
-        RS_BSGS_BCASE(1)
-        RS_BSGS_BCASE(2)
-        RS_BSGS_BCASE(3)
-        RS_BSGS_BCASE(4)
-    default: return cudaErrorInvalidValue;
-    }
-#undef RS_BSGS_BCASE
 }
 
 }  // namespace rs

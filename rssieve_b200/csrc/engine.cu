@@ -34,7 +34,7 @@ struct rs_ctx {
     u32 cand_cap = 0;
     u64 *d_primes = nullptr;
     u32 prime_cap = 0;
-    u32 *d_ctrs = nullptr;      // [0] sieve survivors, [1] primes, [2] BSGS work counter, [3] factor count, [4] mid list
+    u32 *d_ctrs = nullptr;      // [0] sieve survivors, [1] primes, [3] factor count, [4] mid list
     u32 *d_err = nullptr;
     u64 *d_stats = nullptr;
     u32 *h_pin = nullptr;       // pinned: ctrs[4], err
@@ -45,6 +45,7 @@ struct rs_ctx {
     u64 *d_tabs = nullptr;
     u64 *d_tgt = nullptr;
     unsigned short *d_meta = nullptr;
+    BsgsLists lists = {nullptr, 0, nullptr};   // the chunk's records by class
     // job
     bool job_loaded = false;
     JobDev h_job;
@@ -128,6 +129,8 @@ extern "C" void rs_ctx_destroy(rs_ctx *c)
     cudaFree(c->d_tabs);
     cudaFree(c->d_tgt);
     cudaFree(c->d_meta);
+    cudaFree(c->lists.list);
+    cudaFree(c->lists.ctl);
     cudaFree(c->d_job);
     if (c->h_pin) cudaFreeHost(c->h_pin);
     for (auto e : c->ev) cudaEventDestroy(e);
@@ -162,6 +165,7 @@ extern "C" int rs_ctx_create(int device, rs_ctx **out)
     c->cand_cap = 1u << 24;
     c->prime_cap = 1u << 24;
     c->chunk_cap = 1u << 17;
+    c->lists.stride = c->chunk_cap;
     if (cudaMalloc(&c->d_sp, sp.size() * 4) != cudaSuccess ||
         cudaMalloc(&c->d_cands, (size_t)c->cand_cap * 8) != cudaSuccess ||
         cudaMalloc(&c->d_mid, (size_t)c->cand_cap * 8) != cudaSuccess ||
@@ -173,6 +177,8 @@ extern "C" int rs_ctx_create(int device, rs_ctx **out)
         cudaMalloc(&c->d_tabs, (size_t)c->chunk_cap * TABS * 8) != cudaSuccess ||
         cudaMalloc(&c->d_tgt, (size_t)c->chunk_cap * KSTRIDE * 8) != cudaSuccess ||
         cudaMalloc(&c->d_meta, (size_t)c->chunk_cap * KSTRIDE * 2) != cudaSuccess ||
+        cudaMalloc(&c->lists.list, (size_t)NCLASS * c->chunk_cap * 4) != cudaSuccess ||
+        cudaMalloc(&c->lists.ctl, 2 * NCLASS * 4) != cudaSuccess ||
         cudaMalloc(&c->d_job, sizeof(JobDev)) != cudaSuccess ||
         cudaMallocHost(&c->h_pin, 64) != cudaSuccess) {
         rs_set_error("device allocation failed");
@@ -183,7 +189,7 @@ extern "C" int rs_ctx_create(int device, rs_ctx **out)
         cudaMemset(c->d_stats, 0, ST_COUNT * 8) != cudaSuccess)
         return fail(RS_ECUDA);
     if (bsgs_prepare() != cudaSuccess) {
-        rs_set_error("BSGS kernel needs %zu B of shared memory", bsgs_smem_bytes(0));
+        rs_set_error("BSGS kernel needs %zu B of shared memory", bsgs_smem_bytes());
         return fail(RS_ECUDA);
     }
     *out = c;
@@ -220,8 +226,9 @@ static u64 job_shape(const rs_ctx *c)
     return job_shape_key(c->h_job.base, c->h_job.kcount, c->h_job.L);
 }
 
-// Starts the per-job tuner: the candidates are the geometries whose model cost
-// is within 2x of the model's best; the first chunks cycle through them.
+// Starts the per-job tuner: the candidates are the largest geometry of each CTA
+// size (a smaller maximum Q only takes classes away) whose model cost is within
+// 2x of the model's best; the first chunks cycle through them.
 static void tune_start(rs_ctx *c)
 {
     c->tune_ncand = 0;
@@ -239,7 +246,9 @@ static void tune_start(rs_ctx *c)
         if (v < best) { best = v; gb = g; }
     }
     for (int g = 0; g < NGEOM; ++g)
-        if (geom_model_cost(g, c->h_job.kcount, c->h_job.L) <= 2.0 * best) c->tune_cand[c->tune_ncand++] = g;
+        if ((g == 0 || BSGS_GEOMS[g].tpb != BSGS_GEOMS[g - 1].tpb) &&
+            geom_model_cost(g, c->h_job.kcount, c->h_job.L) <= 2.0 * best)
+            c->tune_cand[c->tune_ncand++] = g;
     c->geom = gb;
     c->tuning = (c->tune_ncand > 1);
     const int known = tuned_geom_get(c->device, job_shape(c));
@@ -513,12 +522,11 @@ extern "C" int rs_run_range(rs_ctx *c, uint64_t p0, uint64_t p1, rs_counters *de
             // while tuning, full chunks cycle through the candidate geometries
             const int g = (c->tuning && cnt >= 32768) ? c->tune_cand[c->tune_next++ % c->tune_ncand] : c->geom;
             c->chunk_geom[ci] = g;
+            CU(cudaMemsetAsync(c->lists.ctl, 0, 2 * NCLASS * 4, c->stream));
             CU(launch_setup(c->d_job, c->d_primes, first, cnt, c->d_hdr, c->d_aux, c->d_tabs, c->d_tgt, c->d_meta,
-                            c->d_stats, c->d_err, g, c->stream));
-            CU(cudaMemsetAsync(c->d_ctrs + 2, 0, 4, c->stream));
+                            c->lists, c->d_stats, c->d_err, g, c->stream));
             CU(cudaEventRecord(c->ev[2 + 2 * ci], c->stream));
-            CU(launch_bsgs(a, c->d_hdr, c->d_tabs, c->d_tgt, c->d_meta, cnt, c->d_ctrs + 2, p, hi, g, c->sms,
-                           c->stream));
+            CU(launch_bsgs(a, c->d_hdr, c->d_tabs, c->d_tgt, c->d_meta, c->lists, p, hi, g, c->sms, c->stream));
             CU(cudaEventRecord(c->ev[3 + 2 * ci], c->stream));
             c->last_kernel_launches += 3;
             c->last_bsgs_launches += 1;

@@ -67,6 +67,10 @@ RS_DEV u64 msqr_lazy(u64 a, u64 p, u64 q)
     return hi + p - __umul64hi(t, p);
 }
 
+// A double's bits and back.
+RS_DEV double bits_double(u64 b) { return __longlong_as_double((long long)b); }
+RS_DEV u64 double_bits(double d) { return (u64)__double_as_longlong(d); }
+
 // round(a*b + c) - c for the exact product a*b, with c = 1.5*2^52: the fma
 // rounds once into [2^52, 2^53), where the doubles are the integers, so this
 // is a*b rounded to the nearest integer (ties to even) for |a*b| < 2^51, on

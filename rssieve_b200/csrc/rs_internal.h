@@ -20,36 +20,47 @@ constexpr int KMAX = 100;            // sequences per job (inputfile.cpp:356-361
 constexpr int KSTRIDE = 112;         // padded per-prime target stride (16-byte multiple for bulk copies)
 constexpr int TABS = 128;            // u64 power-table entries per prime
 
-// BSGS kernel geometries: Q = tpb * c baby steps per prime, nb buckets of
-// seven slots (load about 0.4), 1024 / tpb CTAs per SM sharing its 228 KB of
-// shared memory.  The giant phase needs tpb >= KMAX (one thread per target).
+// BSGS classes: a prime of class c is searched by a group of 32 << c threads
+// with Q' = 512 << c baby steps.  A geometry bounds the classes that the set-up
+// chooses from, per prime, by its maximum q, and fixes the CTAs: 1024 / tpb of
+// tpb threads share an SM, each working through the classes.
+constexpr int NCLASS = 6;
 struct BsgsGeom {
-    u32 q, tpb, c, nb;
+    u32 q, tpb, classes;     // classes: bit c set when class c may be chosen
 };
 constexpr int NGEOM = 5;
 constexpr BsgsGeom BSGS_GEOMS[NGEOM] = {
-    {16384, 1024, 16, 6144},   // 1 CTA per SM
-    {8192, 512, 16, 2944},     // 2
-    {4096, 256, 16, 1376},     // 4 (with the 2.2 KB record buffers, 1408 buckets would leave room for 3)
-    {2048, 256, 8, 704},       // 4
-    {1024, 128, 8, 352},       // 8
+    {16384, 1024, 0x3D},     // (16 groups of 64 threads would need more than the 15 named barriers)
+    {8192, 512, 0x1F},
+    {4096, 512, 0x0F},
+    {2048, 512, 0x07},
+    {1024, 512, 0x03},
 };
 constexpr int geom_index(u32 q)
 {
     return q == 16384 ? 0 : q == 8192 ? 1 : q == 4096 ? 2 : q == 2048 ? 3 : q == 1024 ? 4 : -1;
 }
 
-// Model cost of one prime for a geometry, in baby-step units: Q baby steps plus
-// the giant steps of the targets that survive the prefilter (about 0.6 of the
-// sequences), each over one class of n modulo the prime's split modulus e
-// (ceil(L/(eQ)) steps, about 0.15 L/Q on average over primes, and at least
-// one), a giant step costing about 1.2 baby steps, and the per-prime fixed
-// work (table clear, barriers) of about 0.15 Q.
+// Model cost of one prime for a geometry, in steps: over primes, the targets
+// that survive the prefilter times their giant steps' n-range shrink the work
+// kcount*L by D, the part of p-1 made of small primes (as far as the split uses
+// it); SPLIT lists ten quantiles of D.  Each prime takes the best class: 1.5 Q'
+// (baby steps and the work per thread that does not depend on the job) plus the
+// giant steps.
 inline double geom_model_cost(int g, u32 kcount, u32 L)
 {
-    const double q = BSGS_GEOMS[g].q;
-    const double m = 0.15 * (double)L / q + 0.5;
-    return 1.15 * q + 1.2 * 0.6 * kcount * (m < 1.0 ? 1.0 : m);
+    constexpr double SPLIT[10] = {2, 2, 4, 6, 8, 12, 20, 36, 64, 120};
+    double sum = 0;
+    for (double d : SPLIT) {
+        double best = 1e300;
+        for (int c = 0; c < NCLASS; ++c) {
+            if (!((BSGS_GEOMS[g].classes >> c) & 1)) continue;
+            const double q = (double)(512 << c), v = 1.5 * q + (double)kcount * (double)L / (d * q);
+            if (v < best) best = v;
+        }
+        sum += best;
+    }
+    return sum / 10;
 }
 inline int geom_model_best(u32 kcount, u32 L)
 {
@@ -66,9 +77,6 @@ inline u64 job_shape_key(u32 base, u32 kcount, u32 L)
 }
 int tuned_geom_get(int device, u64 shape);
 void tuned_geom_put(int device, u64 shape, int geom);
-constexpr int BSGS_MAXPROBE = 64;
-constexpr int BSGS_SPEC_PROBE = 64;         // bucket walk bound while ord(s) is still unknown
-
 constexpr int SETUP_TPB = 256;              // 8 primes (warps) per block
 constexpr int SIEVE_TPB = 512;
 constexpr int SIEVE_WORDS = 4096;           // 2^17 odd numbers per sieve block
@@ -117,26 +125,29 @@ constexpr u64 FP_BOUND = 1ull << 51;
 // The set-up's chi chains (products of two variable factors, fp_mul) run on
 // the FP64 pipe below FP_BOUND as well.
 
+// A prime's record header.  The set-up's first kernels keep Montgomery
+// constants in it; the last one leaves what the search reads, by step kind:
+// below FP_BOUND every residue is a plain one, as the bits of the double that
+// holds it; from there on residues are in Montgomery form unless said otherwise.
 struct PrimeHdr {        // 128 bytes (a 16-byte multiple: copied by TMA bulk copies)
     u64 p;               // 0 = skipped
-    u64 q;               // p^-1 mod 2^64
+    u64 q;               // p^-1 mod 2^64; below FP_BOUND finally the bits of 1/p
     u64 one;             // 2^64 mod p
-    u64 s;               // Montgomery b^e, e = the split modulus (n runs over one class mod e per target)
-    u64 S;               // Montgomery s^Q' (Q' = this prime's baby-step count), for p >= 2^63; below
-                         // FP_BOUND the bits of the double sp/p (FP64 baby steps)
+    u64 s;               // b^e, e = the split modulus (n runs over one class mod e per target)
+    u64 sw;              // floor(sp*2^64/p), for Shoup's products (0 when p >= 2^63); below FP_BOUND finally s/p
+    u64 sp;              // b^e as a plain integer (0 when p >= 2^63)
+    u64 S, Sw, Sp;       // the same for s^Q', Q' = this prime's baby-step count
+    u64 u8;              // s^8: start offset of a thread's second baby chain
     u32 numk;            // surviving targets
     u32 e;               // split modulus, 1..64
-    u32 G, Lc;           // giant phase: G chunks of Lc giant steps
-    u32 smul;            // b^e as an integer when the baby step uses additions, else 0
+    u32 G, Lc;           // giant phase: G chunks of Lc giant steps per target
+    u32 smul;            // b^e as an integer when it is at most 16, else 0 (2 and 4: baby steps by doublings)
     u32 job;             // job index within a batch (0 for a single job)
-    u32 Mg;              // giant steps per target: ceil(ceil(L/e)/Q'), Q' = TPB*cp
-    u32 cp;              // baby steps per thread for this prime (C, C/2 or C/4 of the launch's geometry)
-    u64 Sh;              // Montgomery S^(Lc/2): start of a thread's second giant chain
-    u64 Sw;              // floor(Sp*2^64/p), Sp = s^Q' mod p (plain), for Shoup giant steps; 0 when p >= 2^63
-    u64 ssw;             // floor(sp*2^64/p), sp = s mod p (plain), for Shoup baby steps; 0 when p >= 2^63
-    u64 sp, Sp;          // s and s^Q' as plain residues, the Shoup multipliers (0 when p >= 2^63)
-    u64 u2;              // Montgomery s^(cp/2): start offset of a thread's second baby chain
-    u64 Sq;              // below FP_BOUND: the bits of the double Sp/p (FP64 giant steps); else 0
+    u32 Mg;              // giant steps per target: ceil(ceil(L/e)/Q')
+    u32 cls;             // class: Q' = 512 << cls, 32 << cls threads
+    float rk;            // 1/numk
+    u32 nseg, rounds;    // segments of a long giant phase: rounds of 2 * (32 << cls) items each
+    u32 pad_;
 };
 static_assert(sizeof(PrimeHdr) == 128, "PrimeHdr is copied in 16-byte units");
 
@@ -176,17 +187,25 @@ struct BatchRange {      // device state of one range slot
 constexpr int BR_CTRS = 4;
 // per-job BSGS geometry as the set-up kernels need it
 struct JobGeom {
-    u32 q, c, tpb, pad_;
+    u32 classes;         // classes to choose from (bit c)
+    u32 group;           // a batch's BSGS launch of the job's primes: this (0, or 3 for 1024-thread CTAs)
+                         // plus the step kind (2 FP64, 1 Shoup, 0 Montgomery)
 };
+constexpr int NGROUP = 6;
 inline JobGeom job_geom(int g)
 {
     JobGeom G;
-    G.q = BSGS_GEOMS[g].q;
-    G.c = BSGS_GEOMS[g].c;
-    G.tpb = BSGS_GEOMS[g].tpb;
-    G.pad_ = 0;
+    G.classes = BSGS_GEOMS[g].classes;
+    G.group = BSGS_GEOMS[g].tpb == 1024 ? 3u : 0u;
     return G;
 }
+// One BSGS launch's primes, sorted by class: ctl[c] record indices of class c
+// at list + c*stride; ctl[NCLASS + c] counts those taken (zero at the start).
+struct BsgsLists {
+    u32 *list;
+    u32 stride;
+    u32 *ctl;
+};
 
 // Index i of work spread over nr ranges with prefix sums prefix[0..nr]:
 // the range k with prefix[k] <= i < prefix[k+1] (i < prefix[nr]).
@@ -209,14 +228,16 @@ cudaError_t launch_mr(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *prim
 // holds cand_cap values and *mid_ctr starts at zero
 cudaError_t launch_mr2(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *primes, u32 prime_cap, u32 *prime_ctr,
                        u64 *mid, u32 *mid_ctr, u32 *err, int sms, cudaStream_t st);
+// (lists: NCLASS lists of at least count records; the counts in lists.ctl start at zero)
 cudaError_t launch_setup(const JobDev *job, const u64 *primes, u32 first, u32 count, PrimeHdr *hdr, void *aux, u64 *tabs,
-                         u64 *tgt, unsigned short *meta, u64 *stats, u32 *err, int geom, cudaStream_t st);
+                         u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err, int geom,
+                         cudaStream_t st);
 size_t setup_aux_bytes();
 // every prime of the launch lies in [pmin, pmax), entirely below or entirely at or above 2^63
 cudaError_t launch_bsgs(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,
-                        const unsigned short *meta, u32 count, u32 *work_ctr, u64 pmin, u64 pmax, int geom, int sms,
+                        const unsigned short *meta, const BsgsLists &lists, u64 pmin, u64 pmax, int geom, int sms,
                         cudaStream_t st);
-size_t bsgs_smem_bytes(int geom);
+size_t bsgs_smem_bytes();     // dynamic shared memory of the largest CTA
 cudaError_t bsgs_prepare();   // per device, before the first launch
 cudaError_t launch_mulmod_peak(u64 *out, int blocks, int iters, cudaStream_t st);
 cudaError_t launch_widemul_peak(u64 *out, int blocks, int iters, cudaStream_t st);
@@ -236,22 +257,19 @@ cudaError_t launch_mr_batch2(const u64 *cands, u32 ccap, u64 *primes, u32 rcap, 
                              const u32 *prefix_c, u64 *mid, u32 *mid_r, u32 mid_cap, u32 *mid_ctr, u32 *err, int sms,
                              cudaStream_t st);
 // set-up of the primes of all ranges (prefix_p: prefix sums of their counts;
-// rec_of: room for one record index per prime, nranges * rcap)
+// rec_of: room for one record index per prime, nranges * rcap); group g's lists
+// are lists.list + g*NCLASS*stride with lists.ctl + 2*NCLASS*g, zero at the start
 cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const BatchRange *ranges, const u64 *primes,
                                u32 rcap, const u32 *prefix_p, u32 nranges, PrimeHdr *hdr, void *aux, u64 *tabs,
-                               u64 *tgt, unsigned short *meta, u64 *stats, u32 *err, u32 *rec_of, int sms,
-                               cudaStream_t st);
-// one BSGS launch per (geometry, mode) group g = 3*geometry + mode over range
-// slots [0, nr): prefix + g*(nr+1) (nr+1 entries) counts the primes of the
-// active slots of that group only; work[g] is cleared
-cudaError_t launch_batch_group_prefix(const BatchRange *ranges, u32 nr, const u32 *ctrs, u32 rcap, u32 *prefix,
-                                      u32 *work, cudaStream_t st);
+                               u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err,
+                               u32 *rec_of, int sms, cudaStream_t st);
 // prefix over every active range of counter `which` (0: survivors, 1: primes), each capped at cap
 cudaError_t launch_batch_prefix_all(const BatchRange *ranges, u32 nr, int which, u32 cap, const u32 *ctrs,
                                     u32 *prefix, cudaStream_t st);
+// one launch per group over its own lists
 cudaError_t launch_bsgs_batch(const BsgsArgs &a, const BsgsArgs *job_args, const PrimeHdr *hdr, const u64 *tabs,
-                              const u64 *tgt, const unsigned short *meta, u32 nr, const u32 *prefix, u32 rcap,
-                              u32 *work_ctr, int mode, int geom, int sms, cudaStream_t st);
+                              const u64 *tgt, const unsigned short *meta, const BsgsLists &lists, int group, int sms,
+                              cudaStream_t st);
 
 }  // namespace rs
 

@@ -47,16 +47,14 @@ constexpr u32 SPLIT_MAX = 64;        // largest split modulus e (6 bits of offse
 // copy of the loop keeps the kernels small enough for the instruction cache.
 __device__ __noinline__ u64 mpow_call(u64 x, u64 e, Mont M) { return mpow(x, e, M); }
 
-constexpr int NCP = 3;            // baby steps per thread: C, C/2 or C/4 (index k: C >> k)
-
 struct PrimeAux {        // kernel 1 -> kernel 2 scalars
     u64 r2;              // R^2 mod p
     u64 bm;              // Montgomery b
     u64 xD;              // (p-1)/D: chi(x) = x^xD
     u64 xe;              // eo/e
     u64 hm1;             // Montgomery h^-1, h = chi(b)^xe of order e
-    u64 wr0[NCP];        // per baby-step count Q'_k = tpb*(C >> k): b^(nmin + e(Q'_k - 1)) * R^2 (mod p)
-    u64 S[NCP];          //   and Montgomery s^Q'_k
+    u64 wr0[NCLASS];     // per class, Q'_c = 512 << c: b^(nmin + e(Q'_c - 1)) * R^2 (mod p)
+    u64 S[NCLASS];       //   and Montgomery s^Q'_c
     u32 e;               // split modulus
     u32 flags;           // AUX_* below
 };
@@ -129,12 +127,11 @@ __device__ __forceinline__ u32 small_power(u32 b, u32 e)
 // Per-prime constants of prime p into record t, with the powers that depend
 // on the baby-step count for each of the counts kernel 2 chooses from.
 __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, u64 p, u32 t, u32 jb,
-                                                PrimeHdr *__restrict__ hdr, PrimeAux *__restrict__ aux,
-                                                const JobGeom &gm)
+                                                PrimeHdr *__restrict__ hdr, PrimeAux *__restrict__ aux)
 {
     PrimeHdr H;
-    H.p = 0; H.q = 0; H.one = 0; H.s = 0; H.S = 0; H.numk = 0; H.e = 0; H.G = 0; H.Lc = 0; H.smul = 0; H.job = jb;
-    H.Mg = 0; H.cp = 0; H.Sh = 0; H.Sw = 0; H.ssw = 0; H.sp = 0; H.Sp = 0; H.u2 = 0; H.Sq = 0;
+    H.p = 0; H.q = 0; H.one = 0; H.s = 0; H.sw = 0; H.sp = 0; H.S = 0; H.Sw = 0; H.Sp = 0; H.u8 = 0; H.numk = 0; H.e = 0;
+    H.G = 0; H.Lc = 0; H.smul = 0; H.job = jb; H.Mg = 0; H.cls = 0; H.rk = 0; H.nseg = 0; H.rounds = 0; H.pad_ = 0;
     const Mont M = mont_init(p);
     const u32 b = job->base;
     const u64 bm = to_mont(b, M);
@@ -176,37 +173,36 @@ __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, 
     X.e = e;
     const bool chi_m1 = (xD & 1) != 0;                    // chi(-1) = (-1)^xD
     X.flags = ((chi_m1 && (eo & 1)) ? AUX_NEG_EO : 0u) | ((chi_m1 && (xe & 1)) ? AUX_NEG_XE : 0u);
-    // Q'_k = 2^(m+2-k), m = log2(Q/4): s^(Q'-1) by t <- t^2 * s from s^(2^m - 1).
-    // Below FP_BOUND the powers are FP64 products of plain residues, moved
-    // into Montgomery form (and R^2 form for wr0) at the end.
-    const int m = __ffs((int)(gm.q >> 2)) - 1;
+    // s^(Q'-1) by t <- t^2 * s from s^511, Q' = 512 << c.  Below FP_BOUND the
+    // powers are FP64 products of plain residues, moved into Montgomery form
+    // (and R^2 form for wr0) at the end.
     if (p < FP_BOUND) {
         const double pd = fp_exact(p), pinv = 1.0 / pd;
         const double sd = fp_exact(from_mont(s, M));
         const double bn = fpow_call(fp_exact(b % p), (u64)job->nmin, pd, pinv);
         double tq = 1.0;
-        for (int i = 0; i < m; ++i) tq = fp_mul(fp_mul(tq, tq, pd, pinv), sd, pd, pinv);
-#pragma unroll
-        for (int k = NCP - 1; k >= 0; --k) {              // k = NCP-1: Q/4, then Q/2, Q
-            if (k != NCP - 1) tq = fp_mul(fp_mul(tq, tq, pd, pinv), sd, pd, pinv);
-            X.wr0[k] = mmul(to_mont(fp_int(fp_mul(bn, tq, pd, pinv)), M), M.r2, p, M.q);
-            X.S[k] = to_mont(fp_int(fp_mul(tq, sd, pd, pinv)), M);
+        for (int i = 0; i < 9; ++i) tq = fp_mul(fp_mul(tq, tq, pd, pinv), sd, pd, pinv);
+#pragma unroll 1
+        for (int c = 0; c < NCLASS; ++c) {
+            if (c) tq = fp_mul(fp_mul(tq, tq, pd, pinv), sd, pd, pinv);
+            X.wr0[c] = mmul(to_mont(fp_int(fp_mul(bn, tq, pd, pinv)), M), M.r2, p, M.q);
+            X.S[c] = to_mont(fp_int(fp_mul(tq, sd, pd, pinv)), M);
         }
     } else {
         const u64 bn = mpow_call(bm, (u64)job->nmin, M);
         u64 tq = M.one;
-        for (int i = 0; i < m; ++i) tq = mmul(mmul(tq, tq, p, M.q), s, p, M.q);
-#pragma unroll
-        for (int k = NCP - 1; k >= 0; --k) {              // k = NCP-1: Q/4, then Q/2, Q
-            if (k != NCP - 1) tq = mmul(mmul(tq, tq, p, M.q), s, p, M.q);
-            X.wr0[k] = mmul(mmul(bn, tq, p, M.q), M.r2, p, M.q);
-            X.S[k] = mmul(tq, s, p, M.q);
+        for (int i = 0; i < 9; ++i) tq = mmul(mmul(tq, tq, p, M.q), s, p, M.q);
+#pragma unroll 1
+        for (int c = 0; c < NCLASS; ++c) {
+            if (c) tq = mmul(mmul(tq, tq, p, M.q), s, p, M.q);
+            X.wr0[c] = mmul(mmul(bn, tq, p, M.q), M.r2, p, M.q);
+            X.S[c] = mmul(tq, s, p, M.q);
         }
     }
     H.p = p; H.q = M.q; H.one = M.one; H.s = s; H.e = e;
     if (!(p >> 63)) {                                     // Shoup multiplier of the baby steps below 2^63
         H.sp = from_mont(s, M);
-        H.ssw = shoup_of_mont(s, M.q);
+        H.sw = shoup_of_mont(s, M.q);
     }
     H.smul = small_power(b, e);
     hdr[t] = H;
@@ -222,8 +218,7 @@ __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, 
 template <bool BATCH>
 __global__ void __launch_bounds__(256) k_setup_prime(const JobDev *__restrict__ jobs, const u64 *__restrict__ primes,
                                                      u32 first, u32 count, PrimeHdr *__restrict__ hdr,
-                                                     PrimeAux *__restrict__ aux, JobGeom gm,
-                                                     const JobGeom *__restrict__ geoms,
+                                                     PrimeAux *__restrict__ aux,
                                                      const BatchRange *__restrict__ ranges,
                                                      const u32 *__restrict__ prefix, u32 nr, u32 rcap,
                                                      u32 *__restrict__ rec_of)
@@ -236,36 +231,30 @@ __global__ void __launch_bounds__(256) k_setup_prime(const JobDev *__restrict__ 
             const u32 rec = r * rcap + (i - prefix[r]);
             const u32 jb = ranges[r].job;
             rec_of[i] = rec;
-            setup_prime_one(jobs + jb, primes[rec], rec, jb, hdr, aux, geoms[jb]);
+            setup_prime_one(jobs + jb, primes[rec], rec, jb, hdr, aux);
         }
     } else {
         for (u32 t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += stride)
-            setup_prime_one(jobs, primes[first + t], t, 0, hdr, aux, gm);
+            setup_prime_one(jobs, primes[first + t], t, 0, hdr, aux);
     }
 }
 
-// Baby steps per thread for a prime with nk targets of Le giant-step units
-// each: the index k of the per-thread count C >> k in {C, C/2, C/4} (Q' =
-// tpb*(C >> k) baby steps) that minimises Q' + GIANT_COST * (nk * ceil(Le/Q')
-// giant steps + 2 start products per giant thread).  A prime with a large
-// split modulus has few giant steps per target and takes fewer baby steps.
-// tpb and C are powers of two, so every division is a shift.
-constexpr float GIANT_COST = 0.8f;
-__device__ __forceinline__ u32 choose_cp(const JobGeom &gm, u32 nk, u64 Le)
+// Class for a prime with nk targets of Le giant-step units each: the c among
+// gm.classes that minimises 1.5 Q' + nk*ceil(Le/Q') with Q' = 512 << c, baby
+// steps, the work of the 32 << c threads that does not depend on their steps
+// (clearing the filter, start values; about eight steps each) and giant steps.
+__device__ __forceinline__ u32 choose_class(const JobGeom &gm, u32 nk, u32 Le)
 {
-    u32 best_k = 0;
+    u32 best_c = 0;
     float best = 3.0e38f;
-    const int lq = 31 - __clz(gm.tpb * gm.c);
-    const u32 g0 = gm.tpb / nk;
-    for (u32 k = 0; k < NCP; ++k) {
-        const u64 qp = 1ull << (lq - k);
-        const u64 mg = (Le + qp - 1) >> (lq - k);
-        u64 g = g0 < 1 ? 1 : g0;
-        if (g > mg) g = mg;
-        const float cost = (float)qp + GIANT_COST * ((float)nk * (float)mg + 2.0f * (float)(nk * g));
-        if (cost < best) { best = cost; best_k = k; }
+#pragma unroll
+    for (u32 c = 0; c < NCLASS; ++c) {
+        const u32 lq = 9 + c;
+        const u32 mg = (Le + (1u << lq) - 1) >> lq;
+        const float cost = 1.5f * (float)(1u << lq) + (float)nk * (float)mg;
+        if (((gm.classes >> c) & 1u) && cost < best) { best = cost; best_c = c; }
     }
-    return best_k;
+    return best_c;
 }
 
 // a[r] = x[r]^ex for r < R, the R chains interleaved (the exponent is the same
@@ -526,166 +515,207 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
         return;
     }
     // baby steps for this prime (the giant-step tables follow in kernel 3)
-    const u64 Le = ((u64)job->L + e - 1) / e;
-    const u32 kc = choose_cp(gm, nk, Le);
+    const u32 cls = choose_class(gm, nk, (job->L + e - 1) / e);
     // targets T = -c * k * b^(nmin + off + e(Q'-1)): wt[r] = b^(nmin + e(Q'-1) + r) * R^2
-    const u64 wr0 = X.wr0[kc];
+    const u64 wr0 = X.wr0[cls];
     for (u32 r = lane; r < e; r += 32) wt[r] = mmul(wr0, wt[r], p, M.q);
     __syncwarp();                                          // also orders pass 1's record writes
     for (u32 j = lane; j < nk; j += 32) {
         const u32 m = mg_[j];
         u64 T = mmul(tg[j], wt[m >> 7], p, M.q);
         if (job->c[m & 0x7Fu] == 1) T = mneg(T, p);
+        if (p < FP_BOUND) T = double_bits(fp_exact(from_mont(T, M)));   // the FP64 steps' form
         tg[j] = T;
     }
     if (lane == 0) {
         hdr[w].numk = nk;
-        hdr[w].cp = gm.c >> kc;
+        hdr[w].cls = cls;
     }
 }
 
+// Giant phase of nk targets with Mg giant steps each, over a group of gs
+// threads: items of G chunks of Lc = ceil(Mg/G) steps per target, a round of
+// 2 gs items at a time, `rounds` rounds per segment.  With h half rounds (one
+// item per thread) G = gs*h/nk; of h = 1..8 the one with the least h * (Lc + 3),
+// an odd h counting half a round more (an item's start values cost about three
+// steps, and an odd half round runs one chain per thread instead of two).  A
+// segment is checked for filter passes at its end: the filter passes one value
+// in 2000 that is not there and Q'/p of all values are there, so a segment of
+// `run` steps per chain (48 unless p is small) leaves about a quarter of the
+// queue's room, GS/16 passes; longer giant phases are cut into chunks and
+// segments of that length.  G is at most 1024 (the start tables), and a
+// target's last chunk is never empty.
+__device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float p, u32 &G, u32 &Lc, u32 &nseg, u32 &rounds)
+{
+    const u32 run = (u32)fminf(48.0f, fmaxf(1.0f, 1.0f / (32.0f * (5.0e-4f + 16.0f * (float)gs / p))));
+    u32 best = 0xFFFFFFFFu, hb = 0;
+    for (u32 h = 1; h <= 8; ++h) {
+        u32 g = gs * h / nk;
+        if (g < 1) continue;
+        g = min(min(g, Mg), 1024u);
+        const u32 lc = (Mg + g - 1) / g, cost = (2 * h + (h & 1)) * (lc + 3);
+        if (cost < best) {
+            best = cost;
+            hb = h;
+            Lc = lc;
+        }
+        if (g == Mg) break;                               // one step per item already
+    }
+    if (((hb + 1) >> 1) * Lc > run) Lc = (Mg + min((Mg + run - 1) / run, 1024u) - 1) / min((Mg + run - 1) / run, 1024u);
+    G = (Mg + Lc - 1) / Lc;
+    const u32 total = (nk * G + 2 * gs - 1) / (2 * gs);   // rounds
+    rounds = min(total, max(run / Lc, 1u));
+    nseg = (total + rounds - 1) / rounds;
+}
+
 // Baby- and giant-step tables of record t (one thread): giant steps per target
-// Mg = ceil(ceil(L/e)/Q'), G chunks of Lc steps per target (numk*G <= tpb),
-// A[l] = s^(cp*l), B[l] = s^(32*cp*l) (baby starts), Z1[l] = S^(Lc*l),
-// Z2[l] = S^(32*Lc*l) (giant starts) with S = s^Q', and the Shoup quotient of S.
-// Adds the prime's targets and its search kind to the thread's tallies.
+// Mg = ceil(ceil(L/e)/Q'), G chunks of Lc steps per target, A[l] = s^(16l),
+// B[l] = s^(512l) (baby starts), Z1[l] = S^(Lc*l), Z2[l] = S^(32*Lc*l) (giant
+// starts) with S = s^Q', and the multipliers' quotients, in the form of the
+// prime's step kind (PrimeHdr).  Adds the prime's targets and its search kind
+// to the thread's tallies.  Each table is only as long as the BSGS kernel
+// reads it: A[t % 32] and B[t / 32] for the group's threads t, Z1[g % 32] and
+// Z2[g / 32] for the giant chunks g < G.
 __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u32 t, PrimeHdr *__restrict__ hdr,
                                                const PrimeAux *__restrict__ aux, u64 *__restrict__ tabs,
-                                               const JobGeom &gm, u32 &n_targets, u32 &n_full, u32 &n_split)
+                                               u32 &n_targets, u32 &n_full, u32 &n_split)
 {
     PrimeHdr H = hdr[t];
-    if (H.p == 0) return;
     const u64 p = H.p, q = H.q;
     Mont M;
     M.p = p; M.q = q; M.one = H.one; M.r2 = 0;
-    const u32 e = H.e, cp = H.cp, nk = H.numk;
-    const u32 kc = 31 - __clz(gm.c / cp);
-    const u32 qp = gm.tpb * cp;
-    const u64 Le = ((u64)job->L + e - 1) / e;
-    const u32 Mg = (u32)((Le + qp - 1) / qp);
-    u32 G = gm.tpb / nk;
-    if (G < 1) G = 1;
-    if (G > Mg) G = Mg;
-    const u32 Lc = (Mg + G - 1) / G;
-    G = (Mg + Lc - 1) / Lc;
-    const u64 S = aux[t].S[kc];
-    const u64 Sh = mpow(S, (u64)(Lc >> 1), M);            // start of a thread's second giant chain
-    const u64 z = (Lc & 1) ? mmul(mmul(Sh, Sh, p, q), S, p, q) : mmul(Sh, Sh, p, q);   // S^Lc
-    u64 u2 = H.s;                                          // s^(cp/2) and s^cp, cp a power of two >= 2
-    for (u32 c = cp >> 1; c > 1; c >>= 1) u2 = mmul(u2, u2, p, q);
-    const u64 u = mmul(u2, u2, p, q);
+    const u32 e = H.e, nk = H.numk, gs = 32u << H.cls, lq = 9 + H.cls;
+    const u32 Le = (job->L + e - 1) / e;
+    const u32 Mg = (Le + (1u << lq) - 1) >> lq;
+    u32 G, Lc, nseg, rounds;
+    giant_split(gs, nk, Mg, (float)p, G, Lc, nseg, rounds);
+    const u64 S = aux[t].S[H.cls];
     u64 *tb = tabs + (size_t)t * TABS;
-    // four power tables, two chains at a time, each only as long as the BSGS
-    // kernel reads it: A[t % 32] and B[t / 32] for its threads t < tpb, Z1[g % 32]
-    // and Z2[g / 32] for the giant chunks g < G (the rest of the record's table
-    // space is left as it is).  Below FP_BOUND the BSGS kernel forms its start
-    // values with FP64 products of plain residues, x*y mod p instead of x*y/R:
-    // there Z2, s^(cp/2) and S^(Lc/2) are stored plain, so baby and giant values
-    // alike carry R^2 instead of R; and the tables' own chains run on the FP64
-    // pipe with plain multipliers (an R-form start times plain powers stays in
-    // R-form).  z^32 is needed only when G > 32, and then the Z1 chain has run
-    // all 32 steps.
-    const u32 nb = gm.tpb >> 5, nz1 = min(G, 32u), nz2 = (G + 31) >> 5;
-    const bool fp = (p < FP_BOUND);
-    if (fp) {
-        const double pd = (double)p, pinv = 1.0 / pd;
-        const double up = fp_exact(from_mont(u, M)), zp = fp_exact(from_mont(z, M));
-        double a = fp_exact(M.one), b = a;
-        for (u32 l = 0; l < 32; ++l) {
-            tb[l] = fp_int(a);
-            a = fp_mul(a, up, pd, pinv);
-            if (l < nz1) {
-                tb[64 + l] = fp_int(b);
-                b = fp_mul(b, zp, pd, pinv);
-            }
-        }
-        const double u32p = fp_exact(from_mont(fp_int(a), M));                  // plain u^32
-        const double z32 = (nz2 > 1) ? fp_exact(from_mont(fp_int(b), M)) : 0.0;  // plain z^32
-        a = fp_exact(M.one);
-        b = 1.0;
-        for (u32 l = 0; l < nb; ++l) {
-            tb[32 + l] = fp_int(a);
-            a = fp_mul(a, u32p, pd, pinv);
-            if (l < nz2) {
-                tb[96 + l] = fp_int(b);
-                b = fp_mul(b, z32, pd, pinv);
-            }
-        }
-    } else {
-        u64 a = M.one, b = M.one;
-        for (u32 l = 0; l < 32; ++l) {
-            tb[l] = a;
-            a = mmul(a, u, p, q);
-            if (l < nz1) {
-                tb[64 + l] = b;
-                b = mmul(b, z, p, q);
-            }
-        }
-        const u64 u32p = a, z32 = b;                       // u^32, and z^32 when G > 32
-        a = M.one;
-        b = M.one;
-        for (u32 l = 0; l < nb; ++l) {
-            tb[32 + l] = a;
-            a = mmul(a, u32p, p, q);
-            if (l < nz2) {
-                tb[96 + l] = b;
-                b = mmul(b, z32, p, q);
-            }
-        }
-    }
+    const u32 nb = gs >> 5, nz1 = min(G, 32u), nz2 = (G + 31) >> 5;
     PrimeHdr &h = hdr[t];
     h.G = G;
     h.Lc = Lc;
     h.Mg = Mg;
-    h.S = S;
-    h.Sh = Sh;
-    h.u2 = u2;
-    if (!(p >> 63)) {                                      // Shoup multiplier of the giant steps below 2^63
-        h.Sp = from_mont(S, M);
-        h.Sw = shoup_of_mont(S, q);
-    }
-    if (fp) {                                              // FP64 quotients of the baby and giant multipliers
-        const double pd = (double)p;
-        h.S = (u64)__double_as_longlong((double)H.sp / pd);
-        h.Sq = (u64)__double_as_longlong((double)h.Sp / pd);
-        // the FP64 start values: plain s^(cp/2) and S^(Lc/2), 1/p in the Shoup
-        // quotients' place and R^2 mod p (the value of s^0) in the other
-        h.u2 = from_mont(u2, M);
-        h.Sh = from_mont(Sh, M);
-        h.Sw = (u64)__double_as_longlong(1.0 / pd);
-        h.ssw = aux[t].r2;
+    h.rk = 1.0f / (float)nk;
+    h.nseg = nseg;
+    h.rounds = rounds;
+    // z^32 is needed only when G > 32, and then the Z1 chain has run all 32 steps
+    if (p < FP_BOUND) {
+        const double pd = fp_exact(p), pinv = 1.0 / pd;
+        auto mul = [&](double x, double y) { return fp_mul(x, y, pd, pinv); };
+        const u64 s1 = H.sp, S1 = from_mont(S, M);        // plain
+        const double sd = fp_exact(s1), Sd = fp_exact(S1);
+        double u8 = mul(sd, sd);
+        u8 = mul(u8, u8);
+        u8 = mul(u8, u8);
+        const double u = mul(u8, u8), z = fpow_call(Sd, Lc, pd, pinv);
+        double a = 1.0, b = 1.0;
+        for (u32 l = 0; l < 32; ++l) {
+            tb[l] = double_bits(a);
+            a = mul(a, u);
+            if (l < nz1) {
+                tb[64 + l] = double_bits(b);
+                b = mul(b, z);
+            }
+        }
+        const double u32p = a, z32 = b;
+        a = 1.0;
+        b = 1.0;
+        for (u32 l = 0; l < max(nb, nz2); ++l) {
+            if (l < nb) {
+                tb[32 + l] = double_bits(a);
+                a = mul(a, u32p);
+            }
+            if (l < nz2) {
+                tb[96 + l] = double_bits(b);
+                b = mul(b, z32);
+            }
+        }
+        h.q = double_bits(pinv);
+        h.s = double_bits(sd);
+        h.sw = double_bits(sd / pd);
+        h.S = double_bits(Sd);
+        h.Sw = double_bits(Sd / pd);
+        h.u8 = double_bits(u8);
+    } else {
+        auto mul = [&](u64 x, u64 y) { return mmul(x, y, p, q); };
+        u64 u8 = mul(H.s, H.s);
+        u8 = mul(u8, u8);
+        u8 = mul(u8, u8);
+        const u64 u = mul(u8, u8), z = mpow(S, (u64)Lc, M);
+        u64 a = M.one, b = M.one;
+        for (u32 l = 0; l < 32; ++l) {
+            tb[l] = a;
+            a = mul(a, u);
+            if (l < nz1) {
+                tb[64 + l] = b;
+                b = mul(b, z);
+            }
+        }
+        const u64 u32p = a, z32 = b;
+        a = M.one;
+        b = M.one;
+        for (u32 l = 0; l < max(nb, nz2); ++l) {
+            if (l < nb) {
+                tb[32 + l] = a;
+                a = mul(a, u32p);
+            }
+            if (l < nz2) {
+                tb[96 + l] = b;
+                b = mul(b, z32);
+            }
+        }
+        h.S = S;
+        h.u8 = u8;
+        if (!(p >> 63)) {                                  // Shoup multiplier of the giant steps below 2^63
+            h.Sp = from_mont(S, M);
+            h.Sw = shoup_of_mont(S, q);
+        }
     }
     n_targets += nk;
     if (e >= 2) ++n_split; else ++n_full;
 }
 
-// Kernel 3: one thread per prime (indexing as kernel 1).
+// Kernel 3: one thread per prime (indexing as kernel 1); then the record's index
+// goes on the list of its class (BATCH: of its job's group and step kind).
 template <bool BATCH>
 __global__ void __launch_bounds__(256) k_setup_tabs(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
                                                     const PrimeAux *__restrict__ aux, u32 count,
-                                                    u64 *__restrict__ tabs, u64 *__restrict__ stats, JobGeom gm,
+                                                    u64 *__restrict__ tabs, u64 *__restrict__ stats,
+                                                    u32 *__restrict__ lists, u32 list_stride, u32 *list_ctl,
                                                     const JobGeom *__restrict__ geoms,
                                                     const u32 *__restrict__ prefix, u32 nr,
                                                     const u32 *__restrict__ rec_of)
 {
     const u32 stride = gridDim.x * blockDim.x;
+    const u32 lane = threadIdx.x & 31;
+    const u32 total = BATCH ? prefix[nr] : count;
     u32 nt = 0, nf = 0, ns = 0;
-    if constexpr (BATCH) {
-        const u32 total = prefix[nr];
-        for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-            const u32 rec = rec_of[i];
-            const u32 jb = hdr[rec].job;
-            setup_tabs_one(jobs + jb, rec, hdr, aux, tabs, geoms[jb], nt, nf, ns);
+    // i0 is uniform over the warp, so that the list claims below stay whole
+    for (u32 i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < total; i0 += stride) {
+        const u32 i = i0 + lane;
+        const u32 rec = (i < total) ? (BATCH ? rec_of[i] : i) : 0;
+        const bool live = i < total && hdr[rec].p != 0;
+        u32 key = 0xFFFFFFFFu;                             // list of the record: group * NCLASS + class
+        if (live) {
+            const u32 jb = BATCH ? hdr[rec].job : 0;
+            setup_tabs_one(jobs + jb, rec, hdr, aux, tabs, nt, nf, ns);
+            const u64 p = hdr[rec].p;
+            const u32 g = BATCH ? geoms[jb].group + (p < FP_BOUND ? 2u : (p >> 63) ? 0u : 1u) : 0u;
+            key = g * NCLASS + hdr[rec].cls;
         }
-    } else {
-        for (u32 t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += stride)
-            setup_tabs_one(jobs, t, hdr, aux, tabs, gm, nt, nf, ns);
+        const u32 same = __match_any_sync(0xFFFFFFFFu, key);
+        const u32 lead = __ffs((int)same) - 1;
+        u32 base = 0;
+        if (live && lane == lead) base = atomicAdd(&list_ctl[(key / NCLASS) * 2 * NCLASS + key % NCLASS], __popc(same));
+        base = __shfl_sync(0xFFFFFFFFu, base, lead);
+        if (live) lists[(size_t)key * list_stride + base + __popc(same & ((1u << lane) - 1))] = rec;
     }
     // one atomic per warp and counter
     nt = __reduce_add_sync(0xFFFFFFFFu, nt);
     nf = __reduce_add_sync(0xFFFFFFFFu, nf);
     ns = __reduce_add_sync(0xFFFFFFFFu, ns);
-    if ((threadIdx.x & 31) == 0) {
+    if (lane == 0) {
         if (nt) atomicAdd(&stats[ST_TARGETS], (u64)nt);
         if (nf) atomicAdd(&stats[ST_FULL], (u64)nf);
         if (ns) atomicAdd(&stats[ST_PARITY], (u64)ns);
@@ -725,12 +755,13 @@ __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restri
 }
 
 cudaError_t launch_setup(const JobDev *job, const u64 *primes, u32 first, u32 count, PrimeHdr *hdr, void *aux, u64 *tabs,
-                         u64 *tgt, unsigned short *meta, u64 *stats, u32 *err, int geom, cudaStream_t st)
+                         u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err, int geom,
+                         cudaStream_t st)
 {
     if (count == 0) return cudaSuccess;
     const JobGeom gm = job_geom(geom);
-    k_setup_prime<false><<<(count + 255) / 256, 256, 0, st>>>(job, primes, first, count, hdr, (PrimeAux *)aux, gm,
-                                                              nullptr, nullptr, nullptr, 0, 0, nullptr);
+    k_setup_prime<false><<<(count + 255) / 256, 256, 0, st>>>(job, primes, first, count, hdr, (PrimeAux *)aux, nullptr,
+                                                              nullptr, 0, 0, nullptr);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const u32 wpb = SETUP_TPB / 32;
@@ -738,28 +769,29 @@ cudaError_t launch_setup(const JobDev *job, const u64 *primes, u32 first, u32 co
                                                                    meta, stats, err, gm, nullptr, nullptr, 0, nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_setup_tabs<false><<<(count + 255) / 256, 256, 0, st>>>(job, hdr, (const PrimeAux *)aux, count, tabs, stats, gm,
-                                                             nullptr, nullptr, 0, nullptr);
+    k_setup_tabs<false><<<(count + 255) / 256, 256, 0, st>>>(job, hdr, (const PrimeAux *)aux, count, tabs, stats,
+                                                             lists.list, lists.stride, lists.ctl, nullptr, nullptr, 0,
+                                                             nullptr);
     return cudaGetLastError();
 }
 
 cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const BatchRange *ranges, const u64 *primes,
                                u32 rcap, const u32 *prefix_p, u32 nranges, PrimeHdr *hdr, void *aux, u64 *tabs,
-                               u64 *tgt, unsigned short *meta, u64 *stats, u32 *err, u32 *rec_of, int sms,
-                               cudaStream_t st)
+                               u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err,
+                               u32 *rec_of, int sms, cudaStream_t st)
 {
     JobGeom gm{};
     // full-device grids; the kernels stride over the primes of every range
-    k_setup_prime<true><<<sms * 4, 256, 0, st>>>(jobs, primes, 0, 0, hdr, (PrimeAux *)aux, gm, geoms, ranges,
-                                                 prefix_p, nranges, rcap, rec_of);
+    k_setup_prime<true><<<sms * 4, 256, 0, st>>>(jobs, primes, 0, 0, hdr, (PrimeAux *)aux, ranges, prefix_p, nranges,
+                                                 rcap, rec_of);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_setup_k<true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, tgt, meta, stats, err,
                                                    gm, geoms, prefix_p, nranges, rec_of);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_setup_tabs<true><<<sms * 4, 256, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, stats, gm, geoms,
-                                                prefix_p, nranges, rec_of);
+    k_setup_tabs<true><<<sms * 4, 256, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, stats, lists.list,
+                                                lists.stride, lists.ctl, geoms, prefix_p, nranges, rec_of);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,66 @@
+"""The search kernel at the edges of its classes, segments and filter queue.
+
+A prime is searched by a group of 32 << c threads with 512 << c baby steps
+(class c), its giant phase dealt as items of several rounds and, when long, cut
+into segments.  Every case compares eliminated terms, bitmap and duplicates
+with the brute-force oracle: whole numbers, equal or not.
+"""
+import numpy as np
+import pytest
+
+from rssieve_b200 import workloads as W
+from tests.conftest import oracle_job
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # kcount, base, n-range, p0, width, Q (0: chosen)
+    (1, 2, 40_000, 3, 30_000, 0),                     # orders from 1 to beyond the largest Q'
+    (100, 2, 40_000, 500, 2_000, 1024),               # p just above Q': most filter passes true, the queue overflows
+    (100, 3, 60_000, 60_000, 4_000, 1024),            # the same with p past the largest class
+    (2, 2, 3_000_000, 1_000_000, 2_000, 1024),        # few targets, many chunks: second-level start powers, segments
+    (1, 10, 2_000_000, 20_000_000, 20_000, 0),        # one target: G up to its limit
+    (100, 2, 1_500_000, 50_000_000, 4_000, 1024),     # segments of many rounds
+    (33, 5, 700_001, 10_000_000, 12_000, 0),          # items past the last one in a round
+    (64, 6, 1_000, 100_000, 20_000, 0),               # n-range shorter than one giant step
+    (100, 2, 900_000, 3_000_000, 4_000, 16384),       # 1024-thread CTAs
+]
+
+
+@pytest.mark.parametrize("kcount,base,width,p0,pw,q", CASES)
+def test_search_matches_brute_force(sieve, oracle, kcount, base, width, p0, pw, q):
+    job = W.small_job(90 + kcount + base, kcount=kcount, base=base, nmin=1001, nmax=1000 + width, keep=0.2, kmax=1 << 24)
+    sieve.set_baby_steps(q)
+    try:
+        sieve.load(W.seqs_of(job))
+        cnt = sieve.run(p0, p0 + pw)
+        fac, bm = sieve.factors(), sieve.bitmap()
+    finally:
+        sieve.set_baby_steps(0)
+    plist = oracle.primes(p0, p0 + pw)
+    ofac, odups, obm = oracle.brute(oracle_job(oracle, job), plist, ref_skip=True)
+    assert cnt["primes"] == len(plist)
+    assert oracle.term_set(fac) == oracle.term_set(ofac)
+    assert np.array_equal(bm, obm)
+    assert cnt["dups"] == odups
+
+
+@pytest.mark.parametrize("p0", [(1 << 45) + 7, (1 << 51) - 2_000, (1 << 57) + 11, (1 << 62) - 5_000, (1 << 63) + 3])
+@pytest.mark.parametrize("kcount,width", [(1, 50_000), (40, 400_000)])
+def test_planted_factors_in_every_step_kind(sieve, oracle, p0, kcount, width):
+    """Primes of each step kind (FP64, Shoup, Montgomery, and a window across
+    2^51): every sequence gets a k that one prime of the window divides a term of."""
+    rng = np.random.default_rng(p0 % 1000 + kcount)
+    plist = oracle.primes(p0, p0 + 3_000)
+    nmin, ks, cs, want = 10_001, [], [], set()
+    for i in range(kcount):
+        p, c, n = int(rng.choice(plist)), 1 if i % 2 else -1, nmin + int(rng.integers(0, width))
+        ks.append(-c * pow(2, -n, p) % p)
+        cs.append(c)
+        want.add((i, n))
+    job = W.job_dict(2, ks, cs, nmin, nmin + width - 1, W.random_bitmap(kcount, nmin, nmin + width - 1, 1.0, 1))
+    sieve.load(W.seqs_of(job))
+    sieve.run(p0, p0 + 3_000)
+    got = oracle.term_set(sieve.factors())
+    # a term may be hit by chance as well: at most width * kcount * primes / p, far below one
+    assert want == got
