@@ -493,8 +493,7 @@ static int batch_round(rs_batch *b)
     BCU(launch_batch_prefix_all(b->d_ranges, R, 1, RCAP, b->d_ctrs, b->d_prefix_p, st));
     BCU(cudaMemsetAsync(b->lists.ctl, 0, (size_t)NGROUP * 2 * NCLASS * 4, st));
     BCU(launch_setup_batch(b->d_jobs, b->d_geoms, b->d_ranges, b->d_primes, RCAP, b->d_prefix_p, R, b->d_hdr,
-                           b->d_aux, b->d_tabs, b->d_tgt, b->d_meta, b->lists, b->d_stats, b->d_err, b->d_rec_of,
-                           b->sms, st));
+                           b->d_aux, b->d_tabs, b->d_tgt, b->d_meta, b->lists, b->d_stats, b->d_rec_of, b->sms, st));
     BsgsArgs a;
     memset(&a, 0, sizeof a);
     a.stats = b->d_stats;

@@ -77,7 +77,7 @@ inline u64 job_shape_key(u32 base, u32 kcount, u32 L)
 }
 int tuned_geom_get(int device, u64 shape);
 void tuned_geom_put(int device, u64 shape, int geom);
-constexpr int SETUP_TPB = 256;              // 8 primes (warps) per block
+constexpr int SETUP_TPB = 256;              // 8 warps per block
 constexpr int SIEVE_TPB = 512;
 constexpr int SIEVE_WORDS = 4096;           // 2^17 odd numbers per sieve block
 constexpr u64 MR_BOUND = 4295098369ULL;     // 65537^2: below it the sieve by all primes < 2^16 is exact
@@ -89,7 +89,6 @@ constexpr u32 ERR_HASH_OVERFLOW = 4u;       // a bucket chain exceeded BSGS_MAXP
 constexpr u32 ERR_FACTOR_OVERFLOW = 8u;     // factor buffer full (cannot happen: sized to the bitmap)
 constexpr u32 ERR_TMA_TIMEOUT = 16u;        // a bulk copy did not complete within the wait bound
 constexpr u32 ERR_SIEVE_TABLE = 32u;        // the sieving-prime table is missing (does not start with 3)
-constexpr u32 ERR_SETUP_CLASS = 64u;        // a target passed the residue test but no class of n matched (cannot happen)
 
 // statistics counters (u64)
 enum Stat {
@@ -122,20 +121,18 @@ struct JobDev {
 // mont.cuh): residues are exact integers in doubles, and a product by a fixed
 // multiplier w takes its quotient from the double w/p.
 constexpr u64 FP_BOUND = 1ull << 51;
-// The set-up's chi chains (products of two variable factors, fp_mul) run on
-// the FP64 pipe below FP_BOUND as well.
+// The set-up runs on the FP64 pipe below FP_BOUND as well.
 
-// A prime's record header.  The set-up's first kernels keep Montgomery
-// constants in it; the last one leaves what the search reads, by step kind:
-// below FP_BOUND every residue is a plain one, as the bits of the double that
-// holds it; from there on residues are in Montgomery form unless said otherwise.
+// A prime's record header.  Residues are held by step kind: below FP_BOUND each is
+// a plain one, as the bits of the double that holds it; from there on residues are
+// in Montgomery form unless said otherwise.
 struct PrimeHdr {        // 128 bytes (a 16-byte multiple: copied by TMA bulk copies)
     u64 p;               // 0 = skipped
-    u64 q;               // p^-1 mod 2^64; below FP_BOUND finally the bits of 1/p
-    u64 one;             // 2^64 mod p
+    u64 q;               // p^-1 mod 2^64; below FP_BOUND the bits of 1/p
+    u64 one;             // 1
     u64 s;               // b^e, e = the split modulus (n runs over one class mod e per target)
-    u64 sw;              // floor(sp*2^64/p), for Shoup's products (0 when p >= 2^63); below FP_BOUND finally s/p
-    u64 sp;              // b^e as a plain integer (0 when p >= 2^63)
+    u64 sw;              // floor(sp*2^64/p), for Shoup's products (0 when p >= 2^63); below FP_BOUND s/p
+    u64 sp;              // b^e as a plain integer for FP_BOUND <= p < 2^63, else 0
     u64 S, Sw, Sp;       // the same for s^Q', Q' = this prime's baby-step count
     u64 u8;              // s^8: start offset of a thread's second baby chain
     u32 numk;            // surviving targets
@@ -228,10 +225,11 @@ cudaError_t launch_mr(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *prim
 // holds cand_cap values and *mid_ctr starts at zero
 cudaError_t launch_mr2(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *primes, u32 prime_cap, u32 *prime_ctr,
                        u64 *mid, u32 *mid_ctr, u32 *err, int sms, cudaStream_t st);
-// (lists: NCLASS lists of at least count records; the counts in lists.ctl start at zero)
-cudaError_t launch_setup(const JobDev *job, const u64 *primes, u32 first, u32 count, PrimeHdr *hdr, void *aux, u64 *tabs,
-                         u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err, int geom,
-                         cudaStream_t st);
+// (lists: NCLASS lists of at least count records; the counts in lists.ctl start at
+// zero; the primes lie below pmax, entirely on one side of FP_BOUND)
+cudaError_t launch_setup(const JobDev *job, u32 kcount, const u64 *primes, u32 first, u32 count, u64 pmax, PrimeHdr *hdr,
+                         void *aux, u64 *tabs, u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats,
+                         int geom, cudaStream_t st);
 size_t setup_aux_bytes();
 // every prime of the launch lies in [pmin, pmax), entirely below or entirely at or above 2^63
 cudaError_t launch_bsgs(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,
@@ -261,8 +259,8 @@ cudaError_t launch_mr_batch2(const u64 *cands, u32 ccap, u64 *primes, u32 rcap, 
 // are lists.list + g*NCLASS*stride with lists.ctl + 2*NCLASS*g, zero at the start
 cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const BatchRange *ranges, const u64 *primes,
                                u32 rcap, const u32 *prefix_p, u32 nranges, PrimeHdr *hdr, void *aux, u64 *tabs,
-                               u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err,
-                               u32 *rec_of, int sms, cudaStream_t st);
+                               u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *rec_of, int sms,
+                               cudaStream_t st);
 // prefix over every active range of counter `which` (0: survivors, 1: primes), each capped at cap
 cudaError_t launch_batch_prefix_all(const BatchRange *ranges, u32 nr, int which, u32 cap, const u32 *ctrs,
                                     u32 *prefix, cudaStream_t st);

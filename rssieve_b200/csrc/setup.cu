@@ -21,7 +21,9 @@
 // generated by chi(b), of order eo (the reference's filters are the cases
 // d | D of this), and (2) n mod e is fixed, for every divisor e of eo, by the
 // discrete logarithm of h = chi(b)^(eo/e) -- a table of e values.  e is the
-// largest divisor of eo up to 64.  Every n the reference finds satisfies both,
+// largest divisor of eo up to 64.  Both take one power per sequence, z = k^E with
+// E = (p-1)/D * eo/e: the logarithm of (-c)^E / z to the base h exists exactly
+// when (chi(-c)/chi(k))^eo = 1, the groups being cyclic.  Every n the reference finds satisfies both,
 // so the eliminated terms are the same, while each sequence's giant steps
 // shrink from L/Q to L/(e*Q) (e = 2 is the reference's parity case; at the
 // 2^50 p-range of the 100-sequence job e averages well above 2).
@@ -29,9 +31,9 @@
 // every sequence as setup.cl:156-162,205-208 do.
 //
 // Kernel 1 (one thread per prime) does the per-prime scalars; kernel 2 (one
-// warp per prime, lanes over k) classifies the sequences, chooses the prime's
-// baby-step count Q' (the launch's Q, Q/2 or Q/4: fewer baby steps when the
-// split modulus leaves few giant steps) and writes the compacted targets;
+// warp per prime, lanes over k; with 16 sequences or fewer, 4 to 16 lanes per
+// prime) classifies the sequences, chooses the prime's class, i.e. its baby-step
+// count Q', and writes the compacted targets;
 // kernel 3 (one thread per prime) writes the giant-step split and the baby-
 // and giant-step start tables.  Per-prime work that is the same for every
 // sequence runs one prime per thread, where it costs 1/32 of the issue slots
@@ -39,78 +41,182 @@
 #include "mont.cuh"
 #include "rs_internal.h"
 
+#include <type_traits>
+#include <utility>
+
 namespace rs {
 
-constexpr u32 SPLIT_MAX = 64;        // largest split modulus e (6 bits of offset per target)
+constexpr u32 SPLIT_MAX = 64;        // largest split modulus e (at most 512: 9 bits of offset per target)
+static_assert(SPLIT_MAX <= 512 && SPLIT_MAX % 32 == 0, "offsets and tables of powers");
 
-// mpow out of line, for the per-prime powers off the kernels' main path: one
-// copy of the loop keeps the kernels small enough for the instruction cache.
-__device__ __noinline__ u64 mpow_call(u64 x, u64 e, Mont M) { return mpow(x, e, M); }
+// The primes whose powers make up D, the smooth part of p-1.
+constexpr u32 SMOOTH[] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61};
+constexpr int NSMOOTH = sizeof(SMOOTH) / sizeof(SMOOTH[0]);
+static_assert(NSMOOTH <= 64, "a prime's smooth factors are a 64-bit mask");
 
-struct PrimeAux {        // kernel 1 -> kernel 2 scalars
-    u64 r2;              // R^2 mod p
-    u64 bm;              // Montgomery b
-    u64 xD;              // (p-1)/D: chi(x) = x^xD
-    u64 xe;              // eo/e
-    u64 hm1;             // Montgomery h^-1, h = chi(b)^xe of order e
-    u64 wr0[NCLASS];     // per class, Q'_c = 512 << c: b^(nmin + e(Q'_c - 1)) * R^2 (mod p)
-    u64 S[NCLASS];       //   and Montgomery s^Q'_c
-    u32 e;               // split modulus
-    u32 flags;           // AUX_* below
+struct PrimeAux {        // kernel 1 -> kernels 2 and 3; residues in the step kind's form (PrimeHdr)
+    u64 E;               // the classes' exponent: z = k^E has order dividing e times the index filtered on
+    u64 r2;              // R^2 mod p (p >= FP_BOUND)
+    u64 b;               // b
+    u64 hm1;             // h^-1, h = b^E of order e
+    u64 wr0[NCLASS];     // per class, Q'_c = 512 << c: b^(nmin + e(Q'_c - 1))
+    u64 S[NCLASS];       //   and s^Q'_c
 };
-constexpr u32 AUX_NEG_EO = 1u;   // chi(-1)^eo = -1: for c = +1 the membership test wants z^eo == -1
-constexpr u32 AUX_NEG_XE = 2u;   // chi(-1)^xe = -1: for c = +1 the class search wants z1*h^r == -1
 
-// Moves every factor L of x into D (L a compile-time prime): applied for each
-// prime up to 61, it leaves D = the 61-smooth part of p-1 and x = (p-1)/D.
-template <u32 L>
-__device__ __forceinline__ void strip(u64 &x, u64 &D)
-{
-    while (x % L == 0) { x /= L; D *= L; }
-}
-
-// Order of g in the group of D-th roots of unity (D 61-smooth): remove the
-// prime factor L from eo while g^(eo/L) is still 1.
-template <u32 L>
-__device__ __forceinline__ void order_step(u64 &eo, u64 g, const Mont &M)
-{
-    while (eo % L == 0 && mpow_call(g, eo / L, M) == M.one) eo /= L;
-}
-
-// x^e mod p on the FP64 pipe (p < FP_BOUND), plain residues held exactly in
-// doubles, pinv = 1/p; e may be 0.  Out of line like mpow_call.
-__device__ __noinline__ double fpow_call(double x, u64 e, double p, double pinv)
-{
-    if (e == 0) return 1.0;
-    double a = x;
-    for (int bit = 62 - __clzll(e); bit >= 0; --bit) {
-        a = fp_mul(a, a, p, pinv);
-        if ((e >> bit) & 1) a = fp_mul(a, x, p, pinv);
+// ---- arithmetic of the set-up: plain residues in doubles below FP_BOUND, else
+// Montgomery residues ----
+template <bool FP>
+struct Field;
+template <>
+struct Field<true> {
+    typedef double V;
+    double p, pinv;
+    __device__ __forceinline__ explicit Field(u64 pi) : p(fp_exact(pi)) { pinv = 1.0 / p; }
+    __device__ __forceinline__ Field(const PrimeHdr &h, const PrimeAux &) : p(fp_exact(h.p)), pinv(bits_double(h.q)) {}
+    static __device__ __forceinline__ V val(u64 b) { return bits_double(b); }
+    static __device__ __forceinline__ u64 bits(V v) { return double_bits(v); }
+    __device__ __forceinline__ V one() const { return 1.0; }
+    __device__ __forceinline__ V of_int(u64 x) const { return fp_exact(x); }        // x < p
+    __device__ __forceinline__ V mul(V a, V b) const { return fp_mul(a, b, p, pinv); }
+    __device__ __forceinline__ V neg(V a) const { return p - a; }                  // a != 0
+    // products inside a power: any signed residue in (-p, p)
+    static constexpr bool lazy = true;
+    template <bool LAZY> __device__ __forceinline__ V pmul(V a, V b) const { return fp_mul_signed(a, b, p, pinv); }
+    template <bool LAZY> __device__ __forceinline__ V psqr(V a) const { return fp_mul_signed(a, a, p, pinv); }
+    template <bool LAZY> __device__ __forceinline__ V pend(V a) const { return (a < 0.0) ? a + p : a; }
+};
+template <>
+struct Field<false> {
+    typedef u64 V;
+    Mont M;
+    bool lazy;           // p < 2^62: products inside a power stay in [0, 2p)
+    __device__ __forceinline__ explicit Field(u64 pi) : M(mont_init(pi)), lazy(pi >> 62 == 0) {}
+    __device__ __forceinline__ Field(const PrimeHdr &h, const PrimeAux &x) : lazy(h.p >> 62 == 0)
+    {
+        M.p = h.p; M.q = h.q; M.one = h.one; M.r2 = x.r2;
     }
-    return a;
-}
+    static __device__ __forceinline__ V val(u64 b) { return b; }
+    static __device__ __forceinline__ u64 bits(V v) { return v; }
+    __device__ __forceinline__ V one() const { return M.one; }
+    __device__ __forceinline__ V of_int(u64 x) const { return to_mont(x, M); }
+    __device__ __forceinline__ V mul(V a, V b) const { return mmul(a, b, M.p, M.q); }
+    __device__ __forceinline__ V neg(V a) const { return M.p - a; }
+    template <bool LAZY> __device__ __forceinline__ V pmul(V a, V b) const
+    {
+        return LAZY ? mmul_lazy(a, b, M.p, M.q) : mmul(a, b, M.p, M.q);
+    }
+    template <bool LAZY> __device__ __forceinline__ V psqr(V a) const
+    {
+        return LAZY ? msqr_lazy(a, M.p, M.q) : mmul(a, a, M.p, M.q);
+    }
+    template <bool LAZY> __device__ __forceinline__ V pend(V a) const { return LAZY ? mred(a, M.p) : a; }
+};
 
-// order_step for a plain g below FP_BOUND, by FP64 powers.
-template <u32 L>
-__device__ __forceinline__ void order_step_fp(u64 &eo, double g, double p, double pinv)
+// x^e, every lane its own e (0 or more): two bits of e at a time, the digit's
+// power (1, x, x^2, x^3) chosen by selects, so lanes do not diverge on their
+// bits: 1.5 products per bit.  Out of line: one copy keeps the kernels small
+// enough for the instruction cache.
+template <bool FP, bool LAZY>
+__device__ __forceinline__ typename Field<FP>::V power_as(const Field<FP> &F, typename Field<FP>::V x, u64 e)
 {
-    while (eo % L == 0 && fpow_call(g, eo / L, p, pinv) == 1.0) eo /= L;
+    typedef typename Field<FP>::V V;
+    const V one = F.one(), x2 = F.template psqr<LAZY>(x), x3 = F.template pmul<LAZY>(x2, x);
+    int i = (63 - __clzll(e)) & ~1;
+    auto digit = [&]() -> V {
+        const u32 d = (u32)(e >> i) & 3u;
+        const V lo = (d & 1) ? x : one, hi = (d & 1) ? x3 : x2;
+        return (d & 2) ? hi : lo;
+    };
+    V a = digit();
+    for (i -= 2; i >= 0; i -= 2) {
+        a = F.template psqr<LAZY>(F.template psqr<LAZY>(a));
+        a = F.template pmul<LAZY>(a, digit());
+    }
+    return F.template pend<LAZY>(a);
+}
+template <bool FP>
+__device__ __noinline__ typename Field<FP>::V power(const Field<FP> F, typename Field<FP>::V x, u64 e)
+{
+    if (e == 0) return F.one();
+    return (FP || F.lazy) ? power_as<FP, true>(F, x, e) : power_as<FP, false>(F, x, e);
 }
 
-// Largest divisor of eo that is at most SPLIT_MAX (by 32-bit remainders when
-// eo fits in 32 bits, the usual case, and from the largest candidate down).
+// Divides every factor L out of x, D taking them; returns whether there was one.
+template <u32 L>
+__device__ __forceinline__ bool strip(u64 &x, u64 &D)
+{
+    if (x % L != 0) return false;
+    do { x /= L; D *= L; } while (x % L == 0);
+    return true;
+}
+// The same for x < 2^52 held in a double: q = x/L rounded; x - q*L, exact in the
+// fma, is zero exactly when L divides x (and then q is the quotient).
+template <u32 L>
+__device__ __forceinline__ bool strip_fp(double &x, double &D)
+{
+    double q = fp_round_prod(x, 1.0 / L);
+    if (fma(-q, (double)L, x) != 0.0) return false;
+    do {
+        x = q;
+        D *= (double)L;
+        q = fp_round_prod(x, 1.0 / L);
+    } while (fma(-q, (double)L, x) == 0.0);
+    return true;
+}
+// every SMOOTH prime but 2, whose index is 0; bit i of the result: SMOOTH[i] divides
+template <size_t... I>
+__device__ __forceinline__ u64 strip_all(u64 &x, u64 &D, std::index_sequence<I...>)
+{
+    u64 m = 0;
+    ((m |= strip<SMOOTH[I + 1]>(x, D) ? 1ull << (I + 1) : 0ull), ...);
+    return m;
+}
+template <size_t... I>
+__device__ __forceinline__ u64 strip_all_fp(double &x, double &D, std::index_sequence<I...>)
+{
+    u64 m = 0;
+    ((m |= strip_fp<SMOOTH[I + 1]>(x, D) ? 1ull << (I + 1) : 0ull), ...);
+    return m;
+}
+
+// SMOOTH and the reciprocals of 1..SPLIT_MAX as tables
+struct SetupTables {
+    u32 smooth[NSMOOTH];
+    double inv[SPLIT_MAX + 1];
+};
+constexpr SetupTables make_tables()
+{
+    SetupTables t{};
+    for (int i = 0; i < NSMOOTH; ++i) t.smooth[i] = SMOOTH[i];
+    for (u32 d = 1; d <= SPLIT_MAX; ++d) t.inv[d] = 1.0 / (double)d;
+    return t;
+}
+__constant__ SetupTables c_tab = make_tables();
+
+// x with every factor l removed
+__device__ __forceinline__ u64 without(u64 x, u32 l)
+{
+    if (x >> 32) {
+        while (x % l == 0) x /= l;
+        return x;
+    }
+    u32 y = (u32)x;
+    while (y % l == 0) y /= l;
+    return y;
+}
+
+// Largest divisor of eo that is at most SPLIT_MAX.
 __device__ __forceinline__ u32 split_modulus(u64 eo)
 {
-    if (eo >> 32) {
-        for (u32 d = SPLIT_MAX; d > 1; --d)
-            if (eo % d == 0) return d;
-        return 1;
+    if (eo <= SPLIT_MAX) return (u32)eo;
+    u32 d = SPLIT_MAX;
+    if (eo >> 52) {
+        while (eo % d != 0) --d;
+        return d;
     }
-    const u32 e32 = (u32)eo;
-#pragma unroll
-    for (u32 d = SPLIT_MAX; d > 1; --d)
-        if (e32 % d == 0) return d;
-    return 1;
+    const double x = fp_exact(eo);
+    while (fma(-fp_round_prod(x, c_tab.inv[d]), (double)d, x) != 0.0) --d;
+    return d;
 }
 
 // b^e as an integer when it is at most 16 (baby steps by additions), else 0.
@@ -124,99 +230,109 @@ __device__ __forceinline__ u32 small_power(u32 b, u32 e)
     return (u32)v;
 }
 
-// Per-prime constants of prime p into record t, with the powers that depend
-// on the baby-step count for each of the counts kernel 2 chooses from.
+// Per-prime constants of prime p into record t, with the powers that depend on
+// the baby-step count for each of the classes kernel 2 chooses from.
+template <bool FP>
 __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, u64 p, u32 t, u32 jb,
                                                 PrimeHdr *__restrict__ hdr, PrimeAux *__restrict__ aux)
 {
-    PrimeHdr H;
-    H.p = 0; H.q = 0; H.one = 0; H.s = 0; H.sw = 0; H.sp = 0; H.S = 0; H.Sw = 0; H.Sp = 0; H.u8 = 0; H.numk = 0; H.e = 0;
-    H.G = 0; H.Lc = 0; H.smul = 0; H.job = jb; H.Mg = 0; H.cls = 0; H.rk = 0; H.nseg = 0; H.rounds = 0; H.pad_ = 0;
-    const Mont M = mont_init(p);
+    typedef Field<FP> F;
+    typedef typename F::V V;
     const u32 b = job->base;
-    const u64 bm = to_mont(b, M);
-    if (bm == 0) { hdr[t] = H; return; }                 // p | b: no term is divisible by p
-    // D = 61-smooth part of p-1, xD = (p-1)/D
-    u64 xD = p - 1, D = 1;
-    strip<2>(xD, D);  strip<3>(xD, D);  strip<5>(xD, D);  strip<7>(xD, D);  strip<11>(xD, D);
-    strip<13>(xD, D); strip<17>(xD, D); strip<19>(xD, D); strip<23>(xD, D); strip<29>(xD, D);
-    strip<31>(xD, D); strip<37>(xD, D); strip<41>(xD, D); strip<43>(xD, D); strip<47>(xD, D);
-    strip<53>(xD, D); strip<59>(xD, D); strip<61>(xD, D);
-    u64 gb, eo = D;                                       // chi(b), of order eo | D
-    if (p < FP_BOUND) {                                   // the power and the order on the FP64 pipe
-        const double pd = fp_exact(p), pinv = 1.0 / pd;
-        const double g = fpow_call(fp_exact(b % p), xD, pd, pinv);
-        order_step_fp<2>(eo, g, pd, pinv);  order_step_fp<3>(eo, g, pd, pinv);  order_step_fp<5>(eo, g, pd, pinv);
-        order_step_fp<7>(eo, g, pd, pinv);  order_step_fp<11>(eo, g, pd, pinv); order_step_fp<13>(eo, g, pd, pinv);
-        order_step_fp<17>(eo, g, pd, pinv); order_step_fp<19>(eo, g, pd, pinv); order_step_fp<23>(eo, g, pd, pinv);
-        order_step_fp<29>(eo, g, pd, pinv); order_step_fp<31>(eo, g, pd, pinv); order_step_fp<37>(eo, g, pd, pinv);
-        order_step_fp<41>(eo, g, pd, pinv); order_step_fp<43>(eo, g, pd, pinv); order_step_fp<47>(eo, g, pd, pinv);
-        order_step_fp<53>(eo, g, pd, pinv); order_step_fp<59>(eo, g, pd, pinv); order_step_fp<61>(eo, g, pd, pinv);
-        gb = to_mont(fp_int(g), M);
+    const u64 bp = (b < p) ? b : b % p;
+    if (bp == 0) {                                        // p | b: no term is divisible by p
+        hdr[t].p = 0;
+        return;
+    }
+    const F f(p);
+    const V bv = f.of_int(bp);
+    // D = smooth part of p-1, x = (p-1)/D, mask: its primes
+    const int v2 = __ffsll((long long)(p - 1)) - 1;
+    u64 x = (p - 1) >> v2, D = 1ull << v2, mask;
+    if constexpr (FP) {
+        double xd = fp_exact(x), Dd = 1.0;
+        mask = strip_all_fp(xd, Dd, std::make_index_sequence<NSMOOTH - 1>());
+        x = fp_int(xd);
+        D *= fp_int(Dd);
     } else {
-        gb = mpow(bm, xD, M);
-        order_step<2>(eo, gb, M);  order_step<3>(eo, gb, M);  order_step<5>(eo, gb, M);  order_step<7>(eo, gb, M);
-        order_step<11>(eo, gb, M); order_step<13>(eo, gb, M); order_step<17>(eo, gb, M); order_step<19>(eo, gb, M);
-        order_step<23>(eo, gb, M); order_step<29>(eo, gb, M); order_step<31>(eo, gb, M); order_step<37>(eo, gb, M);
-        order_step<41>(eo, gb, M); order_step<43>(eo, gb, M); order_step<47>(eo, gb, M); order_step<53>(eo, gb, M);
-        order_step<59>(eo, gb, M); order_step<61>(eo, gb, M);
+        mask = strip_all(x, D, std::make_index_sequence<NSMOOTH - 1>());
+    }
+    mask |= 1;                                            // p is odd
+    // chi(b) = b^x and its order eo | D, one prime of D at a time: the power by
+    // D without that prime has the order's part of it
+    const V g = power<FP>(f, bv, x);
+    const u64 one = F::bits(f.one());
+    u64 eo = 1;
+    while (mask) {
+        const u32 l = c_tab.smooth[__ffsll((long long)mask) - 1];
+        mask &= mask - 1;
+        V y = power<FP>(f, g, without(D, l));
+        for (int i = 0; i < 64 && F::bits(y) != one; ++i) {
+            y = power<FP>(f, y, l);
+            eo *= l;
+        }
     }
     const u32 e = split_modulus(eo);
     const u64 xe = eo / e;
-    const u64 s = mpow_call(bm, e, M);
+    PrimeHdr H;
     PrimeAux X;
-    X.r2 = M.r2;
-    X.bm = bm;
-    X.xD = xD;
-    X.xe = xe;
-    X.hm1 = mpow_call(mpow_call(gb, xe, M), (u64)(e - 1), M);
-    X.e = e;
-    const bool chi_m1 = (xD & 1) != 0;                    // chi(-1) = (-1)^xD
-    X.flags = ((chi_m1 && (eo & 1)) ? AUX_NEG_EO : 0u) | ((chi_m1 && (xe & 1)) ? AUX_NEG_XE : 0u);
-    // s^(Q'-1) by t <- t^2 * s from s^511, Q' = 512 << c.  Below FP_BOUND the
-    // powers are FP64 products of plain residues, moved into Montgomery form
-    // (and R^2 form for wr0) at the end.
-    if (p < FP_BOUND) {
-        const double pd = fp_exact(p), pinv = 1.0 / pd;
-        const double sd = fp_exact(from_mont(s, M));
-        const double bn = fpow_call(fp_exact(b % p), (u64)job->nmin, pd, pinv);
-        double tq = 1.0;
-        for (int i = 0; i < 9; ++i) tq = fp_mul(fp_mul(tq, tq, pd, pinv), sd, pd, pinv);
+    X.E = x * xe;
+    X.b = F::bits(bv);
+    X.hm1 = F::bits(power<FP>(f, g, xe * (e - 1)));
+    const V s = power<FP>(f, bv, e);
+    // s^(Q'-1) by t <- t^2 * s from s^511, Q' = 512 << c
+    const V bn = power<FP>(f, bv, job->nmin);
+    V tq = power<FP>(f, s, 511);
 #pragma unroll 1
-        for (int c = 0; c < NCLASS; ++c) {
-            if (c) tq = fp_mul(fp_mul(tq, tq, pd, pinv), sd, pd, pinv);
-            X.wr0[c] = mmul(to_mont(fp_int(fp_mul(bn, tq, pd, pinv)), M), M.r2, p, M.q);
-            X.S[c] = to_mont(fp_int(fp_mul(tq, sd, pd, pinv)), M);
-        }
+    for (int c = 0; c < NCLASS; ++c) {
+        if (c) tq = f.mul(f.mul(tq, tq), s);
+        X.wr0[c] = F::bits(f.mul(bn, tq));
+        X.S[c] = F::bits(f.mul(tq, s));
+    }
+    H.p = p;
+    H.s = F::bits(s);
+    H.S = 0; H.Sw = 0; H.Sp = 0; H.u8 = 0;
+    if constexpr (FP) {
+        X.r2 = 0;
+        H.q = double_bits(f.pinv);
+        H.one = double_bits(1.0);
+        H.sw = double_bits(s / f.p);
+        H.sp = 0;
     } else {
-        const u64 bn = mpow_call(bm, (u64)job->nmin, M);
-        u64 tq = M.one;
-        for (int i = 0; i < 9; ++i) tq = mmul(mmul(tq, tq, p, M.q), s, p, M.q);
-#pragma unroll 1
-        for (int c = 0; c < NCLASS; ++c) {
-            if (c) tq = mmul(mmul(tq, tq, p, M.q), s, p, M.q);
-            X.wr0[c] = mmul(mmul(bn, tq, p, M.q), M.r2, p, M.q);
-            X.S[c] = mmul(tq, s, p, M.q);
+        X.r2 = f.M.r2;
+        H.q = f.M.q;
+        H.one = f.M.one;
+        H.sw = 0; H.sp = 0;
+        if (!(p >> 63)) {                                 // Shoup multiplier of the baby steps below 2^63
+            H.sp = from_mont(s, f.M);
+            H.sw = shoup_of_mont(s, f.M.q);
         }
     }
-    H.p = p; H.q = M.q; H.one = M.one; H.s = s; H.e = e;
-    if (!(p >> 63)) {                                     // Shoup multiplier of the baby steps below 2^63
-        H.sp = from_mont(s, M);
-        H.sw = shoup_of_mont(s, M.q);
-    }
+    H.numk = 0; H.e = e; H.G = 0; H.Lc = 0; H.job = jb; H.Mg = 0; H.cls = 0;
     H.smul = small_power(b, e);
+    H.rk = 0; H.nseg = 0; H.rounds = 0; H.pad_ = 0;
     hdr[t] = H;
     aux[t] = X;
 }
 
+// Which primes a launch holds: all at or above FP_BOUND, all below, or (batch
+// rounds) both.
+enum Kind { INT_PRIMES = 0, FP_PRIMES = 1, ANY_PRIMES = 2 };
 
 // Kernel 1.  Single job: primes[first, first+count) into records [0, count).
 // Batch (BATCH): the primes of every range as one index space (prefix: prefix
 // sums of the ranges' prime counts); prime i of range r is record r*rcap + i,
 // with its job's sequences.  rec_of[i] keeps that record index, so kernels 2
 // and 3 need no search over the prefix sums.
-template <bool BATCH>
-__global__ void __launch_bounds__(256) k_setup_prime(const JobDev *__restrict__ jobs, const u64 *__restrict__ primes,
+template <int KIND>
+__device__ __forceinline__ void setup_prime_any(const JobDev *__restrict__ job, u64 p, u32 t, u32 jb,
+                                                PrimeHdr *__restrict__ hdr, PrimeAux *__restrict__ aux)
+{
+    if (KIND == FP_PRIMES || (KIND == ANY_PRIMES && p < FP_BOUND)) setup_prime_one<true>(job, p, t, jb, hdr, aux);
+    else setup_prime_one<false>(job, p, t, jb, hdr, aux);
+}
+template <int KIND>
+__global__ void __launch_bounds__(128) k_setup_prime(const JobDev *__restrict__ jobs, const u64 *__restrict__ primes,
                                                      u32 first, u32 count, PrimeHdr *__restrict__ hdr,
                                                      PrimeAux *__restrict__ aux,
                                                      const BatchRange *__restrict__ ranges,
@@ -224,18 +340,18 @@ __global__ void __launch_bounds__(256) k_setup_prime(const JobDev *__restrict__ 
                                                      u32 *__restrict__ rec_of)
 {
     const u32 stride = gridDim.x * blockDim.x;
-    if constexpr (BATCH) {
+    if constexpr (KIND == ANY_PRIMES) {
         const u32 total = prefix[nr];
         for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
             const u32 r = prefix_find(prefix, nr, i);
             const u32 rec = r * rcap + (i - prefix[r]);
             const u32 jb = ranges[r].job;
             rec_of[i] = rec;
-            setup_prime_one(jobs + jb, primes[rec], rec, jb, hdr, aux);
+            setup_prime_any<KIND>(jobs + jb, primes[rec], rec, jb, hdr, aux);
         }
     } else {
         for (u32 t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += stride)
-            setup_prime_one(jobs, primes[first + t], t, 0, hdr, aux);
+            setup_prime_any<KIND>(jobs, primes[first + t], t, 0, hdr, aux);
     }
 }
 
@@ -257,277 +373,276 @@ __device__ __forceinline__ u32 choose_class(const JobGeom &gm, u32 nk, u32 Le)
     return best_c;
 }
 
-// a[r] = x[r]^ex for r < R, the R chains interleaved (the exponent is the same
-// for every lane and chain, so the loop is uniform over the warp); ex >= 1.
-// LAZY (p < 2^62): the chains stay in [0, 2p) without per-product corrections.
-template <int R, bool LAZY>
-__device__ __forceinline__ void mpow_multi(u64 (&a)[4], const u64 (&x)[4], u64 ex, const Mont &M)
+// a[r] = x[r]^ex for r < R, the chains interleaved.  UNIFORM: ex (>= 1) is the
+// same for every lane, so the loop branches on it: a sliding window of two bits,
+// 1.33 products per bit.  Else as power().
+template <bool FP, int R, bool UNIFORM, bool LAZY>
+__device__ __forceinline__ void power_chains_as(const Field<FP> &F, typename Field<FP>::V (&a)[2],
+                                                const typename Field<FP>::V (&x)[2], u64 ex)
 {
-    auto mul = [&](u64 u, u64 v) { return LAZY ? mmul_lazy(u, v, M.p, M.q) : mmul(u, v, M.p, M.q); };
+    typedef typename Field<FP>::V V;
+    V x2[2], x3[2];
 #pragma unroll
-    for (int r = 0; r < R; ++r) a[r] = x[r];
-    for (int bit = 62 - __clzll(ex); bit >= 0; --bit) {
+    for (int r = 0; r < R; ++r) {
+        x2[r] = F.template psqr<LAZY>(x[r]);
+        x3[r] = F.template pmul<LAZY>(x2[r], x[r]);
+    }
+    if constexpr (UNIFORM) {
+        int i = 63 - __clzll(ex);
+        const bool two = i > 0 && ((ex >> (i - 1)) & 1);
 #pragma unroll
-        for (int r = 0; r < R; ++r) a[r] = LAZY ? msqr_lazy(a[r], M.p, M.q) : mmul(a[r], a[r], M.p, M.q);
-        if ((ex >> bit) & 1) {
+        for (int r = 0; r < R; ++r) a[r] = two ? x3[r] : x[r];
+        i -= two ? 2 : 1;
+        while (i >= 0) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) a[r] = mul(a[r], x[r]);
+            for (int r = 0; r < R; ++r) a[r] = F.template psqr<LAZY>(a[r]);
+            if ((ex >> i) & 1) {
+                if (i > 0 && ((ex >> (i - 1)) & 1)) {
+                    --i;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) a[r] = F.template pmul<LAZY>(F.template psqr<LAZY>(a[r]), x3[r]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) a[r] = F.template pmul<LAZY>(a[r], x[r]);
+                }
+            }
+            --i;
+        }
+    } else {
+        const V one = F.one();
+        int i = (63 - __clzll(ex)) & ~1;
+        auto digit = [&](int r) -> V {
+            const u32 d = (u32)(ex >> i) & 3u;
+            const V lo = (d & 1) ? x[r] : one, hi = (d & 1) ? x3[r] : x2[r];
+            return (d & 2) ? hi : lo;
+        };
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[r] = digit(r);
+        for (i -= 2; i >= 0; i -= 2) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                a[r] = F.template pmul<LAZY>(F.template psqr<LAZY>(F.template psqr<LAZY>(a[r])), digit(r));
         }
     }
-    if (LAZY) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) a[r] = mred(a[r], M.p);
-    }
+    for (int r = 0; r < R; ++r) a[r] = F.template pend<LAZY>(a[r]);
+}
+// (Two chains per lane: four would not fit 64 registers.  Issue and the FP64 pipe
+// bound the FP64 form: 100 sequences near 2^50 take 5.2 ns per prime at 73% issue,
+// FP64 58% busy; 7.8 with an exponentiation per sequence to D alone, a second one
+// for the rest of the order, and Montgomery conversions around both.)
+template <bool FP, int R, bool UNIFORM>
+__device__ __forceinline__ void power_chains(const Field<FP> &F, typename Field<FP>::V (&a)[2],
+                                             const typename Field<FP>::V (&x)[2], u64 ex)
+{
+    if (FP || F.lazy) power_chains_as<FP, R, UNIFORM, true>(F, a, x, ex);
+    else power_chains_as<FP, R, UNIFORM, false>(F, a, x, ex);
 }
 
-template <bool LAZY>
-__device__ __forceinline__ void mpow_lanes(u32 R, u64 (&a)[4], const u64 (&x)[4], u64 ex, const Mont &M)
+// Shared memory of a sub-warp of GL lanes in kernel 2: the values h^(-r), r <
+// min(e, TAB), the class lookup over them (open addressing, r + 1 in a 16-bit
+// slot, 0: empty), powers of b, and the targets' parts until the baby-step count
+// is known.
+template <u32 GL>
+struct KScratch {
+    static constexpr u32 KM = GL == 32 ? 128 : GL;       // sequences
+    static constexpr u32 TAB = GL == 4 ? 32 : 64, CLS_SLOTS = 2 * TAB;
+    u64 hv[TAB];
+    u64 part[KM];
+    u64 b1[GL == 32 ? 32 : 1], b2[GL == 32 ? 16 : 1];
+    unsigned short slot[CLS_SLOTS];
+    unsigned short meta[KM];
+};
+
+__device__ __forceinline__ u32 cls_hash(u64 v, u32 mask)
 {
-    if (R == 1) mpow_multi<1, LAZY>(a, x, ex, M);
-    else if (R == 2) mpow_multi<2, LAZY>(a, x, ex, M);
-    else if (R == 3) mpow_multi<3, LAZY>(a, x, ex, M);
-    else mpow_multi<4, LAZY>(a, x, ex, M);
+    return ((((u32)v ^ (u32)(v >> 32)) * 0x9E3779B1u) >> 20) & mask;
 }
 
-// The chains of mpow_multi on the FP64 pipe (p < FP_BOUND): plain residues
-// held exactly in doubles, products by fp_mul_signed, so the chains run in
-// signed residues in (-p, p) and are made canonical once at the end.
-template <int R>
-__device__ __forceinline__ void fpow_multi(double (&a)[4], const double (&x)[4], u64 ex, double pd, double pinv)
+// Sequence classes, targets and baby-step count of record w, by GL lanes (lane l
+// of them) of a warp; live: the record exists and is not skipped.  GL = 32: up to
+// 128 sequences, four rounds of lanes; GL < 32: at most GL sequences, 32/GL
+// primes side by side in a warp.  Called by the whole warp.
+template <bool FP, u32 GL>
+__device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 w, u32 l, bool live,
+                                            PrimeHdr *__restrict__ hdr, const PrimeAux *__restrict__ aux,
+                                            u64 *__restrict__ tgt, unsigned short *__restrict__ meta,
+                                            u64 *__restrict__ stats, const JobGeom &gm, KScratch<GL> &sc)
 {
-#pragma unroll
-    for (int r = 0; r < R; ++r) a[r] = x[r];
-    for (int bit = 62 - __clzll(ex); bit >= 0; --bit) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) a[r] = fp_mul_signed(a[r], a[r], pd, pinv);
-        if ((ex >> bit) & 1) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) a[r] = fp_mul_signed(a[r], x[r], pd, pinv);
+    typedef Field<FP> F;
+    typedef typename F::V V;
+    const u32 lane = threadIdx.x & 31;
+    const u32 sub = lane & ~(GL - 1);                      // the sub-warp's first lane
+    const u32 gmask = GL == 32 ? 0xFFFFFFFFu : ((1u << (GL & 31)) - 1u) << sub;
+    const PrimeAux &X = aux[w];
+    const F f(hdr[w], X);
+    const u64 p = hdr[w].p;
+    const u32 K = job->kcount, e = hdr[w].e;
+    const u64 E = X.E;
+    // class table: lane l forms h^(-l) by a multiplicative scan over the GL lanes,
+    // then every GL-th value from there by products with h^(-GL)
+    constexpr u32 TAB = KScratch<GL>::TAB, CLS_SLOTS = KScratch<GL>::CLS_SLOTS, smask = CLS_SLOTS - 1;
+    const u32 ne = min(e, TAB);
+    V hT = f.one();                                        // h^(-TAB), for e > TAB
+    __syncwarp();                                          // the previous prime's readers are done
+    for (u32 i = l; i < CLS_SLOTS / 2; i += GL) reinterpret_cast<u32 *>(sc.slot)[i] = 0;
+    {
+        const V hm1 = F::val(X.hm1);
+        V hv = (l == 0) ? f.one() : hm1;
+#pragma unroll 1
+        for (u32 o = 1; o < GL; o <<= 1) {
+            const V hu = F::val(__shfl_up_sync(0xFFFFFFFFu, F::bits(hv), o, GL));
+            const V m = f.mul(hv, hu);
+            hv = (l >= o) ? m : hv;
+        }
+        const V hG = f.mul(F::val(__shfl_sync(0xFFFFFFFFu, F::bits(hv), GL - 1, GL)), hm1);
+        if (SPLIT_MAX > TAB) {
+            hT = hG;
+#pragma unroll 1
+            for (u32 n = GL; n < TAB; n *= 2) hT = f.mul(hT, hT);
+        }
+        __syncwarp();
+        // (sub-warps of different e stay together: every lane loops until the last is done)
+        for (u32 r = l; __any_sync(0xFFFFFFFFu, live && r < ne); r += GL) {
+            const u64 v = F::bits(hv);
+            bool pend = live && r < ne;
+            if (pend) sc.hv[r] = v;
+            u32 s = cls_hash(v, smask);
+            while (__any_sync(0xFFFFFFFFu, pend)) {
+                if (pend && sc.slot[s] == 0) sc.slot[s] = (unsigned short)(r + 1);
+                __syncwarp();
+                if (pend) {
+                    if (sc.slot[s] == r + 1) pend = false;
+                    else s = (s + 1) & smask;
+                }
+                __syncwarp();
+            }
+            hv = f.mul(hv, hG);
         }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) a[r] = (a[r] < 0.0) ? a[r] + pd : a[r];
-}
-
-// z = chi(k_i) = k_i^xD in Montgomery form for the lane's sequences
-// i = lane + 32r < K, into zs[i].  (Out of line, with the caller's state
-// saved once per prime instead of spilled, it measured 3-6% slower.)
-// Below FP_BOUND the chains run on the FP64 pipe two at a time (four
-// interleaved chains would not fit the kernel's 64 registers), as a rolled
-// loop over pairs of rounds so that one copy of the chain code serves them.
-__device__ __forceinline__ void chi_of_ks(const JobDev *__restrict__ job, u32 lane, u32 K, const Mont M, u64 xD,
-                                          u64 *zs)
-{
-    const u64 p = M.p;
-    const u32 R = (K + 31) / 32;
-    if (p < FP_BOUND) {
-        const double pd = fp_exact(p), pinv = 1.0 / pd;
+    if constexpr (GL == 32) {                              // b^l, and b^(32 j) for e > 32
+        const V b1 = F::val(X.b);
+        V bv = (lane == 0) ? f.one() : b1;
+#pragma unroll 1
+        for (u32 o = 1; o < 32; o <<= 1) {
+            const V bu = F::val(__shfl_up_sync(0xFFFFFFFFu, F::bits(bv), o));
+            const V m = f.mul(bv, bu);
+            bv = (lane >= o) ? m : bv;
+        }
+        sc.b1[lane] = F::bits(bv);
+        if (e > 32) {
+            const V b32 = f.mul(F::val(__shfl_sync(0xFFFFFFFFu, F::bits(bv), 31)), b1);
+            V v = (lane == 0) ? f.one() : b32;
+#pragma unroll 1
+            for (u32 o = 1; o < SPLIT_MAX / 32; o <<= 1) {
+                const V u = F::val(__shfl_up_sync(0xFFFFFFFFu, F::bits(v), o));
+                const V m = f.mul(v, u);
+                v = (lane >= o) ? m : v;
+            }
+            if (lane < SPLIT_MAX / 32) sc.b2[lane] = F::bits(v);
+        }
+    }
+    __syncwarp();
+    // z = k^E of every sequence, two rounds of lanes at a time, and its class: n == r
+    // (mod e) where z * h^r == (-c)^E, i.e. h^(-r) == z or, for c = +1 and odd E,
+    // == p - z (z is a unit); no such r: no term is divisible.  r is looked up as
+    // r0 - TAB*j: z * h^(-TAB*j) == h^(-r0).  A kept sequence's k * b^off
+    // (negated for c = +1) and meta are compacted.
+    const u32 nmod = job->nmin % e;
+    u32 nk = 0;
+    bool divk = false;
+    auto classify = [&](u32 i, u64 kr, V z) {
+        bool keep = false;
+        u32 off = 0;
+        V u = z;
+        if (live && i < K) {
+            if (kr == 0) {
+                divk = true;
+            } else {
+                const bool plus = job->c[i] == 1;
+                V y = (plus && (E & 1)) ? f.neg(z) : z;
+                u32 r0 = 0;
+                for (u32 j = 0; j < e && !keep; j += TAB) {
+                    const u64 v = F::bits(y);
+                    u32 s = cls_hash(v, smask);
+                    while ((r0 = sc.slot[s]) != 0) {
+                        if (sc.hv[r0 - 1] == v) {
+                            keep = true;
+                            off = (r0 - 1 + 2 * e - j - nmod) % e;
+                            break;
+                        }
+                        s = (s + 1) & smask;
+                    }
+                    if (SPLIT_MAX > TAB && !keep) y = f.mul(y, hT);
+                }
+                if (keep) {
+                    u = f.of_int(kr);
+                    if constexpr (GL == 32) {
+                        u = f.mul(u, F::val(sc.b1[off & 31]));
+                        if (off >= 32) u = f.mul(u, F::val(sc.b2[off >> 5]));
+                    }
+                    if (plus) u = f.neg(u);
+                }
+            }
+        }
+        if constexpr (GL < 32) {
+            const V bo = power<FP>(f, F::val(X.b), off);
+            if (keep) u = f.mul(u, bo);
+        }
+        const u32 km = __ballot_sync(0xFFFFFFFFu, keep) & gmask;
+        if (keep) {
+            const u32 pos = nk + __popc(km & ((1u << lane) - 1));
+            sc.part[pos] = F::bits(u);
+            sc.meta[pos] = (unsigned short)(i | (off << 7));
+        }
+        nk += __popc(km);
+    };
+    if constexpr (GL == 32) {
+        const u32 R = (K + 31) / 32;
 #pragma unroll 1
         for (u32 r0 = 0; r0 < R; r0 += 2) {
-            double x[4], zd[4];
+            V x[2], z[2];
+            u64 kr[2];
 #pragma unroll
             for (u32 h = 0; h < 2; ++h) {
                 const u32 i = lane + 32 * (r0 + h);
                 const u64 kv = (i < K) ? job->k[i] : 1;
-                x[h] = fp_exact((kv < p) ? kv : kv % p);
+                kr[h] = (kv < p) ? kv : kv % p;
+                x[h] = f.of_int(kr[h]);
             }
-            if (r0 + 1 < R) fpow_multi<2>(zd, x, xD, pd, pinv);
-            else fpow_multi<1>(zd, x, xD, pd, pinv);
-#pragma unroll
-            for (u32 h = 0; h < 2; ++h)
-                if (r0 + h < R) zs[lane + 32 * (r0 + h)] = to_mont(fp_int(zd[h]), M);
+            if (r0 + 1 < R) {
+                power_chains<FP, 2, true>(f, z, x, E);
+#pragma unroll 1
+                for (u32 h = 0; h < 2; ++h) classify(lane + 32 * (r0 + h), h ? kr[1] : kr[0], h ? z[1] : z[0]);
+            } else {
+                power_chains<FP, 1, true>(f, z, x, E);
+                classify(lane + 32 * r0, kr[0], z[0]);
+            }
         }
     } else {
-        u64 x[4], z[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const u32 i = lane + 32 * r;
-            const u64 kv = (i < K) ? job->k[i] : 1;
-            x[r] = to_mont((kv < p) ? kv : kv % p, M);
-        }
-        if (p >> 62) mpow_lanes<false>(R, z, x, xD, M);
-        else mpow_lanes<true>(R, z, x, xD, M);
-#pragma unroll
-        for (u32 r = 0; r < 4; ++r)
-            if (r < R) zs[lane + 32 * r] = z[r];
+        const u64 kv = (l < K) ? job->k[l] : 1;
+        const u64 kr = (kv < p) ? kv : kv % p;
+        V x[2] = {f.of_int(kr), f.one()}, z[2];
+        power_chains<FP, 1, false>(f, z, x, E);
+        classify(l, kr, z[0]);
     }
-}
-
-// Class lookup: the e values h^(-r) (r < e <= SPLIT_MAX, all distinct and
-// nonzero) in an open-addressed table of CLS_SLOTS 64-bit keys with their r
-// beside them, so a sequence's class costs one or two probes instead of a
-// walk over up to e entries (e averages about 28 at 2^50).
-constexpr u32 CLS_SLOTS = 2 * SPLIT_MAX;
-static_assert((CLS_SLOTS & (CLS_SLOTS - 1)) == 0, "slot index wraps by a mask");
-
-__device__ __forceinline__ u32 cls_hash(u64 v) { return (((u32)v ^ (u32)(v >> 32)) * 0x9E3779B1u) >> 25; }
-static_assert(CLS_SLOTS == 128, "cls_hash yields 7 bits");
-
-// Inserts key v (nonzero, not yet present) with index r; lanes insert
-// concurrently, a slot going to the lane whose compare-and-swap finds it empty.
-// At most SPLIT_MAX keys share CLS_SLOTS slots, so the walk always ends.
-__device__ __forceinline__ void cls_insert(u64 *ck, unsigned char *cr, u64 v, u32 r)
-{
-    u32 s = cls_hash(v);
-    for (u32 n = 0; n < CLS_SLOTS; ++n) {
-        if (atomicCAS(reinterpret_cast<unsigned long long *>(&ck[s]), 0ull, (unsigned long long)v) == 0ull) {
-            cr[s] = (unsigned char)r;
-            return;
-        }
-        s = (s + 1) & (CLS_SLOTS - 1);
+    divk = (__ballot_sync(0xFFFFFFFFu, divk) & gmask) != 0;
+    const bool skip = divk || nk == 0;
+    if (live && skip && l == 0) {
+        hdr[w].p = 0;
+        atomicAdd(&stats[ST_SKIPPED], 1ull);
     }
-}
-
-// r with ck[.] == v, or none when v is absent (an empty slot ends the walk).
-__device__ __forceinline__ u32 cls_find(const u64 *ck, const unsigned char *cr, u64 v, u32 none)
-{
-    u32 s = cls_hash(v);
-    for (u32 n = 0; n < CLS_SLOTS; ++n) {
-        const u64 k = ck[s];
-        if (k == v) return cr[s];
-        if (k == 0) break;
-        s = (s + 1) & (CLS_SLOTS - 1);
-    }
-    return none;
-}
-
-// Sequence classes, targets, baby-step count and the start tables of record w
-// (one warp).  tw: this warp's table of SPLIT_MAX powers of b, the CLS_SLOTS
-// keys of its class lookup and chi(k) of up to 128 sequences; cr: the
-// lookup's indices.
-__device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 w, u32 lane, PrimeHdr *__restrict__ hdr,
-                                            const PrimeAux *__restrict__ aux, u64 *__restrict__ tabs,
-                                            u64 *__restrict__ tgt, unsigned short *__restrict__ meta,
-                                            u64 *__restrict__ stats, u32 *__restrict__ err, const JobGeom &gm,
-                                            u64 *tw, unsigned char *cr)
-{
-    PrimeHdr H = hdr[w];
-    if (H.p == 0) {
-        if (lane == 0) atomicAdd(&stats[ST_SKIPPED], 1ull);
-        return;
-    }
-    const PrimeAux &X = aux[w];
-    Mont M;
-    M.p = H.p; M.q = H.q; M.one = H.one; M.r2 = X.r2;
-    const u64 p = H.p;
-    const u32 K = job->kcount;
-    const u32 e = X.e;
-    const u64 mone = p - M.one;
-    u64 *tg = tgt + (size_t)w * KSTRIDE;
-    unsigned short *mg_ = meta + (size_t)w * KSTRIDE;
-    // the class lookup gets h^(-r) and, for now, wt[r] = b^r, for r < e: lane
-    // l forms h^(-l) and b^l by a multiplicative scan over the warp (five
-    // products each); entries 32..63 take one more product by h^(-32) and b^32
-    static_assert(SPLIT_MAX <= 64, "two rounds of 32 table entries");
-    u64 *wt = tw, *ck = tw + SPLIT_MAX, *zs = ck + CLS_SLOTS;
-    __syncwarp();                                          // the previous prime's readers are done
-#pragma unroll
-    for (u32 i = 0; i < CLS_SLOTS; i += 32) ck[i + lane] = 0;
-    __syncwarp();
-    {
-        const u64 hm1 = X.hm1, bm = X.bm;
-        u64 hv = (lane == 0) ? M.one : hm1, bv = (lane == 0) ? M.one : bm;
-#pragma unroll 1
-        for (int o = 1; o < 32; o <<= 1) {
-            const u64 hu = __shfl_up_sync(0xFFFFFFFFu, hv, o), bu = __shfl_up_sync(0xFFFFFFFFu, bv, o);
-            if (lane >= (u32)o) {
-                hv = mmul(hv, hu, p, M.q);
-                bv = mmul(bv, bu, p, M.q);
-            }
-        }
-        if (lane < e) {
-            cls_insert(ck, cr, hv, lane);
-            wt[lane] = bv;
-        }
-        if (e > 32) {
-            const u64 h32 = mmul(__shfl_sync(0xFFFFFFFFu, hv, 31), hm1, p, M.q);
-            const u64 b32 = mmul(__shfl_sync(0xFFFFFFFFu, bv, 31), bm, p, M.q);
-            if (lane + 32 < e) {
-                cls_insert(ck, cr, mmul(hv, h32, p, M.q), lane + 32);
-                wt[lane + 32] = mmul(bv, b32, p, M.q);
-            }
-        }
-    }
-    // z = chi(k) = k^xD for the lane's sequences i = lane + 32r, r < R: one
-    // exponent for the whole warp, R independent chains per lane
-    const u32 R = (K + 31) / 32;
-    chi_of_ks(job, lane, K, M, X.xD, zs);
-    __syncwarp();
-    // pass 1: the class of every sequence; the kept ones' k mod p and class
-    // offset go to the record (compacted), the target itself once Q' is known.
-    // The rounds read chi(k) back from shared memory, so the loop is not
-    // unrolled: one copy of its code keeps the kernel's hot path short.
-    const u32 nmod = job->nmin % e;
-    u32 nk = 0;
-    bool divk = false, lost = false;
-#pragma unroll 1
-    for (u32 rd = 0; rd < R; ++rd) {
-        const u32 i = lane + 32 * rd;
-        const u64 zr = zs[i];
-        bool keep = false;
-        u64 kr = 0;
-        unsigned short mt = 0;
-        if (i < K) {
-            const u64 kv = job->k[i];
-            kr = (kv < p) ? kv : kv % p;
-            if (kr == 0) {
-                divk = true;
-            } else {
-                const int ci = job->c[i];
-                // the target is possible iff (chi(-c)/z)^eo == 1, i.e.
-                // z1^e == chi(-c)^eo with z1 = z^xe; chi(-c) is 1 for c = -1.
-                // When xe = 1 (eo = e, the usual case) that is exactly "the class
-                // search below finds r", so the power is skipped.
-                const u64 z1 = (X.xe == 1) ? zr : mpow_call(zr, X.xe, M);
-                const u64 want = (ci == 1 && (X.flags & AUX_NEG_EO)) ? mone : M.one;
-                const bool pass = (X.xe == 1) || mpow_call(z1, (u64)e, M) == want;
-                if (pass) {
-                    // n == r (mod e) where z1 * h^r == chi(-c)^xe, i.e.
-                    // h^(-r) == z1 or, when chi(-c)^xe == -1, == p - z1
-                    // (z1 is a unit, so both lie in (0, p))
-                    const bool neg = (ci == 1) && (X.flags & AUX_NEG_XE);
-                    const u32 r = cls_find(ck, cr, neg ? p - z1 : z1, e);
-                    if (r < e) {
-                        const u32 off = (r + e - nmod) % e;
-                        mt = (unsigned short)(i | (off << 7));
-                        keep = true;
-                    } else if (X.xe != 1) {
-                        lost = true;                      // cannot happen: the class exists when the test passes
-                    }
-                }
-            }
-        }
-        const u32 km_ = __ballot_sync(0xFFFFFFFFu, keep);
-        if (keep) {
-            const u32 pos = nk + __popc(km_ & ((1u << lane) - 1));
-            tg[pos] = kr;
-            mg_[pos] = mt;
-        }
-        nk += __popc(km_);
-    }
-    if (lost) atomicOr(err, ERR_SETUP_CLASS);
-    divk = __any_sync(0xFFFFFFFFu, divk);
-    if (divk || nk == 0) {
-        if (lane == 0) {
-            hdr[w].p = 0;
-            atomicAdd(&stats[ST_SKIPPED], 1ull);
-        }
-        return;
-    }
-    // baby steps for this prime (the giant-step tables follow in kernel 3)
+    __syncwarp();                                          // the compacted parts are written
+    if (!live || skip) return;
+    // baby steps for this prime (the giant-step tables follow in kernel 3), and the
+    // targets T = -c * k * b^(nmin + off + e(Q'-1))
     const u32 cls = choose_class(gm, nk, (job->L + e - 1) / e);
-    // targets T = -c * k * b^(nmin + off + e(Q'-1)): wt[r] = b^(nmin + e(Q'-1) + r) * R^2
-    const u64 wr0 = X.wr0[cls];
-    for (u32 r = lane; r < e; r += 32) wt[r] = mmul(wr0, wt[r], p, M.q);
-    __syncwarp();                                          // also orders pass 1's record writes
-    for (u32 j = lane; j < nk; j += 32) {
-        const u32 m = mg_[j];
-        u64 T = mmul(tg[j], wt[m >> 7], p, M.q);
-        if (job->c[m & 0x7Fu] == 1) T = mneg(T, p);
-        if (p < FP_BOUND) T = double_bits(fp_exact(from_mont(T, M)));   // the FP64 steps' form
-        tg[j] = T;
+    const V wr0 = F::val(X.wr0[cls]);
+    for (u32 j = l; j < nk; j += GL) {
+        tgt[(size_t)w * KSTRIDE + j] = F::bits(f.mul(F::val(sc.part[j]), wr0));
+        meta[(size_t)w * KSTRIDE + j] = sc.meta[j];
     }
-    if (lane == 0) {
+    if (l == 0) {
         hdr[w].numk = nk;
         hdr[w].cls = cls;
     }
@@ -576,110 +691,71 @@ __device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float p, u32
 // to the thread's tallies.  Each table is only as long as the BSGS kernel
 // reads it: A[t % 32] and B[t / 32] for the group's threads t, Z1[g % 32] and
 // Z2[g / 32] for the giant chunks g < G.
+template <bool FP>
 __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u32 t, PrimeHdr *__restrict__ hdr,
                                                const PrimeAux *__restrict__ aux, u64 *__restrict__ tabs,
                                                u32 &n_targets, u32 &n_full, u32 &n_split)
 {
-    PrimeHdr H = hdr[t];
-    const u64 p = H.p, q = H.q;
-    Mont M;
-    M.p = p; M.q = q; M.one = H.one; M.r2 = 0;
-    const u32 e = H.e, nk = H.numk, gs = 32u << H.cls, lq = 9 + H.cls;
+    typedef Field<FP> F;
+    typedef typename F::V V;
+    PrimeHdr &h = hdr[t];
+    const F f(h, aux[t]);
+    const u32 e = h.e, nk = h.numk, cls = h.cls, gs = 32u << cls, lq = 9 + cls;
     const u32 Le = (job->L + e - 1) / e;
     const u32 Mg = (Le + (1u << lq) - 1) >> lq;
     u32 G, Lc, nseg, rounds;
-    giant_split(gs, nk, Mg, (float)p, G, Lc, nseg, rounds);
-    const u64 S = aux[t].S[H.cls];
-    u64 *tb = tabs + (size_t)t * TABS;
-    const u32 nb = gs >> 5, nz1 = min(G, 32u), nz2 = (G + 31) >> 5;
-    PrimeHdr &h = hdr[t];
+    giant_split(gs, nk, Mg, (float)h.p, G, Lc, nseg, rounds);
     h.G = G;
     h.Lc = Lc;
     h.Mg = Mg;
     h.rk = 1.0f / (float)nk;
     h.nseg = nseg;
     h.rounds = rounds;
-    // z^32 is needed only when G > 32, and then the Z1 chain has run all 32 steps
-    if (p < FP_BOUND) {
-        const double pd = fp_exact(p), pinv = 1.0 / pd;
-        auto mul = [&](double x, double y) { return fp_mul(x, y, pd, pinv); };
-        const u64 s1 = H.sp, S1 = from_mont(S, M);        // plain
-        const double sd = fp_exact(s1), Sd = fp_exact(S1);
-        double u8 = mul(sd, sd);
-        u8 = mul(u8, u8);
-        u8 = mul(u8, u8);
-        const double u = mul(u8, u8), z = fpow_call(Sd, Lc, pd, pinv);
-        double a = 1.0, b = 1.0;
-        for (u32 l = 0; l < 32; ++l) {
-            tb[l] = double_bits(a);
-            a = mul(a, u);
-            if (l < nz1) {
-                tb[64 + l] = double_bits(b);
-                b = mul(b, z);
-            }
+    const V s = F::val(h.s), S = F::val(aux[t].S[cls]);
+    V u8 = f.mul(s, s);
+    u8 = f.mul(u8, u8);
+    u8 = f.mul(u8, u8);
+    const V u = f.mul(u8, u8), z = power<FP>(f, S, Lc);
+    u64 *tb = tabs + (size_t)t * TABS;
+    const u32 nb = gs >> 5, nz1 = min(G, 32u), nz2 = (G + 31) >> 5;
+    V a = f.one(), b = a;
+    for (u32 l = 0; l < 32; ++l) {
+        tb[l] = F::bits(a);
+        a = f.mul(a, u);
+        if (l < nz1) {
+            tb[64 + l] = F::bits(b);
+            b = f.mul(b, z);
         }
-        const double u32p = a, z32 = b;
-        a = 1.0;
-        b = 1.0;
-        for (u32 l = 0; l < max(nb, nz2); ++l) {
-            if (l < nb) {
-                tb[32 + l] = double_bits(a);
-                a = mul(a, u32p);
-            }
-            if (l < nz2) {
-                tb[96 + l] = double_bits(b);
-                b = mul(b, z32);
-            }
+    }
+    // (z^32 is needed only when G > 32, and then the Z1 chain has run all 32 steps)
+    const V u32p = a, z32 = b;
+    a = b = f.one();
+    for (u32 l = 0; l < max(nb, nz2); ++l) {
+        if (l < nb) {
+            tb[32 + l] = F::bits(a);
+            a = f.mul(a, u32p);
         }
-        h.q = double_bits(pinv);
-        h.s = double_bits(sd);
-        h.sw = double_bits(sd / pd);
-        h.S = double_bits(Sd);
-        h.Sw = double_bits(Sd / pd);
-        h.u8 = double_bits(u8);
-    } else {
-        auto mul = [&](u64 x, u64 y) { return mmul(x, y, p, q); };
-        u64 u8 = mul(H.s, H.s);
-        u8 = mul(u8, u8);
-        u8 = mul(u8, u8);
-        const u64 u = mul(u8, u8), z = mpow(S, (u64)Lc, M);
-        u64 a = M.one, b = M.one;
-        for (u32 l = 0; l < 32; ++l) {
-            tb[l] = a;
-            a = mul(a, u);
-            if (l < nz1) {
-                tb[64 + l] = b;
-                b = mul(b, z);
-            }
+        if (l < nz2) {
+            tb[96 + l] = F::bits(b);
+            b = f.mul(b, z32);
         }
-        const u64 u32p = a, z32 = b;
-        a = M.one;
-        b = M.one;
-        for (u32 l = 0; l < max(nb, nz2); ++l) {
-            if (l < nb) {
-                tb[32 + l] = a;
-                a = mul(a, u32p);
-            }
-            if (l < nz2) {
-                tb[96 + l] = b;
-                b = mul(b, z32);
-            }
-        }
-        h.S = S;
-        h.u8 = u8;
-        if (!(p >> 63)) {                                  // Shoup multiplier of the giant steps below 2^63
-            h.Sp = from_mont(S, M);
-            h.Sw = shoup_of_mont(S, q);
-        }
+    }
+    h.S = F::bits(S);
+    h.u8 = F::bits(u8);
+    if constexpr (FP) {
+        h.Sw = double_bits(S / f.p);
+    } else if (!(f.M.p >> 63)) {                           // Shoup multiplier of the giant steps below 2^63
+        h.Sp = from_mont(S, f.M);
+        h.Sw = shoup_of_mont(S, f.M.q);
     }
     n_targets += nk;
     if (e >= 2) ++n_split; else ++n_full;
 }
 
 // Kernel 3: one thread per prime (indexing as kernel 1); then the record's index
-// goes on the list of its class (BATCH: of its job's group and step kind).
-template <bool BATCH>
-__global__ void __launch_bounds__(256) k_setup_tabs(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
+// goes on the list of its class (ANY_PRIMES: of its job's group and step kind).
+template <int KIND>
+__global__ void __launch_bounds__(128) k_setup_tabs(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
                                                     const PrimeAux *__restrict__ aux, u32 count,
                                                     u64 *__restrict__ tabs, u64 *__restrict__ stats,
                                                     u32 *__restrict__ lists, u32 list_stride, u32 *list_ctl,
@@ -687,6 +763,7 @@ __global__ void __launch_bounds__(256) k_setup_tabs(const JobDev *__restrict__ j
                                                     const u32 *__restrict__ prefix, u32 nr,
                                                     const u32 *__restrict__ rec_of)
 {
+    constexpr bool BATCH = KIND == ANY_PRIMES;
     const u32 stride = gridDim.x * blockDim.x;
     const u32 lane = threadIdx.x & 31;
     const u32 total = BATCH ? prefix[nr] : count;
@@ -699,8 +776,9 @@ __global__ void __launch_bounds__(256) k_setup_tabs(const JobDev *__restrict__ j
         u32 key = 0xFFFFFFFFu;                             // list of the record: group * NCLASS + class
         if (live) {
             const u32 jb = BATCH ? hdr[rec].job : 0;
-            setup_tabs_one(jobs + jb, rec, hdr, aux, tabs, nt, nf, ns);
             const u64 p = hdr[rec].p;
+            if (KIND == FP_PRIMES || (BATCH && p < FP_BOUND)) setup_tabs_one<true>(jobs + jb, rec, hdr, aux, tabs, nt, nf, ns);
+            else setup_tabs_one<false>(jobs + jb, rec, hdr, aux, tabs, nt, nf, ns);
             const u32 g = BATCH ? geoms[jb].group + (p < FP_BOUND ? 2u : (p >> 63) ? 0u : 1u) : 0u;
             key = g * NCLASS + hdr[rec].cls;
         }
@@ -723,75 +801,103 @@ __global__ void __launch_bounds__(256) k_setup_tabs(const JobDev *__restrict__ j
 }
 
 
-// Kernel 2: one warp per prime; lanes walk the sequences.  BATCH as kernel 1.
-template <bool BATCH>
+// Kernel 2: GL lanes per prime.  KIND as kernel 1 (ANY_PRIMES: the primes of a
+// batch round, GL = 32).
+template <int KIND, u32 GL>
 __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
                                                        const PrimeAux *__restrict__ aux, u32 count,
-                                                       u64 *__restrict__ tabs, u64 *__restrict__ tgt,
-                                                       unsigned short *__restrict__ meta, u64 *__restrict__ stats,
-                                                       u32 *__restrict__ err, JobGeom gm,
+                                                       u64 *__restrict__ tgt, unsigned short *__restrict__ meta,
+                                                       u64 *__restrict__ stats, JobGeom gm,
                                                        const JobGeom *__restrict__ geoms,
                                                        const u32 *__restrict__ prefix, u32 nr,
                                                        const u32 *__restrict__ rec_of)
 {
-    __shared__ u64 s_tw[SETUP_TPB / 32][SPLIT_MAX + CLS_SLOTS + 4 * 32];   // per warp: powers of b, class lookup keys, chi(k)
-    __shared__ unsigned char s_cr[SETUP_TPB / 32][CLS_SLOTS];     //   and the lookup's class indices
-    const u32 lane = threadIdx.x & 31;
-    const u32 nwarps = gridDim.x * (SETUP_TPB / 32);
-    u64 *tw = s_tw[threadIdx.x >> 5];
-    unsigned char *cr = s_cr[threadIdx.x >> 5];
-    // w is uniform over the warp, so the warp-wide ballots of a prime stay whole
-    if constexpr (BATCH) {
+    __shared__ KScratch<GL> s_sc[SETUP_TPB / GL];
+    const u32 l = threadIdx.x & (GL - 1);
+    KScratch<GL> &sc = s_sc[threadIdx.x / GL];
+    const u32 stride = gridDim.x * (SETUP_TPB / GL);
+    u32 i = (blockIdx.x * SETUP_TPB + threadIdx.x) / GL;
+    if constexpr (KIND == ANY_PRIMES) {
+        static_assert(GL == 32, "a warp holds primes of one step kind");
         const u32 total = prefix[nr];
-        for (u32 i = (blockIdx.x * SETUP_TPB + threadIdx.x) >> 5; i < total; i += nwarps) {
+        for (; i < total; i += stride) {
             const u32 rec = rec_of[i];
+            const u64 p = hdr[rec].p;
+            if (p == 0) {
+                if (l == 0) atomicAdd(&stats[ST_SKIPPED], 1ull);
+                continue;
+            }
             const u32 jb = hdr[rec].job;
-            setup_k_one(jobs + jb, rec, lane, hdr, aux, tabs, tgt, meta, stats, err, geoms[jb], tw, cr);
+            if (p < FP_BOUND) setup_k_one<true, GL>(jobs + jb, rec, l, true, hdr, aux, tgt, meta, stats, geoms[jb], sc);
+            else setup_k_one<false, GL>(jobs + jb, rec, l, true, hdr, aux, tgt, meta, stats, geoms[jb], sc);
         }
     } else {
-        for (u32 w = (blockIdx.x * SETUP_TPB + threadIdx.x) >> 5; w < count; w += nwarps)
-            setup_k_one(jobs, w, lane, hdr, aux, tabs, tgt, meta, stats, err, gm, tw, cr);
+        // i - l / GL of a warp's sub-warps: the warp stays until its last prime is done
+        for (; __any_sync(0xFFFFFFFFu, i < count); i += stride) {
+            const bool in = i < count;
+            const bool live = in && hdr[i].p != 0;
+            if (in && !live && l == 0) atomicAdd(&stats[ST_SKIPPED], 1ull);
+            if (!__any_sync(0xFFFFFFFFu, live)) continue;
+            setup_k_one<KIND == FP_PRIMES, GL>(jobs, in ? i : 0, l, live, hdr, aux, tgt, meta, stats, gm, sc);
+        }
     }
 }
 
-cudaError_t launch_setup(const JobDev *job, const u64 *primes, u32 first, u32 count, PrimeHdr *hdr, void *aux, u64 *tabs,
-                         u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err, int geom,
-                         cudaStream_t st)
+template <int KIND>
+static cudaError_t launch_setup_kind(const JobDev *job, u32 kcount, const u64 *primes, u32 first, u32 count,
+                                     PrimeHdr *hdr, PrimeAux *aux, u64 *tabs, u64 *tgt, unsigned short *meta,
+                                     const BsgsLists &lists, u64 *stats, const JobGeom &gm, cudaStream_t st)
+{
+    k_setup_prime<KIND><<<(count + 127) / 128, 128, 0, st>>>(job, primes, first, count, hdr, aux, nullptr, nullptr, 0, 0,
+                                                             nullptr);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    auto go = [&](auto gl) {
+        constexpr u32 GL = decltype(gl)::value;
+        const u32 ppb = SETUP_TPB / GL;                    // primes per block
+        k_setup_k<KIND, GL><<<(count + ppb - 1) / ppb, SETUP_TPB, 0, st>>>(job, hdr, aux, count, tgt, meta, stats, gm,
+                                                                          nullptr, nullptr, 0, nullptr);
+    };
+    if (kcount <= 4) go(std::integral_constant<u32, 4>{});
+    else if (kcount <= 8) go(std::integral_constant<u32, 8>{});
+    else if (kcount <= 16) go(std::integral_constant<u32, 16>{});
+    else go(std::integral_constant<u32, 32>{});
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_setup_tabs<KIND><<<(count + 127) / 128, 128, 0, st>>>(job, hdr, aux, count, tabs, stats, lists.list, lists.stride,
+                                                            lists.ctl, nullptr, nullptr, 0, nullptr);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_setup(const JobDev *job, u32 kcount, const u64 *primes, u32 first, u32 count, u64 pmax, PrimeHdr *hdr,
+                         void *aux, u64 *tabs, u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats,
+                         int geom, cudaStream_t st)
 {
     if (count == 0) return cudaSuccess;
     const JobGeom gm = job_geom(geom);
-    k_setup_prime<false><<<(count + 255) / 256, 256, 0, st>>>(job, primes, first, count, hdr, (PrimeAux *)aux, nullptr,
-                                                              nullptr, 0, 0, nullptr);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const u32 wpb = SETUP_TPB / 32;
-    k_setup_k<false><<<(count + wpb - 1) / wpb, SETUP_TPB, 0, st>>>(job, hdr, (const PrimeAux *)aux, count, tabs, tgt,
-                                                                   meta, stats, err, gm, nullptr, nullptr, 0, nullptr);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_setup_tabs<false><<<(count + 255) / 256, 256, 0, st>>>(job, hdr, (const PrimeAux *)aux, count, tabs, stats,
-                                                             lists.list, lists.stride, lists.ctl, nullptr, nullptr, 0,
-                                                             nullptr);
-    return cudaGetLastError();
+    PrimeAux *x = (PrimeAux *)aux;
+    return pmax <= FP_BOUND
+               ? launch_setup_kind<FP_PRIMES>(job, kcount, primes, first, count, hdr, x, tabs, tgt, meta, lists, stats, gm, st)
+               : launch_setup_kind<INT_PRIMES>(job, kcount, primes, first, count, hdr, x, tabs, tgt, meta, lists, stats, gm, st);
 }
 
 cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const BatchRange *ranges, const u64 *primes,
                                u32 rcap, const u32 *prefix_p, u32 nranges, PrimeHdr *hdr, void *aux, u64 *tabs,
-                               u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *err,
-                               u32 *rec_of, int sms, cudaStream_t st)
+                               u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *rec_of, int sms,
+                               cudaStream_t st)
 {
     JobGeom gm{};
     // full-device grids; the kernels stride over the primes of every range
-    k_setup_prime<true><<<sms * 4, 256, 0, st>>>(jobs, primes, 0, 0, hdr, (PrimeAux *)aux, ranges, prefix_p, nranges,
-                                                 rcap, rec_of);
+    k_setup_prime<ANY_PRIMES><<<sms * 8, 128, 0, st>>>(jobs, primes, 0, 0, hdr, (PrimeAux *)aux, ranges, prefix_p, nranges,
+                                                       rcap, rec_of);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_setup_k<true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, tgt, meta, stats, err,
-                                                   gm, geoms, prefix_p, nranges, rec_of);
+    k_setup_k<ANY_PRIMES, 32><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tgt, meta, stats, gm,
+                                                             geoms, prefix_p, nranges, rec_of);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_setup_tabs<true><<<sms * 4, 256, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, stats, lists.list,
-                                                lists.stride, lists.ctl, geoms, prefix_p, nranges, rec_of);
+    k_setup_tabs<ANY_PRIMES><<<sms * 8, 128, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, stats, lists.list,
+                                                      lists.stride, lists.ctl, geoms, prefix_p, nranges, rec_of);
     return cudaGetLastError();
 }
 
