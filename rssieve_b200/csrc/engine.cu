@@ -315,6 +315,7 @@ void jobdev_from_seqs(const rs_seqs *s, JobDev *out)
     out->nmax = s->nmax;
     out->L = s->nmax - s->nmin + 1;
     out->words = (u32)s->words_per_seq;
+    out->split = split_limit(out->kcount, out->L);
     for (u32 i = 0; i < s->kcount; ++i) {
         out->k[i] = s->k[i];
         out->c[i] = s->c[i];

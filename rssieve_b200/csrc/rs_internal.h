@@ -49,7 +49,7 @@ constexpr int geom_index(u32 q)
 // giant steps.
 inline double geom_model_cost(int g, u32 kcount, u32 L)
 {
-    constexpr double SPLIT[10] = {2, 2, 4, 6, 8, 12, 20, 36, 64, 120};
+    constexpr double SPLIT[10] = {2, 2, 4, 6, 10, 16, 30, 60, 120, 230};
     double sum = 0;
     for (double d : SPLIT) {
         double best = 1e300;
@@ -60,7 +60,8 @@ inline double geom_model_cost(int g, u32 kcount, u32 L)
         }
         sum += best;
     }
-    return sum / 10;
+    // (1024-thread CTAs run alone on an SM, so nothing covers their barriers: 5%)
+    return sum / 10 * (BSGS_GEOMS[g].tpb == 1024 ? 1.05 : 1.0);
 }
 inline int geom_model_best(u32 kcount, u32 L)
 {
@@ -112,10 +113,17 @@ struct JobDev {
     u32 base, kcount, nmin, nmax;
     u32 L;               // nmax - nmin + 1
     u32 words;           // bitmap words per sequence
+    u32 split;           // largest split modulus (split_limit)
     u64 k[KMAX];
     int c[KMAX];
     u32 *bitmap;         // kcount * words
 };
+// A larger split modulus e means fewer giant steps and a longer class table per
+// prime.  With a warp per prime (more than 16 sequences) 256 always pays: 100
+// sequences over 6*10^6, 26.0 -> 21.8 ns per prime against 64; 68 over 10^5, 8.5
+// -> 8.4.  With a few lanes per prime the table weighs more: one sequence over
+// 10^7, 4.24 -> 4.07; 8 over 2*10^5, 3.74 -> 3.92, so small searches keep 64.
+constexpr u32 split_limit(u32 kcount, u32 L) { return kcount > 16 || (u64)kcount * L > 4000000 ? 256u : 64u; }
 
 // Below FP_BOUND = 2^51 the BSGS steps run on the FP64 pipe (fp_mulfix in
 // mont.cuh): residues are exact integers in doubles, and a product by a fixed
@@ -136,7 +144,7 @@ struct PrimeHdr {        // 128 bytes (a 16-byte multiple: copied by TMA bulk co
     u64 S, Sw, Sp;       // the same for s^Q', Q' = this prime's baby-step count
     u64 u8;              // s^8: start offset of a thread's second baby chain
     u32 numk;            // surviving targets
-    u32 e;               // split modulus, 1..64
+    u32 e;               // split modulus, 1..256
     u32 G, Lc;           // giant phase: G chunks of Lc giant steps per target
     u32 smul;            // b^e as an integer when it is at most 16, else 0 (2 and 4: baby steps by doublings)
     u32 job;             // job index within a batch (0 for a single job)

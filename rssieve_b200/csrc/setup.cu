@@ -14,14 +14,14 @@
 // Residue classes of n.  The reference splits n by parity when b is a
 // quadratic non-residue mod p (e = 2) and filters with d-th power residues
 // (setup.cl:22-87).  Here both come from one character of larger order.  Let D
-// be the part of p-1 made of the primes up to 61, and chi(x) = x^((p-1)/D),
+// be the part of p-1 made of the primes up to 251, and chi(x) = x^((p-1)/D),
 // which maps onto the D-th roots of unity.  If k*b^n == -c then
 //      chi(b)^n = chi(-c) / chi(k),
 // so (1) a target is impossible unless chi(-c)/chi(k) lies in the subgroup
 // generated by chi(b), of order eo (the reference's filters are the cases
 // d | D of this), and (2) n mod e is fixed, for every divisor e of eo, by the
 // discrete logarithm of h = chi(b)^(eo/e) -- a table of e values.  e is the
-// largest divisor of eo up to 64.  Both take one power per sequence, z = k^E with
+// largest divisor of eo up to 256 (64 for small jobs, JobDev::split).  Both take one power per sequence, z = k^E with
 // E = (p-1)/D * eo/e: the logarithm of (-c)^E / z to the base h exists exactly
 // when (chi(-c)/chi(k))^eo = 1, the groups being cyclic.  Every n the reference finds satisfies both,
 // so the eliminated terms are the same, while each sequence's giant steps
@@ -46,11 +46,14 @@
 
 namespace rs {
 
-constexpr u32 SPLIT_MAX = 64;        // largest split modulus e (at most 512: 9 bits of offset per target)
+constexpr u32 SPLIT_MAX = 256;       // largest split modulus e of any job (at most 512: 9 bits of offset per target)
 static_assert(SPLIT_MAX <= 512 && SPLIT_MAX % 32 == 0, "offsets and tables of powers");
 
 // The primes whose powers make up D, the smooth part of p-1.
-constexpr u32 SMOOTH[] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61};
+constexpr u32 SMOOTH[] = {
+    2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 67, 71, 73, 79,
+    83, 89, 97, 101, 103, 107, 109, 113, 127, 131, 137, 139, 149, 151, 157, 163, 167, 173,
+    179, 181, 191, 193, 197, 199, 211, 223, 227, 229, 233, 239, 241, 251};
 constexpr int NSMOOTH = sizeof(SMOOTH) / sizeof(SMOOTH[0]);
 static_assert(NSMOOTH <= 64, "a prime's smooth factors are a 64-bit mask");
 
@@ -205,11 +208,11 @@ __device__ __forceinline__ u64 without(u64 x, u32 l)
     return y;
 }
 
-// Largest divisor of eo that is at most SPLIT_MAX.
-__device__ __forceinline__ u32 split_modulus(u64 eo)
+// Largest divisor of eo that is at most most.
+__device__ __forceinline__ u32 split_modulus(u64 eo, u32 most)
 {
-    if (eo <= SPLIT_MAX) return (u32)eo;
-    u32 d = SPLIT_MAX;
+    if (eo <= most) return (u32)eo;
+    u32 d = most;
     if (eo >> 52) {
         while (eo % d != 0) --d;
         return d;
@@ -272,7 +275,7 @@ __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, 
             eo *= l;
         }
     }
-    const u32 e = split_modulus(eo);
+    const u32 e = split_modulus(eo, job->split);
     const u64 xe = eo / e;
     PrimeHdr H;
     PrimeAux X;
@@ -440,17 +443,18 @@ __device__ __forceinline__ void power_chains(const Field<FP> &F, typename Field<
 }
 
 // Shared memory of a sub-warp of GL lanes in kernel 2: the values h^(-r), r <
-// min(e, TAB), the class lookup over them (open addressing, r + 1 in a 16-bit
+// min(e, TAB) (all of them for GL = 32; the others look a class up in several
+// turns, which with 64 entries cost GL = 32 a third of the kernel), the class lookup over them (open addressing, r + 1 in a 16-bit
 // slot, 0: empty), powers of b, and the targets' parts until the baby-step count
 // is known.
 template <u32 GL>
 struct KScratch {
     static constexpr u32 KM = GL == 32 ? 128 : GL;       // sequences
-    static constexpr u32 TAB = GL == 4 ? 32 : 64, CLS_SLOTS = 2 * TAB;
+    static constexpr u32 TAB = GL == 4 ? 32 : GL < 32 ? 64 : SPLIT_MAX, CLS_SLOTS = GL < 32 ? 2 * TAB : 4 * TAB;
     u64 hv[TAB];
     u64 part[KM];
     u64 b1[GL == 32 ? 32 : 1], b2[GL == 32 ? 16 : 1];
-    unsigned short slot[CLS_SLOTS];
+    alignas(16) unsigned short slot[CLS_SLOTS];
     unsigned short meta[KM];
 };
 
@@ -481,11 +485,15 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
     const u64 E = X.E;
     // class table: lane l forms h^(-l) by a multiplicative scan over the GL lanes,
     // then every GL-th value from there by products with h^(-GL)
-    constexpr u32 TAB = KScratch<GL>::TAB, CLS_SLOTS = KScratch<GL>::CLS_SLOTS, smask = CLS_SLOTS - 1;
+    constexpr u32 TAB = KScratch<GL>::TAB, CLS_SLOTS = KScratch<GL>::CLS_SLOTS;
     const u32 ne = min(e, TAB);
+    // (four slots or more per entry for a whole warp's prime: the warp inserts in as
+    // many turns as its slowest lane; a power of two, at least 64)
+    const u32 nslot = GL < 32 ? CLS_SLOTS : max(64u, 1u << (34 - __clz(ne - 1 | 15)));
+    const u32 smask = nslot - 1;
     V hT = f.one();                                        // h^(-TAB), for e > TAB
     __syncwarp();                                          // the previous prime's readers are done
-    for (u32 i = l; i < CLS_SLOTS / 2; i += GL) reinterpret_cast<u32 *>(sc.slot)[i] = 0;
+    for (u32 i = l; i < nslot / 8; i += GL) reinterpret_cast<uint4 *>(sc.slot)[i] = make_uint4(0u, 0u, 0u, 0u);
     {
         const V hm1 = F::val(X.hm1);
         V hv = (l == 0) ? f.one() : hm1;
@@ -496,7 +504,7 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
             hv = (l >= o) ? m : hv;
         }
         const V hG = f.mul(F::val(__shfl_sync(0xFFFFFFFFu, F::bits(hv), GL - 1, GL)), hm1);
-        if (SPLIT_MAX > TAB) {
+        if constexpr (SPLIT_MAX > TAB) {
             hT = hG;
 #pragma unroll 1
             for (u32 n = GL; n < TAB; n *= 2) hT = f.mul(hT, hT);
