@@ -55,7 +55,9 @@ constexpr u32 SMOOTH[] = {
     83, 89, 97, 101, 103, 107, 109, 113, 127, 131, 137, 139, 149, 151, 157, 163, 167, 173,
     179, 181, 191, 193, 197, 199, 211, 223, 227, 229, 233, 239, 241, 251};
 constexpr int NSMOOTH = sizeof(SMOOTH) / sizeof(SMOOTH[0]);
-static_assert(NSMOOTH <= 64, "a prime's smooth factors are a 64-bit mask");
+constexpr int NSMALL = 18;           // those up to 61
+static_assert(NSMOOTH <= 64 && SMOOTH[NSMALL - 1] == 61, "a prime's smooth factors are a 64-bit mask");
+static_assert(SMOOTH[NSMOOTH - 1] <= SPLIT_MAX, "the reciprocals' table covers them");
 
 struct PrimeAux {        // kernel 1 -> kernels 2 and 3; residues in the step kind's form (PrimeHdr)
     u64 E;               // the classes' exponent: z = k^E has order dividing e times the index filtered on
@@ -144,41 +146,55 @@ __device__ __noinline__ typename Field<FP>::V power(const Field<FP> F, typename 
     return (FP || F.lazy) ? power_as<FP, true>(F, x, e) : power_as<FP, false>(F, x, e);
 }
 
-// Divides every factor L out of x, D taking them; returns whether there was one.
-template <u32 L>
-__device__ __forceinline__ bool strip(u64 &x, u64 &D)
+// The SMOOTH primes of index FROM to END-1 that divide x, as a mask of their
+// indices.  No branches: the tests are independent.  Below 2^52 x is held in a
+// double: q = x/L rounded; x - q*L, exact in the fma, is zero exactly when L divides
+// x.  Else x is reduced by products of primes below 2^32, and those remainders by
+// the primes.
+template <int I>
+__device__ __forceinline__ u64 divides_fp(double x)
 {
-    if (x % L != 0) return false;
-    do { x /= L; D *= L; } while (x % L == 0);
-    return true;
+    constexpr u32 L = SMOOTH[I];
+    return fma(-fp_round_prod(x, 1.0 / L), (double)L, x) == 0.0 ? 1ull << I : 0ull;
 }
-// The same for x < 2^52 held in a double: q = x/L rounded; x - q*L, exact in the
-// fma, is zero exactly when L divides x (and then q is the quotient).
-template <u32 L>
-__device__ __forceinline__ bool strip_fp(double &x, double &D)
+template <int FROM, size_t... I>
+__device__ __forceinline__ u64 smooth_mask(double x, std::index_sequence<I...>)
 {
-    double q = fp_round_prod(x, 1.0 / L);
-    if (fma(-q, (double)L, x) != 0.0) return false;
-    do {
-        x = q;
-        D *= (double)L;
-        q = fp_round_prod(x, 1.0 / L);
-    } while (fma(-q, (double)L, x) == 0.0);
-    return true;
+    return (divides_fp<FROM + (int)I>(x) | ...);
 }
-// every SMOOTH prime but 2, whose index is 0; bit i of the result: SMOOTH[i] divides
-template <size_t... I>
-__device__ __forceinline__ u64 strip_all(u64 &x, u64 &D, std::index_sequence<I...>)
+template <int FROM, int END>
+__device__ __forceinline__ u64 smooth_mask(double x) { return smooth_mask<FROM>(x, std::make_index_sequence<END - FROM>()); }
+
+__host__ __device__ constexpr int group_end(int from, int end)
 {
-    u64 m = 0;
-    ((m |= strip<SMOOTH[I + 1]>(x, D) ? 1ull << (I + 1) : 0ull), ...);
+    u64 m = 1;
+    while (from < end && m * SMOOTH[from] < (1ull << 32)) m *= SMOOTH[from++];
+    return from;
+}
+__host__ __device__ constexpr u32 group_product(int from, int end)
+{
+    u32 m = 1;
+    for (; from < end; ++from) m *= SMOOTH[from];
     return m;
 }
-template <size_t... I>
-__device__ __forceinline__ u64 strip_all_fp(double &x, double &D, std::index_sequence<I...>)
+template <int I>
+__device__ __forceinline__ u64 divides(u32 r)
 {
-    u64 m = 0;
-    ((m |= strip_fp<SMOOTH[I + 1]>(x, D) ? 1ull << (I + 1) : 0ull), ...);
+    constexpr u32 L = SMOOTH[I];
+    return r % L == 0 ? 1ull << I : 0ull;
+}
+template <int FROM, size_t... I>
+__device__ __forceinline__ u64 group_mask(u32 r, std::index_sequence<I...>)
+{
+    return (divides<FROM + (int)I>(r) | ...);
+}
+template <int FROM, int END>
+__device__ __forceinline__ u64 smooth_mask(u64 x)
+{
+    constexpr int J = group_end(FROM, END);
+    constexpr u32 P = group_product(FROM, J);
+    u64 m = group_mask<FROM>((u32)(x % P), std::make_index_sequence<J - FROM>());
+    if constexpr (J < END) m |= smooth_mask<J, END>(x);
     return m;
 }
 
@@ -196,30 +212,38 @@ constexpr SetupTables make_tables()
 }
 __constant__ SetupTables c_tab = make_tables();
 
-// x with every factor l removed
+// x with every factor l (at most SPLIT_MAX) removed
 __device__ __forceinline__ u64 without(u64 x, u32 l)
 {
-    if (x >> 32) {
+    if (x >> 52) {
         while (x % l == 0) x /= l;
         return x;
     }
-    u32 y = (u32)x;
-    while (y % l == 0) y /= l;
-    return y;
+    const double inv = c_tab.inv[l];
+    double y = fp_exact(x);
+    for (;;) {
+        const double q = fp_round_prod(y, inv);
+        if (fma(-q, (double)l, y) != 0.0) return fp_int(y);
+        y = q;
+    }
 }
 
-// Largest divisor of eo that is at most most.
+// Largest divisor of eo that is at most most (a multiple of 4); four candidates
+// at a time, so that their tests overlap.
 __device__ __forceinline__ u32 split_modulus(u64 eo, u32 most)
 {
     if (eo <= most) return (u32)eo;
-    u32 d = most;
     if (eo >> 52) {
+        u32 d = most;
         while (eo % d != 0) --d;
         return d;
     }
     const double x = fp_exact(eo);
-    while (fma(-fp_round_prod(x, c_tab.inv[d]), (double)d, x) != 0.0) --d;
-    return d;
+    auto divides = [&](u32 d) { return fma(-fp_round_prod(x, c_tab.inv[d]), (double)d, x) == 0.0; };
+    for (u32 d = most;; d -= 4) {
+        const bool a = divides(d), b = divides(d - 1), c = divides(d - 2), e = divides(d - 3);
+        if (a | b | c | e) return a ? d : b ? d - 1 : c ? d - 2 : d - 3;
+    }
 }
 
 // b^e as an integer when it is at most 16 (baby steps by additions), else 0.
@@ -249,17 +273,17 @@ __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, 
     }
     const F f(p);
     const V bv = f.of_int(bp);
-    // D = smooth part of p-1, x = (p-1)/D, mask: its primes
+    // D = smooth part of p-1, x = (p-1)/D, mask: its primes (small searches stop at 61)
     const int v2 = __ffsll((long long)(p - 1)) - 1;
-    u64 x = (p - 1) >> v2, D = 1ull << v2, mask;
-    if constexpr (FP) {
-        double xd = fp_exact(x), Dd = 1.0;
-        mask = strip_all_fp(xd, Dd, std::make_index_sequence<NSMOOTH - 1>());
-        x = fp_int(xd);
-        D *= fp_int(Dd);
-    } else {
-        mask = strip_all(x, D, std::make_index_sequence<NSMOOTH - 1>());
-    }
+    const u64 odd = (p - 1) >> v2;
+    typename std::conditional<FP, double, u64>::type o;
+    if constexpr (FP) o = fp_exact(odd);
+    else o = odd;
+    u64 mask = smooth_mask<1, NSMALL>(o);
+    if (job->split > 64) mask |= smooth_mask<NSMALL, NSMOOTH>(o);
+    u64 x = odd;
+    for (u64 m = mask; m; m &= m - 1) x = without(x, c_tab.smooth[__ffsll((long long)m) - 1]);
+    const u64 D = (p - 1) / x;
     mask |= 1;                                            // p is odd
     // chi(b) = b^x and its order eo | D, one prime of D at a time: the power by
     // D without that prime has the order's part of it
@@ -335,7 +359,7 @@ __device__ __forceinline__ void setup_prime_any(const JobDev *__restrict__ job, 
     else setup_prime_one<false>(job, p, t, jb, hdr, aux);
 }
 template <int KIND>
-__global__ void __launch_bounds__(128) k_setup_prime(const JobDev *__restrict__ jobs, const u64 *__restrict__ primes,
+__global__ void __launch_bounds__(128, 8) k_setup_prime(const JobDev *__restrict__ jobs, const u64 *__restrict__ primes,
                                                      u32 first, u32 count, PrimeHdr *__restrict__ hdr,
                                                      PrimeAux *__restrict__ aux,
                                                      const BatchRange *__restrict__ ranges,
@@ -702,52 +726,56 @@ __device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float p, u32
 template <bool FP>
 __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u32 t, PrimeHdr *__restrict__ hdr,
                                                const PrimeAux *__restrict__ aux, u64 *__restrict__ tabs,
-                                               u32 &n_targets, u32 &n_full, u32 &n_split)
+                                               u64 (*tile)[33], bool run, u32 &n_targets, u32 &n_full, u32 &n_split)
 {
+    const u32 lane = threadIdx.x & 31;
     typedef Field<FP> F;
     typedef typename F::V V;
     PrimeHdr &h = hdr[t];
     const F f(h, aux[t]);
-    const u32 e = h.e, nk = h.numk, cls = h.cls, gs = 32u << cls, lq = 9 + cls;
+    const u32 e = run ? h.e : 1, nk = run ? h.numk : 1, cls = run ? h.cls : 0, gs = 32u << cls, lq = 9 + cls;
     const u32 Le = (job->L + e - 1) / e;
     const u32 Mg = (Le + (1u << lq) - 1) >> lq;
     u32 G, Lc, nseg, rounds;
     giant_split(gs, nk, Mg, (float)h.p, G, Lc, nseg, rounds);
+    const V s = F::val(h.s), S = F::val(aux[t].S[cls]);          // (not a record's when !run: never stored)
+    V u8 = f.mul(s, s);
+    u8 = f.mul(u8, u8);
+    u8 = f.mul(u8, u8);
+    const V u = f.mul(u8, u8), z = power<FP>(f, S, Lc);
+    const u32 nb = gs >> 5, nz1 = min(G, 32u), nz2 = (G + 31) >> 5;
+    // n powers of x into row `lane` of the warp's tile, then the rows out to the
+    // lanes' records at offset o, a row at a time (one thread's own stores would
+    // touch a line each); returns x^n (z^32 is needed only when G > 32, and then
+    // the Z1 table runs to 32 entries)
+    auto table = [&](V x, u32 n, u32 o) -> V {
+        if (!run) n = 0;
+        V a = f.one();
+        for (u32 l = 0; __any_sync(0xFFFFFFFFu, l < n); ++l) {
+            if (l >= n) continue;
+            tile[lane][l] = F::bits(a);
+            a = f.mul(a, x);
+        }
+        __syncwarp();
+#pragma unroll 4
+        for (u32 r = 0; r < 32; ++r) {
+            const u32 tr = __shfl_sync(0xFFFFFFFFu, t, r), nr = __shfl_sync(0xFFFFFFFFu, n, r);
+            if (lane < nr) tabs[(size_t)tr * TABS + o + lane] = tile[r][lane];
+        }
+        __syncwarp();
+        return a;
+    };
+    const V u32p = table(u, 32, 0);
+    const V z32 = table(z, nz1, 64);
+    table(u32p, nb, 32);
+    table(z32, nz2, 96);
+    if (!run) return;
     h.G = G;
     h.Lc = Lc;
     h.Mg = Mg;
     h.rk = 1.0f / (float)nk;
     h.nseg = nseg;
     h.rounds = rounds;
-    const V s = F::val(h.s), S = F::val(aux[t].S[cls]);
-    V u8 = f.mul(s, s);
-    u8 = f.mul(u8, u8);
-    u8 = f.mul(u8, u8);
-    const V u = f.mul(u8, u8), z = power<FP>(f, S, Lc);
-    u64 *tb = tabs + (size_t)t * TABS;
-    const u32 nb = gs >> 5, nz1 = min(G, 32u), nz2 = (G + 31) >> 5;
-    V a = f.one(), b = a;
-    for (u32 l = 0; l < 32; ++l) {
-        tb[l] = F::bits(a);
-        a = f.mul(a, u);
-        if (l < nz1) {
-            tb[64 + l] = F::bits(b);
-            b = f.mul(b, z);
-        }
-    }
-    // (z^32 is needed only when G > 32, and then the Z1 chain has run all 32 steps)
-    const V u32p = a, z32 = b;
-    a = b = f.one();
-    for (u32 l = 0; l < max(nb, nz2); ++l) {
-        if (l < nb) {
-            tb[32 + l] = F::bits(a);
-            a = f.mul(a, u32p);
-        }
-        if (l < nz2) {
-            tb[96 + l] = F::bits(b);
-            b = f.mul(b, z32);
-        }
-    }
     h.S = F::bits(S);
     h.u8 = F::bits(u8);
     if constexpr (FP) {
@@ -763,7 +791,7 @@ __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u
 // Kernel 3: one thread per prime (indexing as kernel 1); then the record's index
 // goes on the list of its class (ANY_PRIMES: of its job's group and step kind).
 template <int KIND>
-__global__ void __launch_bounds__(128) k_setup_tabs(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
+__global__ void __launch_bounds__(128, 8) k_setup_tabs(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
                                                     const PrimeAux *__restrict__ aux, u32 count,
                                                     u64 *__restrict__ tabs, u64 *__restrict__ stats,
                                                     u32 *__restrict__ lists, u32 list_stride, u32 *list_ctl,
@@ -775,6 +803,8 @@ __global__ void __launch_bounds__(128) k_setup_tabs(const JobDev *__restrict__ j
     const u32 stride = gridDim.x * blockDim.x;
     const u32 lane = threadIdx.x & 31;
     const u32 total = BATCH ? prefix[nr] : count;
+    __shared__ u64 s_tile[128 / 32][32][33];
+    u64 (*tile)[33] = s_tile[threadIdx.x >> 5];
     u32 nt = 0, nf = 0, ns = 0;
     // i0 is uniform over the warp, so that the list claims below stay whole
     for (u32 i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < total; i0 += stride) {
@@ -782,11 +812,14 @@ __global__ void __launch_bounds__(128) k_setup_tabs(const JobDev *__restrict__ j
         const u32 rec = (i < total) ? (BATCH ? rec_of[i] : i) : 0;
         const bool live = i < total && hdr[rec].p != 0;
         u32 key = 0xFFFFFFFFu;                             // list of the record: group * NCLASS + class
+        const u64 p = hdr[rec].p;
+        const u32 jb = BATCH ? hdr[rec].job : 0;
+        const bool fp = KIND == FP_PRIMES || (BATCH && p < FP_BOUND);
+        if (KIND != INT_PRIMES && __any_sync(0xFFFFFFFFu, live && fp))
+            setup_tabs_one<true>(jobs + jb, rec, hdr, aux, tabs, tile, live && fp, nt, nf, ns);
+        if (KIND != FP_PRIMES && __any_sync(0xFFFFFFFFu, live && !fp))
+            setup_tabs_one<false>(jobs + jb, rec, hdr, aux, tabs, tile, live && !fp, nt, nf, ns);
         if (live) {
-            const u32 jb = BATCH ? hdr[rec].job : 0;
-            const u64 p = hdr[rec].p;
-            if (KIND == FP_PRIMES || (BATCH && p < FP_BOUND)) setup_tabs_one<true>(jobs + jb, rec, hdr, aux, tabs, nt, nf, ns);
-            else setup_tabs_one<false>(jobs + jb, rec, hdr, aux, tabs, nt, nf, ns);
             const u32 g = BATCH ? geoms[jb].group + (p < FP_BOUND ? 2u : (p >> 63) ? 0u : 1u) : 0u;
             key = g * NCLASS + hdr[rec].cls;
         }
