@@ -401,7 +401,7 @@ static int gen_segment(rs_ctx *c, u64 lo, u64 hi, u32 *np, bool *overflow)
     CU(cudaMemsetAsync(c->d_ctrs, 0, 2 * 4, c->stream));
     CU(cudaMemsetAsync(c->d_ctrs + 4, 0, 4, c->stream));
     CU(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
-    CU(launch_sieve(base, nodd, hi, c->d_sp, c->nsp, c->d_cands, c->cand_cap, c->d_ctrs, c->d_err, c->stream));
+    CU(launch_sieve(base, nodd, c->d_sp, c->nsp, c->d_cands, c->cand_cap, c->d_ctrs, c->d_err, c->sms, c->stream));
     CU(launch_mr2(c->d_cands, c->d_ctrs, c->cand_cap, c->d_primes, c->prime_cap, c->d_ctrs + 1, c->d_mid,
                   c->d_ctrs + 4, c->d_err, c->sms, c->stream));
     CU(cudaMemcpyAsync(c->h_pin, c->d_ctrs, 2 * 4, cudaMemcpyDeviceToHost, c->stream));

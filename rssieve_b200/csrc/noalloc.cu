@@ -7,13 +7,15 @@
 // rs_primes_generate keeps these in its context, allocated with cudaMalloc.
 // This variant keeps them in one file-scope device array of fixed size,
 // g_na_scratch below, so a call allocates nothing; the caller passes the
-// output array and the count word.  It runs the one-pass form of the test
-// (k_mr), which needs no second list of base-2 probable primes; the primes it
-// returns are the same.
+// output array and the count word.
 //
 // Limit: a call covers at most RS_NOALLOC_MAX_WIDTH = 2^22 integers, i.e. at
-// most 2^21 odd values, which is exactly the survivor capacity, so the
-// survivor buffer can never overflow.  Wider ranges are rejected with RS_EARG.
+// most 2^21 odd values.  Survivors are coprime to 3, 5 and 7 or among them (a
+// window that reaches 49 is sieved by all three, and one that does not has at
+// most 24 odd values), i.e. at most 48 in every run of 105 odd values, below
+// 2^21 * 48/105 + 105 < 2^20: the survivor list and the list of base-2 probable
+// primes each take half of the array and can never overflow.  Wider ranges are
+// rejected with RS_EARG.
 //
 // Set-up: the first call in a CUDA context (the primary context of the device
 // current on the calling thread, or the driver-API context made current)
@@ -42,14 +44,14 @@ using namespace rs;
 
 namespace {
 
-constexpr u32 NA_CAND_CAP = 1u << 21;        // survivor slots (u64 each): 16 MiB
+constexpr u32 NA_CAND_CAP = 1u << 20;        // survivor slots, and as many for the base-2 probable primes (u64 each): 16 MiB
 constexpr u32 NA_SP_SLOTS = 6656;            // u32 slots for the 6541 odd primes < 2^16
 constexpr u32 NA_NSP = 6541;                 // pi(2^16) - 1
-constexpr u32 NA_CTR_SLOTS = 64;             // u32: [0] survivors [1] error flags [2] set-up count
-constexpr size_t NA_WORDS = NA_CAND_CAP + NA_SP_SLOTS / 2 + NA_CTR_SLOTS / 2;
-static_assert(RS_NOALLOC_MAX_WIDTH / 2 == NA_CAND_CAP, "survivor capacity must cover every odd value of a call");
+constexpr u32 NA_CTR_SLOTS = 64;             // u32: [0] survivors [1] error flags [2] set-up count [3] probable primes
+constexpr size_t NA_WORDS = 2 * NA_CAND_CAP + NA_SP_SLOTS / 2 + NA_CTR_SLOTS / 2;
+static_assert(RS_NOALLOC_MAX_WIDTH / 2 * 48 / 105 + 105 < NA_CAND_CAP, "survivor capacity must cover every call");
 
-// The scratch: survivors, then sieving primes, then counters (all offsets
+// The scratch: survivors, base-2 probable primes, sieving primes, counters (all offsets
 // are multiples of 256 bytes).
 static __device__ __align__(256) u64 g_na_scratch[NA_WORDS];
 
@@ -153,7 +155,7 @@ int na_setup(int dev, void *ptr, cudaStream_t st, CtxState *out)
     int sms = 0;
     NA_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     u64 *scr = (u64 *)ptr;
-    u32 *sp = (u32 *)(scr + NA_CAND_CAP);
+    u32 *sp = (u32 *)(scr + 2 * NA_CAND_CAP);
     u32 *ctrs = sp + NA_SP_SLOTS;
     k_na_small_primes<<<1, 1024, 0, st>>>(sp, ctrs + 2);
     NA_CU(cudaGetLastError());
@@ -229,15 +231,16 @@ extern "C" int rs_primes_generate_noalloc(uint64_t p0, uint64_t p1, uint64_t *d_
         ds = g_na_ctx[slot];
     }
     u64 *cands = ds.scratch;
-    u32 *sp = (u32 *)(ds.scratch + NA_CAND_CAP);
+    u64 *mid = ds.scratch + NA_CAND_CAP;
+    u32 *sp = (u32 *)(ds.scratch + 2 * NA_CAND_CAP);
     u32 *ctrs = sp + NA_SP_SLOTS;
     if (p0 < 3) p0 = 3;
     u64 base = p0 | 1ull;
     u64 nodd = (base < p1) ? (p1 - base + 1) / 2 : 0;
-    NA_CU(cudaMemsetAsync(ctrs, 0, 2 * sizeof(u32), st));
+    NA_CU(cudaMemsetAsync(ctrs, 0, 4 * sizeof(u32), st));
     NA_CU(cudaMemsetAsync(d_count, 0, sizeof(u32), st));
     if (nodd == 0) return RS_OK;
-    NA_CU(launch_sieve(base, nodd, p1, sp, NA_NSP, cands, NA_CAND_CAP, ctrs, ctrs + 1, st));
-    NA_CU(launch_mr(cands, ctrs, NA_CAND_CAP, (u64 *)d_primes, cap, d_count, ctrs + 1, ds.sms, st));
+    NA_CU(launch_sieve(base, nodd, sp, NA_NSP, cands, NA_CAND_CAP, ctrs, ctrs + 1, ds.sms, st));
+    NA_CU(launch_mr2(cands, ctrs, NA_CAND_CAP, (u64 *)d_primes, cap, d_count, mid, ctrs + 3, ctrs + 1, ds.sms, st));
     return RS_OK;
 }

@@ -80,7 +80,7 @@ int tuned_geom_get(int device, u64 shape);
 void tuned_geom_put(int device, u64 shape, int geom);
 constexpr int SETUP_TPB = 256;              // 8 warps per block
 constexpr int SIEVE_TPB = 512;
-constexpr int SIEVE_WORDS = 4096;           // 2^17 odd numbers per sieve block
+constexpr int SIEVE_WORDS = 4096;           // 2^17 odd numbers per sieve block at most
 constexpr u64 MR_BOUND = 4295098369ULL;     // 65537^2: below it the sieve by all primes < 2^16 is exact
 
 // error bits (JobDev-independent, one word per context)
@@ -225,12 +225,10 @@ __device__ __forceinline__ u32 prefix_find(const u32 *prefix, u32 nr, u32 i)
 }
 
 // launch wrappers (sieve.cu, setup.cu, bsgs.cu)
-cudaError_t launch_sieve(u64 base_odd, u64 nodd, u64 hi, const u32 *sp, u32 nsp, u64 *cands, u32 cand_cap,
-                         u32 *ctrs, u32 *err, cudaStream_t st);
-cudaError_t launch_mr(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *primes, u32 prime_cap, u32 *prime_ctr,
-                      u32 *err, int sms, cudaStream_t st);
-// the same test in two passes (base 2 into mid, then Lucas over mid); mid
-// holds cand_cap values and *mid_ctr starts at zero
+cudaError_t launch_sieve(u64 base_odd, u64 nodd, const u32 *sp, u32 nsp, u64 *cands, u32 cand_cap, u32 *ctrs, u32 *err,
+                         int sms, cudaStream_t st);
+// Baillie-PSW in two passes (base 2 into mid, then Lucas over mid); mid holds
+// cand_cap values and *mid_ctr starts at zero
 cudaError_t launch_mr2(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *primes, u32 prime_cap, u32 *prime_ctr,
                        u64 *mid, u32 *mid_ctr, u32 *err, int sms, cudaStream_t st);
 // (lists: NCLASS lists of at least count records; the counts in lists.ctl start at

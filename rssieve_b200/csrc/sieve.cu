@@ -8,7 +8,7 @@
 // prime below 2^16, compacts the survivors with warp ballots/popc, and a
 // second kernel proves the survivors at or above 65537^2 prime with the
 // Baillie-PSW test (a base-2 strong probable-prime test, then a strong Lucas
-// test; deterministic below 2^64, see is_prime_bpsw).  Survivors below
+// test; deterministic below 2^64, see below).  Survivors below
 // 65537^2 are prime already.  The result is the exact set of odd primes in
 // [lo, hi).
 #include "mont.cuh"
@@ -16,26 +16,26 @@
 
 namespace rs {
 
-// x mod r for a 64-bit x and a 32-bit r, from three 32-bit remainders.
-__device__ __forceinline__ u32 mod64_32(u64 x, u32 r)
+// x mod r for x < 2^32 and r < 2^16, rinv = 1/r to 2^-40: x*rinv rounded to an
+// integer (read off the mantissa) is the quotient or one more.
+__device__ __forceinline__ u32 mod_small(u32 x, u32 r, double rinv)
 {
-    u32 hi = (u32)(x >> 32), lo = (u32)x;
-    u32 t = (u32)(0u - r) % r;            // 2^32 mod r
-    u64 a = (u64)(hi % r) * t + (lo % r); // < r^2 + r < 2^33
-    return (u32)(a % r);
+    const double two52 = 4503599627370496.0;
+    const u32 q = (u32)__double2loint(fma(__hiloint2double(0x43300000, (int)x) - two52, rinv, two52));
+    const u32 m = x - q * r;
+    return ((int)m < 0) ? m + r : m;
 }
 
-// One CTA sieves odd values base_odd + 2*i for i in [blk*BITS, blk*BITS+nbits).
-// ctrs[0] counts survivors written to cands.  The caller's exit test is
-// uniform over the CTA.
-__device__ __forceinline__ void sieve_block(u64 base_odd, u64 nodd, u32 blk, const u32 *__restrict__ sp, u32 nsp,
-                                            u64 *__restrict__ cands, u32 cand_cap, u32 *ctrs, u32 *err)
+// One CTA sieves odd values base_odd + 2*i for i in [blk*bits, (blk+1)*bits),
+// bits = 32*words, words <= SIEVE_WORDS.  ctrs[0] counts survivors written to
+// cands.  The caller's exit test is uniform over the CTA.
+__device__ __forceinline__ void sieve_block(u64 base_odd, u64 nodd, u32 blk, u32 words, const u32 *__restrict__ sp,
+                                            u32 nsp, u64 *__restrict__ cands, u32 cand_cap, u32 *ctrs, u32 *err)
 {
-    constexpr u32 BITS = SIEVE_WORDS * 32;
     __shared__ u32 bits[SIEVE_WORDS];
     __shared__ u32 starts[7000];
-    const u32 tid = threadIdx.x;
-    const u64 i0 = (u64)blk * BITS;
+    const u32 tid = threadIdx.x, lane = tid & 31;
+    const u64 i0 = (u64)blk * words * 32;
     if (i0 >= nodd) return;
     // the table must start with 3: an empty or zeroed table would make the
     // one-prime-per-thread marking loop below step by 0 forever
@@ -43,28 +43,14 @@ __device__ __forceinline__ void sieve_block(u64 base_odd, u64 nodd, u32 blk, con
         if (tid == 0) atomicOr(err, ERR_SIEVE_TABLE);
         return;
     }
-    const u32 nbits = (u32)min((u64)BITS, nodd - i0);
+    const u32 nbits = (u32)min((u64)words * 32, nodd - i0);
     const u64 bb = base_odd + 2 * i0;                   // value of bit 0 (odd)
     const u64 vlast = bb + 2 * (u64)(nbits - 1);
-    for (u32 w = tid; w < SIEVE_WORDS; w += SIEVE_TPB) bits[w] = 0;
+    for (u32 w = tid; w < words; w += SIEVE_TPB) bits[w] = 0;
 
-    // first index to mark for each sieving prime r with r^2 <= vlast
-    u32 np_used = 0;
-    for (u32 k = tid; k < nsp; k += SIEVE_TPB) {
-        u32 r = sp[k];
-        u64 rr = (u64)r * r;
-        u32 s = 0xFFFFFFFFu;
-        if (rr <= vlast) {
-            u32 m = mod64_32(bb, r);
-            u32 j = (u32)(((u64)((r - m) % r) * ((r + 1) >> 1)) % r);   // bb + 2j == 0 (mod r)
-            u64 v = bb + 2 * (u64)j;
-            if (v < rr) j = (u32)((rr - bb) >> 1);                     // start at r^2, never at r
-            if ((u64)j < nbits) s = j;
-        }
-        starts[k] = s;
-    }
     // number of primes with r^2 <= vlast (sp is ascending)
-    {
+    u32 np_used = nsp;
+    if (vlast < MR_BOUND) {
         u32 lo = 0, hi2 = nsp;
         while (lo < hi2) {
             u32 mid = (lo + hi2) >> 1;
@@ -72,26 +58,52 @@ __device__ __forceinline__ void sieve_block(u64 base_odd, u64 nodd, u32 blk, con
         }
         np_used = lo;
     }
+    // first index to mark for each of them: bb + 2j == 0 (mod r), and at least r^2
+    const u32 b2 = (u32)(bb >> 32), b1 = (u32)(bb >> 16) & 0xFFFFu, b0 = (u32)bb & 0xFFFFu;
+    for (u32 k = tid; k < np_used; k += SIEVE_TPB) {
+        const u32 r = sp[k];
+        const double rd = (double)r, r0 = (double)(1.0f / (float)r), rinv = r0 * (2.0 - rd * r0);
+        u32 m = mod_small(b2, r, rinv);
+        m = mod_small((m << 16) | b1, r, rinv);
+        m = mod_small((m << 16) | b0, r, rinv);
+        const u32 d = m ? r - m : 0;
+        u64 j = (d & 1) ? (d + r) >> 1 : d >> 1;
+        const u64 rr = (u64)r * r;
+        if (bb + 2 * j < rr) j = (rr - bb) >> 1;        // start at r^2, never at r
+        starts[k] = (j < nbits) ? (u32)j : 0xFFFFFFFFu;
+    }
     __syncthreads();
 
-    // small primes: all threads stride over the multiples of one prime
+    // small primes: all threads stride over the multiples of one prime; medium
+    // ones a warp each, large ones a thread each (a round of the wider form would
+    // leave most threads without a multiple)
     u32 k = 0;
-    for (; k < np_used && sp[k] < 2 * SIEVE_TPB; ++k) {
-        u32 r = sp[k], s = starts[k];
-        if (s == 0xFFFFFFFFu) continue;
-        for (u32 i = s + tid * r; i < nbits; i += SIEVE_TPB * r) atomicOr(&bits[i >> 5], 1u << (i & 31));
+    for (; k < np_used && sp[k] * SIEVE_TPB < nbits; ++k) {
+        const u32 r = sp[k];
+        for (u32 i = starts[k] + tid * r; i < nbits && starts[k] != 0xFFFFFFFFu; i += SIEVE_TPB * r)
+            atomicOr(&bits[i >> 5], 1u << (i & 31));
     }
-    // large primes: one prime per thread
-    for (u32 kk = k + tid; kk < np_used; kk += SIEVE_TPB) {
-        u32 r = sp[kk], s = starts[kk];
-        for (u32 i = s; i < nbits; i += r) atomicOr(&bits[i >> 5], 1u << (i & 31));
+    u32 kw = k + (tid >> 5);
+    for (; kw < np_used && sp[kw] * 32 < nbits; kw += SIEVE_TPB / 32) {
+        const u32 r = sp[kw], s = starts[kw];
+        if (s == 0xFFFFFFFFu) continue;
+        for (u32 i = s + lane * r; i < nbits; i += 32 * r) atomicOr(&bits[i >> 5], 1u << (i & 31));
+    }
+    // the first large prime, the same for every warp: those below nbits/32 are taken
+    u32 lo = k, hi2 = np_used;
+    while (lo < hi2) {
+        const u32 mid = (lo + hi2) >> 1;
+        if (sp[mid] * 32 < nbits) lo = mid + 1; else hi2 = mid;
+    }
+    for (u32 kk = lo + tid; kk < np_used; kk += SIEVE_TPB) {
+        const u32 r = sp[kk];
+        for (u32 i = starts[kk]; i < nbits; i += r) atomicOr(&bits[i >> 5], 1u << (i & 31));
     }
     __syncthreads();
 
     // warp-ballot / popc compaction of the unmarked (prime or MR-candidate) values
-    const u32 lane = tid & 31;
     const u32 nw = (nbits + 31) >> 5;
-    for (u32 w0 = 0; w0 < SIEVE_WORDS; w0 += SIEVE_TPB) {
+    for (u32 w0 = 0; w0 < nw; w0 += SIEVE_TPB) {
         u32 w = w0 + tid;
         u32 live = 0;
         if (w < nw) {
@@ -124,10 +136,11 @@ __device__ __forceinline__ void sieve_block(u64 base_odd, u64 nodd, u32 blk, con
     }
 }
 
-__global__ void __launch_bounds__(SIEVE_TPB) k_sieve(u64 base_odd, u64 nodd, const u32 *__restrict__ sp, u32 nsp,
-                                                     u64 *__restrict__ cands, u32 cand_cap, u32 *ctrs, u32 *err)
+__global__ void __launch_bounds__(SIEVE_TPB) k_sieve(u64 base_odd, u64 nodd, u32 words, const u32 *__restrict__ sp,
+                                                     u32 nsp, u64 *__restrict__ cands, u32 cand_cap, u32 *ctrs,
+                                                     u32 *err)
 {
-    sieve_block(base_odd, nodd, blockIdx.x, sp, nsp, cands, cand_cap, ctrs, err);
+    sieve_block(base_odd, nodd, blockIdx.x, words, sp, nsp, cands, cand_cap, ctrs, err);
 }
 
 // Batch round: blockIdx.y is the range; its window and buffers come from the
@@ -138,7 +151,8 @@ __global__ void __launch_bounds__(SIEVE_TPB) k_sieve_batch(const BatchWin *__res
 {
     const u32 r = blockIdx.y;
     const BatchWin w = wins[r];
-    sieve_block(w.base_odd, w.nodd, blockIdx.x, sp, nsp, cands + (size_t)r * ccap, ccap, ctrs + r * BR_CTRS, err);
+    sieve_block(w.base_odd, w.nodd, blockIdx.x, SIEVE_WORDS, sp, nsp, cands + (size_t)r * ccap, ccap,
+                ctrs + r * BR_CTRS, err);
 }
 
 // Strong probable prime to base a (a < n), n - 1 = d * 2^t with d odd.
@@ -320,6 +334,32 @@ __device__ __forceinline__ bool sprp2(u64 n, const Mont &M, u64 d, int t)
     return false;
 }
 
+// sprp2 for n < 2^51 on the FP64 pipe, on plain residues (0.16 -> 0.07 ns per prime
+// found near 10^12).
+__device__ __forceinline__ bool sprp2_fp(u64 n, u64 d, int t)
+{
+    const double nd = fp_exact(n), ninv = 1.0 / nd, mone = nd - 1.0;
+    double x = 2.0;
+    for (int bit = 62 - __clzll(d); bit >= 0; --bit) {
+        x = fp_mul(x, x, nd, ninv);
+        const double x2 = fp_dbl(x, nd);
+        x = ((d >> bit) & 1) ? x2 : x;
+    }
+    if (x == 1.0 || x == mone) return true;
+    for (int i = 1; i < t; ++i) {
+        x = fp_mul(x, x, nd, ninv);
+        if (x == mone) return true;
+    }
+    return false;
+}
+
+// The base-2 test on the pipe that suits n (n odd, above 65537^2).
+__device__ __forceinline__ bool base2_test(u64 n)
+{
+    const int t = __ffsll((long long)(n - 1)) - 1;
+    return (n < FP_BOUND) ? sprp2_fp(n, (n - 1) >> t, t) : sprp2(n, mont_init(n), (n - 1) >> t, t);
+}
+
 // Deterministic primality of a sieve survivor below 2^64 (Baillie-PSW): a
 // strong probable prime to base 2 that also passes the strong Lucas test with
 // Selfridge's parameters.  No composite below 2^64 passes both: J. Feitsma and
@@ -330,17 +370,6 @@ __device__ __forceinline__ bool sprp2(u64 n, const Mont &M, u64 d, int t)
 // the verification that makes BPSW a deterministic test in that range).  About
 // 3.5 Miller-Rabin rounds of work per prime instead of the seven bases of
 // is_prime_mr, which remains the answer when no Lucas parameter is found.
-__device__ bool is_prime_bpsw(u64 n)
-{
-    if (n < MR_BOUND) return true;        // sieve survivor below 65537^2
-    if (n == ~0ull) return false;         // 2^64 - 1 = 3 * 5 * 17 * 257 * 641 * 65537 * 6700417
-    const Mont M = mont_init(n);
-    const u64 nm1 = n - 1;
-    const int t = __ffsll((long long)nm1) - 1;
-    if (!sprp2(n, M, nm1 >> t, t)) return false;
-    const int l = lucas_strong(n, M);
-    return (l >= 0) ? (l == 1) : is_prime_mr(n);
-}
 
 // Appends v of the lanes with keep set to list[*ctr ...] with one atomic per
 // warp (ballot compaction); flags err and drops the warp's values when the
@@ -361,34 +390,7 @@ __device__ __forceinline__ void warp_push(bool keep, u64 v, u64 *__restrict__ li
     if (keep) list[basepos + __popc(mask & ((1u << lane) - 1))] = v;
 }
 
-// Warp-stride Baillie-PSW over cands[0, min(*cand_ctr, cand_cap)) with ballot compaction into primes.
-__device__ __forceinline__ void mr_list(const u64 *__restrict__ cands, const u32 *cand_ctr, u32 cand_cap,
-                                        u64 *__restrict__ primes, u32 prime_cap, u32 *prime_ctr, u32 *err)
-{
-    const u32 n = min(*cand_ctr, cand_cap);
-    const u32 lane = threadIdx.x & 31;
-    const u32 warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const u32 nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (u32 b0 = warp * 32; b0 < n; b0 += nwarps * 32) {
-        const u32 idx = b0 + lane;
-        u64 v = 0;
-        bool pr = false;
-        if (idx < n) {
-            v = cands[idx];
-            pr = is_prime_bpsw(v);
-        }
-        warp_push(pr, v, primes, prime_cap, prime_ctr, err, ERR_PRIME_OVERFLOW);
-    }
-}
-
-__global__ void __launch_bounds__(256) k_mr(const u64 *__restrict__ cands, const u32 *__restrict__ ctrs,
-                                            u32 cand_cap, u64 *__restrict__ primes, u32 prime_cap, u32 *prime_ctr,
-                                            u32 *err)
-{
-    mr_list(cands, ctrs, cand_cap, primes, prime_cap, prime_ctr, err);
-}
-
-// The same test in two passes, so that the Lucas ladder runs on full warps.
+// The test runs in two passes, so that the Lucas ladder runs on full warps.
 // About 57% of the survivors of a sieve by the primes below 2^16 are prime at
 // p near 2^50 (Mertens: 1/ln p over e^-gamma/ln 2^16), and the base-2 test
 // rejects almost every composite; in one pass a warp runs the Lucas ladder
@@ -413,9 +415,7 @@ __global__ void __launch_bounds__(256) k_mr_sprp(const u64 *__restrict__ cands, 
             if (v < MR_BOUND) {
                 small = true;
             } else if (v != ~0ull) {       // 2^64 - 1 = 3 * 5 * 17 * 257 * 641 * 65537 * 6700417
-                const Mont M = mont_init(v);
-                const int t = __ffsll((long long)(v - 1)) - 1;
-                pass = sprp2(v, M, (v - 1) >> t, t);
+                pass = base2_test(v);
             }
         }
         warp_push(small, v, primes, prime_cap, prime_ctr, err, ERR_PRIME_OVERFLOW);
@@ -471,9 +471,7 @@ __global__ void __launch_bounds__(256) k_mr_batch_sprp(const u64 *__restrict__ c
                 if (pos < rcap) primes[(size_t)r * rcap + pos] = v;
                 else atomicOr(err, ERR_PRIME_OVERFLOW);
             } else if (v != ~0ull) {
-                const Mont M = mont_init(v);
-                const int t = __ffsll((long long)(v - 1)) - 1;
-                pass = sprp2(v, M, (v - 1) >> t, t);
+                pass = base2_test(v);
             }
         }
         const u32 mask = __ballot_sync(0xFFFFFFFFu, pass);
@@ -536,14 +534,18 @@ __global__ void k_batch_windows(BatchRange *ranges, BatchWin *wins, const u32 *w
     for (int i = 0; i < BR_CTRS; ++i) ctrs[r * BR_CTRS + i] = 0;
 }
 
-cudaError_t launch_sieve(u64 base_odd, u64 nodd, u64 hi, const u32 *sp, u32 nsp, u64 *cands, u32 cand_cap, u32 *ctrs,
-                         u32 *err, cudaStream_t st)
+// Blocks of 2^17 odd values, smaller (down to 2^13) while there are fewer than two
+// per SM: a small window waits for its one block (2^15 odd values near 2^50: 46 us in
+// one block, 16 in four), and every block reduces the window's start by all 6541
+// sieving primes, so larger ones are cheaper where they fill the chip.
+cudaError_t launch_sieve(u64 base_odd, u64 nodd, const u32 *sp, u32 nsp, u64 *cands, u32 cand_cap, u32 *ctrs, u32 *err,
+                         int sms, cudaStream_t st)
 {
-    (void)hi;
     if (nodd == 0) return cudaSuccess;
-    constexpr u64 BITS = (u64)SIEVE_WORDS * 32;
-    u64 blocks = (nodd + BITS - 1) / BITS;
-    k_sieve<<<(unsigned)blocks, SIEVE_TPB, 0, st>>>(base_odd, nodd, sp, nsp, cands, cand_cap, ctrs, err);
+    u32 words = SIEVE_WORDS;
+    while (words > 256 && nodd < (u64)words * 32 * 2 * sms) words /= 2;
+    const u64 blocks = (nodd + words * 32 - 1) / (words * 32);
+    k_sieve<<<(unsigned)blocks, SIEVE_TPB, 0, st>>>(base_odd, nodd, words, sp, nsp, cands, cand_cap, ctrs, err);
     return cudaGetLastError();
 }
 
@@ -568,13 +570,6 @@ cudaError_t launch_mr_batch2(const u64 *cands, u32 ccap, u64 *primes, u32 rcap, 
     k_mr_batch_sprp<<<sms * 8, 256, 0, st>>>(cands, ccap, primes, rcap, ctrs, prefix_c, nranges, mid, mid_r, mid_cap,
                                               mid_ctr, err);
     k_mr_batch_lucas<<<sms * 8, 256, 0, st>>>(mid, mid_r, mid_cap, mid_ctr, primes, rcap, ctrs, err);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_mr(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *primes, u32 prime_cap, u32 *prime_ctr,
-                      u32 *err, int sms, cudaStream_t st)
-{
-    k_mr<<<sms * 8, 256, 0, st>>>(cands, ctrs, cand_cap, primes, prime_cap, prime_ctr, err);
     return cudaGetLastError();
 }
 
