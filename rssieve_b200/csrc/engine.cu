@@ -525,7 +525,7 @@ extern "C" int rs_run_range(rs_ctx *c, uint64_t p0, uint64_t p1, rs_counters *de
             c->chunk_geom[ci] = g;
             CU(cudaMemsetAsync(c->lists.ctl, 0, 2 * NCLASS * 4, c->stream));
             CU(launch_setup(c->d_job, c->h_job.kcount, c->d_primes, first, cnt, hi, c->d_hdr, c->d_aux, c->d_tabs,
-                            c->d_tgt, c->d_meta, c->lists, c->d_stats, g, c->stream));
+                            c->d_tgt, c->d_meta, c->lists, c->d_stats, g, c->sms, c->stream));
             CU(cudaEventRecord(c->ev[2 + 2 * ci], c->stream));
             CU(launch_bsgs(a, c->d_hdr, c->d_tabs, c->d_tgt, c->d_meta, c->lists, p, hi, g, c->sms, c->stream));
             CU(cudaEventRecord(c->ev[3 + 2 * ci], c->stream));

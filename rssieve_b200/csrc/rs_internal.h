@@ -235,7 +235,7 @@ cudaError_t launch_mr2(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *pri
 // zero; the primes lie below pmax, entirely on one side of FP_BOUND)
 cudaError_t launch_setup(const JobDev *job, u32 kcount, const u64 *primes, u32 first, u32 count, u64 pmax, PrimeHdr *hdr,
                          void *aux, u64 *tabs, u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats,
-                         int geom, cudaStream_t st);
+                         int geom, int sms, cudaStream_t st);
 size_t setup_aux_bytes();
 // every prime of the launch lies in [pmin, pmax), entirely below or entirely at or above 2^63
 cudaError_t launch_bsgs(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,

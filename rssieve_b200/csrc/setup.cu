@@ -401,8 +401,9 @@ __device__ __forceinline__ u32 choose_class(const JobGeom &gm, u32 nk, u32 Le)
 }
 
 // a[r] = x[r]^ex for r < R, the chains interleaved.  UNIFORM: ex (>= 1) is the
-// same for every lane, so the loop branches on it: a sliding window of two bits,
-// 1.33 products per bit.  Else as power().
+// same for every lane, so the loop branches on it: by two-bit digits, 1.375 products
+// per bit, or for integers, whose products cost more than the loop, by a sliding
+// window of two bits, 1.33.  Else as power().
 template <bool FP, int R, bool UNIFORM, bool LAZY>
 __device__ __forceinline__ void power_chains_as(const Field<FP> &F, typename Field<FP>::V (&a)[2],
                                                 const typename Field<FP>::V (&x)[2], u64 ex)
@@ -414,7 +415,35 @@ __device__ __forceinline__ void power_chains_as(const Field<FP> &F, typename Fie
         x2[r] = F.template psqr<LAZY>(x[r]);
         x3[r] = F.template pmul<LAZY>(x2[r], x[r]);
     }
-    if constexpr (UNIFORM) {
+    if constexpr (UNIFORM && FP) {
+        // the exponent's digits from the top, two bits each, at the top of t
+        const u32 n = (65 - __clzll(ex)) >> 1;             // digits
+        u64 t = ex << (64 - 2 * n);
+        u32 d = (u32)(t >> 62);                            // 1..3
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[r] = d == 1 ? x[r] : d == 2 ? x2[r] : x3[r];
+#pragma unroll 1
+        for (u32 i = 1; i < n; ++i) {
+            t <<= 2;
+            d = (u32)(t >> 62);
+#pragma unroll
+            for (int r = 0; r < R; ++r) a[r] = F.template psqr<LAZY>(a[r]);
+#pragma unroll
+            for (int r = 0; r < R; ++r) a[r] = F.template psqr<LAZY>(a[r]);
+            if (d & 1) {
+                if (d & 2) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) a[r] = F.template pmul<LAZY>(a[r], x3[r]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) a[r] = F.template pmul<LAZY>(a[r], x[r]);
+                }
+            } else if (d) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) a[r] = F.template pmul<LAZY>(a[r], x2[r]);
+            }
+        }
+    } else if constexpr (UNIFORM) {
         int i = 63 - __clzll(ex);
         const bool two = i > 0 && ((ex >> (i - 1)) & 1);
 #pragma unroll
@@ -487,15 +516,57 @@ __device__ __forceinline__ u32 cls_hash(u64 v, u32 mask)
     return ((((u32)v ^ (u32)(v >> 32)) * 0x9E3779B1u) >> 20) & mask;
 }
 
+// The powers of four primes' last sequences together.  With K = 32R + m sequences,
+// 0 < m <= REST_MAX, a warp's last round of lanes would leave 32 - m of them idle
+// (and for odd R it runs beside another, as the second chain of its lanes, where it
+// costs little: shares_rest);
+// here m8 = 8*ceil(m/8) lanes take a prime's m sequences, so that m8/8 rounds serve
+// four primes (each lane its own exponent, 1.5 products per bit against 1.375).
+// z = k^E goes to the target row of its record until setup_k_one takes it up.
+// Records rec[0..3] (rec[q] valid for q < n), all of one job and step kind.  Called
+// by the whole warp.
+// Measured: 68 sequences near 2^50.6 4.15 -> 3.62 ns per prime, 20 below 2^64 6.44 ->
+// 6.00; 100 (R = 3) 4.76 -> 4.83.
+constexpr u32 REST_MAX = 24;
+__host__ __device__ __forceinline__ bool shares_rest(u32 kcount)
+{
+    const u32 m = kcount & 31;
+    return m != 0 && m <= REST_MAX && ((kcount >> 5) & 1) == 0;
+}
+template <bool FP>
+__device__ __forceinline__ void rest_powers(const JobDev *__restrict__ job, u32 rec, u32 n, const PrimeHdr *hdr,
+                                            const PrimeAux *aux, u64 *tgt)
+{
+    typedef Field<FP> F;
+    const u32 lane = threadIdx.x & 31, m = job->kcount & 31, base = job->kcount - m, m8 = (m + 7) & ~7u;
+    const u32 alive = __ballot_sync(0xFFFFFFFFu, lane < n && hdr[rec].p != 0);
+    if (!alive) return;
+    const u32 any = __ffs((int)alive) - 1;
+#pragma unroll 1
+    for (u32 c = lane; c < 4 * m8; c += 32) {              // (4*m8 is a multiple of 32: the warp stays whole)
+        const u32 q = c / m8, j = c - q * m8;
+        // (lane q holds rec[q]; a lane without work repeats the first live prime's)
+        const u32 w = __shfl_sync(0xFFFFFFFFu, rec, q), w0 = __shfl_sync(0xFFFFFFFFu, rec, any);
+        const bool ok = j < m && q < n && hdr[w].p != 0;
+        const u32 wv = ok ? w : w0;
+        const F f(hdr[wv], aux[wv]);
+        const u64 p = hdr[wv].p, kv = job->k[base + (j < m ? j : 0)];
+        const u64 z = F::bits(power<FP>(f, f.of_int((kv < p) ? kv : kv % p), ok ? aux[wv].E : 1));
+        if (ok) tgt[(size_t)wv * KSTRIDE + j] = z;
+    }
+    __syncwarp();
+}
+
 // Sequence classes, targets and baby-step count of record w, by GL lanes (lane l
 // of them) of a warp; live: the record exists and is not skipped.  GL = 32: up to
-// 128 sequences, four rounds of lanes; GL < 32: at most GL sequences, 32/GL
-// primes side by side in a warp.  Called by the whole warp.
+// 128 sequences, four rounds of lanes (rest: the last, partial round's powers are in
+// the record's target row); GL < 32: at most GL sequences, 32/GL primes side by side
+// in a warp.  Called by the whole warp.
 template <bool FP, u32 GL>
 __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 w, u32 l, bool live,
                                             PrimeHdr *__restrict__ hdr, const PrimeAux *__restrict__ aux,
-                                            u64 *__restrict__ tgt, unsigned short *__restrict__ meta,
-                                            u64 *__restrict__ stats, const JobGeom &gm, KScratch<GL> &sc)
+                                            u64 *tgt, unsigned short *__restrict__ meta,
+                                            u64 *__restrict__ stats, const JobGeom &gm, bool rest, KScratch<GL> &sc)
 {
     typedef Field<FP> F;
     typedef typename F::V V;
@@ -630,7 +701,7 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
         nk += __popc(km);
     };
     if constexpr (GL == 32) {
-        const u32 R = (K + 31) / 32;
+        const u32 R = rest ? K / 32 : (K + 31) / 32;
 #pragma unroll 1
         for (u32 r0 = 0; r0 < R; r0 += 2) {
             V x[2], z[2];
@@ -650,6 +721,11 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
                 power_chains<FP, 1, true>(f, z, x, E);
                 classify(lane + 32 * r0, kr[0], z[0]);
             }
+        }
+        if (rest) {
+            const u32 i = lane + 32 * R;
+            const u64 kv = (i < K) ? job->k[i] : 1;
+            classify(i, (kv < p) ? kv : kv % p, (i < K) ? F::val(tgt[(size_t)w * KSTRIDE + lane]) : f.one());
         }
     } else {
         const u64 kv = (l < K) ? job->k[l] : 1;
@@ -842,12 +918,13 @@ __global__ void __launch_bounds__(128, 8) k_setup_tabs(const JobDev *__restrict_
 }
 
 
-// Kernel 2: GL lanes per prime.  KIND as kernel 1 (ANY_PRIMES: the primes of a
-// batch round, GL = 32).
-template <int KIND, u32 GL>
+// Kernel 2: GL lanes per prime.  KIND as kernel 1.  BATCH: the primes of KIND of a
+// batch round, GL = 32 (one launch per kind: with both in one kernel its registers
+// spilled: 11.9 against 10.2 ms on twelve jobs).
+template <int KIND, u32 GL, bool BATCH = false>
 __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
-                                                       const PrimeAux *__restrict__ aux, u32 count,
-                                                       u64 *__restrict__ tgt, unsigned short *__restrict__ meta,
+                                                       const PrimeAux *__restrict__ aux, u32 count, bool four,
+                                                       u64 *tgt, unsigned short *__restrict__ meta,
                                                        u64 *__restrict__ stats, JobGeom gm,
                                                        const JobGeom *__restrict__ geoms,
                                                        const u32 *__restrict__ prefix, u32 nr,
@@ -858,28 +935,49 @@ __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restri
     KScratch<GL> &sc = s_sc[threadIdx.x / GL];
     const u32 stride = gridDim.x * (SETUP_TPB / GL);
     u32 i = (blockIdx.x * SETUP_TPB + threadIdx.x) / GL;
-    if constexpr (KIND == ANY_PRIMES) {
-        static_assert(GL == 32, "a warp holds primes of one step kind");
-        const u32 total = prefix[nr];
-        for (; i < total; i += stride) {
-            const u32 rec = rec_of[i];
-            const u64 p = hdr[rec].p;
-            if (p == 0) {
-                if (l == 0) atomicAdd(&stats[ST_SKIPPED], 1ull);
-                continue;
+    if constexpr (GL == 32) {
+        // four consecutive primes per warp when the sequences leave a partial round
+        // that they can share, else one
+        static_assert(KIND != ANY_PRIMES, "a warp holds primes of one step kind");
+        const u32 total = BATCH ? prefix[nr] : count;
+        const u32 per = four ? 4 : 1;
+        for (i *= per; i < total; i += stride * per) {
+            const u32 n = min(per, total - i);
+            // lane q: prime q (mine: of this launch's kind; a skipped one, p = 0, counts
+            // as FP)
+            u32 rec = 0, jb = 0;
+            bool mine = false, rest = false;
+            if (l < n) {
+                rec = BATCH ? rec_of[i + l] : i + l;
+                if (BATCH) jb = hdr[rec].job;
+                mine = !BATCH || (hdr[rec].p < FP_BOUND) == (KIND == FP_PRIMES);
             }
-            const u32 jb = hdr[rec].job;
-            if (p < FP_BOUND) setup_k_one<true, GL>(jobs + jb, rec, l, true, hdr, aux, tgt, meta, stats, geoms[jb], sc);
-            else setup_k_one<false, GL>(jobs + jb, rec, l, true, hdr, aux, tgt, meta, stats, geoms[jb], sc);
+            const u32 todo = __ballot_sync(0xFFFFFFFFu, mine);
+            if (four && todo) {
+                const u32 j0 = __shfl_sync(0xFFFFFFFFu, jb, 0);
+                rest = shares_rest(jobs[j0].kcount) && __all_sync(0xFFFFFFFFu, l >= n || (mine && jb == j0));
+                if (rest) rest_powers<KIND == FP_PRIMES>(jobs + j0, rec, n, hdr, aux, tgt);
+            }
+#pragma unroll 1
+            for (u32 t = todo; t; t &= t - 1) {
+                const u32 q = __ffs((int)t) - 1;
+                const u32 w = __shfl_sync(0xFFFFFFFFu, rec, q), j = __shfl_sync(0xFFFFFFFFu, jb, q);
+                if (hdr[w].p == 0) {
+                    if (l == 0) atomicAdd(&stats[ST_SKIPPED], 1ull);
+                    continue;
+                }
+                setup_k_one<KIND == FP_PRIMES, GL>(jobs + j, w, l, true, hdr, aux, tgt, meta, stats, BATCH ? geoms[j] : gm,
+                                                   rest, sc);
+            }
         }
     } else {
-        // i - l / GL of a warp's sub-warps: the warp stays until its last prime is done
+        // (the warp stays until the last of its sub-warps' primes is done)
         for (; __any_sync(0xFFFFFFFFu, i < count); i += stride) {
             const bool in = i < count;
             const bool live = in && hdr[i].p != 0;
             if (in && !live && l == 0) atomicAdd(&stats[ST_SKIPPED], 1ull);
             if (!__any_sync(0xFFFFFFFFu, live)) continue;
-            setup_k_one<KIND == FP_PRIMES, GL>(jobs, in ? i : 0, l, live, hdr, aux, tgt, meta, stats, gm, sc);
+            setup_k_one<KIND == FP_PRIMES, GL>(jobs, in ? i : 0, l, live, hdr, aux, tgt, meta, stats, gm, false, sc);
         }
     }
 }
@@ -887,7 +985,7 @@ __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restri
 template <int KIND>
 static cudaError_t launch_setup_kind(const JobDev *job, u32 kcount, const u64 *primes, u32 first, u32 count,
                                      PrimeHdr *hdr, PrimeAux *aux, u64 *tabs, u64 *tgt, unsigned short *meta,
-                                     const BsgsLists &lists, u64 *stats, const JobGeom &gm, cudaStream_t st)
+                                     const BsgsLists &lists, u64 *stats, const JobGeom &gm, int sms, cudaStream_t st)
 {
     k_setup_prime<KIND><<<(count + 127) / 128, 128, 0, st>>>(job, primes, first, count, hdr, aux, nullptr, nullptr, 0, 0,
                                                              nullptr);
@@ -895,9 +993,12 @@ static cudaError_t launch_setup_kind(const JobDev *job, u32 kcount, const u64 *p
     if (e != cudaSuccess) return e;
     auto go = [&](auto gl) {
         constexpr u32 GL = decltype(gl)::value;
-        const u32 ppb = SETUP_TPB / GL;                    // primes per block
-        k_setup_k<KIND, GL><<<(count + ppb - 1) / ppb, SETUP_TPB, 0, st>>>(job, hdr, aux, count, tgt, meta, stats, gm,
-                                                                          nullptr, nullptr, 0, nullptr);
+        // four primes share a partial round of lanes when there are enough of them to
+        // fill the chip all the same (4 CTAs of 8 warps per SM)
+        const bool four = GL == 32 && shares_rest(kcount) && count >= 4u * 4 * 8 * (u32)sms;
+        const u32 ppb = SETUP_TPB / GL * (four ? 4 : 1);   // primes per block
+        k_setup_k<KIND, GL><<<(count + ppb - 1) / ppb, SETUP_TPB, 0, st>>>(job, hdr, aux, count, four, tgt, meta, stats,
+                                                                          gm, nullptr, nullptr, 0, nullptr);
     };
     if (kcount <= 4) go(std::integral_constant<u32, 4>{});
     else if (kcount <= 8) go(std::integral_constant<u32, 8>{});
@@ -912,14 +1013,16 @@ static cudaError_t launch_setup_kind(const JobDev *job, u32 kcount, const u64 *p
 
 cudaError_t launch_setup(const JobDev *job, u32 kcount, const u64 *primes, u32 first, u32 count, u64 pmax, PrimeHdr *hdr,
                          void *aux, u64 *tabs, u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats,
-                         int geom, cudaStream_t st)
+                         int geom, int sms, cudaStream_t st)
 {
     if (count == 0) return cudaSuccess;
     const JobGeom gm = job_geom(geom);
     PrimeAux *x = (PrimeAux *)aux;
     return pmax <= FP_BOUND
-               ? launch_setup_kind<FP_PRIMES>(job, kcount, primes, first, count, hdr, x, tabs, tgt, meta, lists, stats, gm, st)
-               : launch_setup_kind<INT_PRIMES>(job, kcount, primes, first, count, hdr, x, tabs, tgt, meta, lists, stats, gm, st);
+               ? launch_setup_kind<FP_PRIMES>(job, kcount, primes, first, count, hdr, x, tabs, tgt, meta, lists, stats, gm, sms,
+                                            st)
+               : launch_setup_kind<INT_PRIMES>(job, kcount, primes, first, count, hdr, x, tabs, tgt, meta, lists, stats, gm, sms,
+                                            st);
 }
 
 cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const BatchRange *ranges, const u64 *primes,
@@ -933,8 +1036,10 @@ cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const B
                                                        rcap, rec_of);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_setup_k<ANY_PRIMES, 32><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tgt, meta, stats, gm,
-                                                             geoms, prefix_p, nranges, rec_of);
+    k_setup_k<INT_PRIMES, 32, true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, true, tgt, meta,
+                                                                   stats, gm, geoms, prefix_p, nranges, rec_of);
+    k_setup_k<FP_PRIMES, 32, true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, true, tgt, meta,
+                                                                  stats, gm, geoms, prefix_p, nranges, rec_of);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_setup_tabs<ANY_PRIMES><<<sms * 8, 128, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, stats, lists.list,
