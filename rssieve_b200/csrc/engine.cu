@@ -34,10 +34,17 @@ struct rs_ctx {
     u32 cand_cap = 0;
     u64 *d_primes = nullptr;
     u32 prime_cap = 0;
-    u32 *d_ctrs = nullptr;      // [0] sieve survivors, [1] primes, [3] factor count, [4] mid list
-    u32 *d_err = nullptr;
-    u64 *d_stats = nullptr;
-    u32 *h_pin = nullptr;       // pinned: ctrs[4], err
+    // one block: u32 [0] sieve survivors, [1] primes, [2] mid list, [3] error flags
+    // (cleared per segment), [4] factor count; from byte 32 the statistics
+    u32 *d_ctrs = nullptr;
+    u32 *d_err = nullptr;       // d_ctrs + 3
+    u64 *d_stats = nullptr;     // d_ctrs + 8
+    u32 *h_pin = nullptr;       // pinned copy of the block
+    // what the device holds, as the last call that changed it left it there (so that
+    // the next one need not wait to read it): statistics, and the factor count
+    u64 h_stats[ST_COUNT] = {};
+    u32 h_factors = 0;
+    bool h_known = false;
     // per-chunk prime records
     u32 chunk_cap = 0;
     PrimeHdr *d_hdr = nullptr;
@@ -73,6 +80,9 @@ struct rs_ctx {
     double last_bsgs_ms = 0, last_total_ms = 0;
     u32 last_bsgs_launches = 0, last_kernel_launches = 0;
 };
+
+constexpr int CTR_ERR = 3, CTR_FACTORS = 4, CTR_STATS = 8;      // in d_ctrs and h_pin
+constexpr size_t BLOCK_BYTES = CTR_STATS * 4 + ST_COUNT * 8;
 
 #define CU(call)                                                                  \
     do {                                                                          \
@@ -122,8 +132,6 @@ extern "C" void rs_ctx_destroy(rs_ctx *c)
     cudaFree(c->d_mid);
     cudaFree(c->d_primes);
     cudaFree(c->d_ctrs);
-    cudaFree(c->d_err);
-    cudaFree(c->d_stats);
     cudaFree(c->d_hdr);
     cudaFree(c->d_aux);
     cudaFree(c->d_tabs);
@@ -170,8 +178,7 @@ extern "C" int rs_ctx_create(int device, rs_ctx **out)
         cudaMalloc(&c->d_cands, (size_t)c->cand_cap * 8) != cudaSuccess ||
         cudaMalloc(&c->d_mid, (size_t)c->cand_cap * 8) != cudaSuccess ||
         cudaMalloc(&c->d_primes, (size_t)c->prime_cap * 8) != cudaSuccess ||
-        cudaMalloc(&c->d_ctrs, 16 * 4) != cudaSuccess || cudaMalloc(&c->d_err, 4) != cudaSuccess ||
-        cudaMalloc(&c->d_stats, ST_COUNT * 8) != cudaSuccess ||
+        cudaMalloc(&c->d_ctrs, BLOCK_BYTES) != cudaSuccess ||
         cudaMalloc(&c->d_hdr, (size_t)c->chunk_cap * sizeof(PrimeHdr)) != cudaSuccess ||
         cudaMalloc(&c->d_aux, (size_t)c->chunk_cap * setup_aux_bytes()) != cudaSuccess ||
         cudaMalloc(&c->d_tabs, (size_t)c->chunk_cap * TABS * 8) != cudaSuccess ||
@@ -180,14 +187,15 @@ extern "C" int rs_ctx_create(int device, rs_ctx **out)
         cudaMalloc(&c->lists.list, (size_t)NCLASS * c->chunk_cap * 4) != cudaSuccess ||
         cudaMalloc(&c->lists.ctl, 2 * NCLASS * 4) != cudaSuccess ||
         cudaMalloc(&c->d_job, sizeof(JobDev)) != cudaSuccess ||
-        cudaMallocHost(&c->h_pin, 64) != cudaSuccess) {
+        cudaMallocHost(&c->h_pin, BLOCK_BYTES) != cudaSuccess) {
         rs_set_error("device allocation failed");
         return fail(RS_ENOMEM);
     }
     if (cudaMemcpy(c->d_sp, sp.data(), sp.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(c->d_ctrs, 0, 64) != cudaSuccess || cudaMemset(c->d_err, 0, 4) != cudaSuccess ||
-        cudaMemset(c->d_stats, 0, ST_COUNT * 8) != cudaSuccess)
+        cudaMemset(c->d_ctrs, 0, BLOCK_BYTES) != cudaSuccess)
         return fail(RS_ECUDA);
+    c->d_err = c->d_ctrs + CTR_ERR;
+    c->d_stats = reinterpret_cast<u64 *>(c->d_ctrs + CTR_STATS);
     if (bsgs_prepare() != cudaSuccess) {
         rs_set_error("BSGS kernel needs %zu B of shared memory", bsgs_smem_bytes());
         return fail(RS_ECUDA);
@@ -354,11 +362,12 @@ extern "C" int rs_job_load(rs_ctx *c, const rs_seqs *s)
     c->h_job = J;
     CU(cudaMemcpyAsync(c->d_bitmap, s->bitmap, c->bitmap_words * 4, cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemcpyAsync(c->d_job, &c->h_job, sizeof(JobDev), cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemsetAsync(c->d_ctrs, 0, 64, c->stream));
-    CU(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
-    CU(cudaMemsetAsync(c->d_stats, 0, ST_COUNT * 8, c->stream));
+    CU(cudaMemsetAsync(c->d_ctrs, 0, BLOCK_BYTES, c->stream));
     CU(cudaStreamSynchronize(c->stream));
     c->primes_total = 0;
+    memset(c->h_stats, 0, sizeof c->h_stats);
+    c->h_factors = 0;
+    c->h_known = true;
     c->job_loaded = true;
     tune_start(c);
     return RS_OK;
@@ -398,16 +407,13 @@ static int gen_segment(rs_ctx *c, u64 lo, u64 hi, u32 *np, bool *overflow)
     u64 base = lo | 1ull;
     if (base >= hi) return RS_OK;
     u64 nodd = (hi - base + 1) / 2;
-    CU(cudaMemsetAsync(c->d_ctrs, 0, 2 * 4, c->stream));
-    CU(cudaMemsetAsync(c->d_ctrs + 4, 0, 4, c->stream));
-    CU(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
+    CU(cudaMemsetAsync(c->d_ctrs, 0, 4 * 4, c->stream));
     CU(launch_sieve(base, nodd, c->d_sp, c->nsp, c->d_cands, c->cand_cap, c->d_ctrs, c->d_err, c->sms, c->stream));
     CU(launch_mr2(c->d_cands, c->d_ctrs, c->cand_cap, c->d_primes, c->prime_cap, c->d_ctrs + 1, c->d_mid,
-                  c->d_ctrs + 4, c->d_err, c->sms, c->stream));
-    CU(cudaMemcpyAsync(c->h_pin, c->d_ctrs, 2 * 4, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaMemcpyAsync(c->h_pin + 4, c->d_err, 4, cudaMemcpyDeviceToHost, c->stream));
+                  c->d_ctrs + 2, c->d_err, c->sms, c->stream));
+    CU(cudaMemcpyAsync(c->h_pin, c->d_ctrs, 4 * 4, cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
-    u32 err = c->h_pin[4];
+    u32 err = c->h_pin[CTR_ERR];
     if (err & (ERR_CAND_OVERFLOW | ERR_PRIME_OVERFLOW)) {
         *overflow = true;
         return RS_OK;
@@ -449,10 +455,16 @@ extern "C" int rs_primes_generate(rs_ctx *c, uint64_t p0, uint64_t p1, uint64_t 
     return (dst && total > cap) ? RS_EARG : RS_OK;
 }
 
-static int read_stats(rs_ctx *c, u64 *out)
+// The device's statistics and factor count into the host's copies, together with
+// the error flags (h_pin[CTR_ERR]): one wait.
+static int read_state(rs_ctx *c)
 {
-    CU(cudaMemcpyAsync(out, c->d_stats, ST_COUNT * 8, cudaMemcpyDeviceToHost, c->stream));
+    c->h_known = false;
+    CU(cudaMemcpyAsync(c->h_pin, c->d_ctrs, BLOCK_BYTES, cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
+    memcpy(c->h_stats, c->h_pin + CTR_STATS, ST_COUNT * 8);
+    c->h_factors = c->h_pin[CTR_FACTORS];
+    c->h_known = true;
     return RS_OK;
 }
 
@@ -468,9 +480,10 @@ extern "C" int rs_run_range(rs_ctx *c, uint64_t p0, uint64_t p1, rs_counters *de
         return RS_OK;
     }
     CU(cudaSetDevice(c->device));
-    u64 before[ST_COUNT];
-    int rc = read_stats(c, before);
+    int rc = c->h_known ? RS_OK : read_state(c);
     if (rc) return rc;
+    u64 before[ST_COUNT];
+    memcpy(before, c->h_stats, sizeof before);
     c->last_bsgs_ms = 0;
     c->last_total_ms = 0;
     c->last_bsgs_launches = 0;
@@ -482,7 +495,7 @@ extern "C" int rs_run_range(rs_ctx *c, uint64_t p0, uint64_t p1, rs_counters *de
     a.words = c->h_job.words;
     a.bitmap = c->d_bitmap;
     a.factors = c->d_factors;
-    a.factor_ctr = c->d_ctrs + 3;
+    a.factor_ctr = c->d_ctrs + CTR_FACTORS;
     a.factor_cap = c->factor_cap;
     a.stats = c->d_stats;
     a.err = c->d_err;
@@ -515,7 +528,7 @@ extern "C" int rs_run_range(rs_ctx *c, uint64_t p0, uint64_t p1, rs_counters *de
         u32 nchunks = (np + c->chunk_cap - 1) / c->chunk_cap;
         rc = ensure_events(c, 2 + 2 * (size_t)nchunks);
         if (rc) return rc;
-        CU(cudaMemsetAsync(c->d_err, 0, 4, c->stream));
+        c->h_known = false;                          // until read_state below
         c->chunk_geom.assign(nchunks, c->geom);
         for (u32 ci = 0; ci < nchunks; ++ci) {
             u32 first = ci * c->chunk_cap;
@@ -533,10 +546,10 @@ extern "C" int rs_run_range(rs_ctx *c, uint64_t p0, uint64_t p1, rs_counters *de
             c->last_bsgs_launches += 1;
         }
         CU(cudaEventRecord(c->ev[1], c->stream));
-        CU(cudaMemcpyAsync(c->h_pin + 4, c->d_err, 4, cudaMemcpyDeviceToHost, c->stream));
-        CU(cudaStreamSynchronize(c->stream));
-        if (c->h_pin[4]) {
-            rs_set_error("BSGS raised error flags 0x%x at p in [%llu,%llu)", c->h_pin[4], (unsigned long long)p,
+        rc = read_state(c);
+        if (rc) return rc;
+        if (c->h_pin[CTR_ERR]) {
+            rs_set_error("BSGS raised error flags 0x%x at p in [%llu,%llu)", c->h_pin[CTR_ERR], (unsigned long long)p,
                          (unsigned long long)hi);
             return RS_EDEVICE;
         }
@@ -552,13 +565,10 @@ extern "C" int rs_run_range(rs_ctx *c, uint64_t p0, uint64_t p1, rs_counters *de
         p = hi;
         width = segment_width(c, p);
     }
-    u64 after[ST_COUNT];
-    rc = read_stats(c, after);
-    if (rc) return rc;
     c->primes_total += seg_primes;
     if (delta) {
         u64 *d = reinterpret_cast<u64 *>(delta);
-        for (int i = 0; i < ST_COUNT; ++i) d[i] = after[i] - before[i];
+        for (int i = 0; i < ST_COUNT; ++i) d[i] = c->h_stats[i] - before[i];
         delta->primes = seg_primes;     // counted on the host: the device only sees segment totals
     }
     return RS_OK;
@@ -568,9 +578,11 @@ extern "C" int rs_factors_fetch(rs_ctx *c, rs_factor *buf, size_t cap, size_t *n
 {
     if (!c || !n || !c->job_loaded) return RS_EARG;
     CU(cudaSetDevice(c->device));
-    CU(cudaMemcpyAsync(c->h_pin + 8, c->d_ctrs + 3, 4, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
-    u32 cnt = c->h_pin[8];
+    if (!c->h_known) {
+        const int rc = read_state(c);
+        if (rc) return rc;
+    }
+    const u32 cnt = c->h_factors;
     *n = cnt;
     if (cnt > c->factor_cap) {
         rs_set_error("factor buffer overflowed (%u > %u)", cnt, c->factor_cap);
@@ -578,9 +590,11 @@ extern "C" int rs_factors_fetch(rs_ctx *c, rs_factor *buf, size_t cap, size_t *n
     }
     if (cnt > cap || (cnt && !buf)) return RS_EARG;
     static_assert(sizeof(rs_factor) == sizeof(FactorRec), "factor layout");
-    if (cnt) CU(cudaMemcpyAsync(buf, c->d_factors, (size_t)cnt * sizeof(FactorRec), cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaMemsetAsync(c->d_ctrs + 3, 0, 4, c->stream));
+    if (!cnt) return RS_OK;
+    CU(cudaMemcpyAsync(buf, c->d_factors, (size_t)cnt * sizeof(FactorRec), cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaMemsetAsync(c->d_ctrs + CTR_FACTORS, 0, 4, c->stream));
     CU(cudaStreamSynchronize(c->stream));
+    c->h_factors = 0;
     return RS_OK;
 }
 
@@ -597,9 +611,11 @@ extern "C" int rs_counters_get(rs_ctx *c, rs_counters *out)
 {
     if (!c || !out) return RS_EARG;
     CU(cudaSetDevice(c->device));
-    int rc = read_stats(c, reinterpret_cast<u64 *>(out));
+    const int rc = read_state(c);
+    if (rc) return rc;
+    memcpy(out, c->h_stats, sizeof c->h_stats);
     out->primes = c->primes_total;
-    return rc;
+    return RS_OK;
 }
 
 extern "C" int rs_last_timing(rs_ctx *c, double *bsgs_ms, double *total_ms, uint32_t *bl, uint32_t *kl)
