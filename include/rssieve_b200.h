@@ -154,8 +154,9 @@ int rs_device_count(void);
 /* Baby steps per prime Q for the BSGS search of this context's jobs: 1024,
  * 2048, 4096, 8192 or 16384, or 0 (the default) to choose per job.  Replaces
  * the reference's Q/M rule, which fixes Q from the n-range when the kernels
- * are built (cl_sieve.cpp:893-938).  In automatic mode a model of the per-prime
- * cost keeps the candidates within 2x of its best, the first full chunks of
+ * are built (cl_sieve.cpp:893-938).  Q is the most baby steps a prime gets; each
+ * takes 512 to Q of them by its own work.  In automatic mode a model of the per-prime
+ * cost keeps its best Q and the runner-up, the first full chunks of
  * the job run with each in turn (their results count, as every Q is exact),
  * and the fastest measured one is kept; later jobs of the same shape (base,
  * sequence count, n-range length) on the context reuse it.  Takes effect at

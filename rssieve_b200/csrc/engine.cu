@@ -234,9 +234,11 @@ static u64 job_shape(const rs_ctx *c)
     return job_shape_key(c->h_job.base, c->h_job.kcount, c->h_job.L);
 }
 
-// Starts the per-job tuner: the candidates are the largest geometry of each CTA
-// size (a smaller maximum Q only takes classes away) whose model cost is within
-// 2x of the model's best; the first chunks cycle through them.
+// Starts the per-job tuner: the candidates are the model's best geometry and its
+// runner-up (of equal costs the larger maximum Q; only if its cost is within 15%);
+// the first chunks cycle through them.  1024-thread CTAs are tried only where the
+// model wants 16384 baby steps: on a short n-range they ran the search 1.9 times
+// slower, which a job of a few chunks never won back.
 static void tune_start(rs_ctx *c)
 {
     c->tune_ncand = 0;
@@ -247,17 +249,13 @@ static void tune_start(rs_ctx *c)
         c->tuning = false;
         return;
     }
-    double best = 1e300;
-    int gb = 0;
-    for (int g = 0; g < NGEOM; ++g) {
-        double v = geom_model_cost(g, c->h_job.kcount, c->h_job.L);
-        if (v < best) { best = v; gb = g; }
-    }
-    for (int g = 0; g < NGEOM; ++g)
-        if ((g == 0 || BSGS_GEOMS[g].tpb != BSGS_GEOMS[g - 1].tpb) &&
-            geom_model_cost(g, c->h_job.kcount, c->h_job.L) <= 2.0 * best)
-            c->tune_cand[c->tune_ncand++] = g;
-    c->geom = gb;
+    auto cost = [&](int g) { return geom_model_cost(g, c->h_job.kcount, c->h_job.L); };
+    int by_cost[NGEOM];
+    for (int g = 0; g < NGEOM; ++g) by_cost[g] = g;
+    std::stable_sort(by_cost, by_cost + NGEOM, [&](int x, int y) { return cost(x) < cost(y); });
+    c->tune_cand[c->tune_ncand++] = by_cost[0];
+    if (cost(by_cost[1]) <= 1.15 * cost(by_cost[0])) c->tune_cand[c->tune_ncand++] = by_cost[1];
+    c->geom = by_cost[0];
     c->tuning = (c->tune_ncand > 1);
     const int known = tuned_geom_get(c->device, job_shape(c));
     if (known >= 0) {
