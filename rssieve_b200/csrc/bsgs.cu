@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
     typedef typename RM::V V;
     // (the integer products' longer code runs slower unrolled further: 8% at p
     // near 2^64)
-    constexpr int BABY_UNROLL = MODE == 2 ? 8 : 2, GIANT_UNROLL = MODE == 2 ? 4 : 2;
+    constexpr int BABY_UNROLL = MODE == 2 ? 8 : 2, GIANT_UNROLL = MODE == 2 ? 2 : 1;
     __shared__ __align__(8) u64 s_bar[TPB / 32][2];               // record copies of each group (by its first warp)
     __shared__ __align__(8) u64 s_dead;                           // never completed (failure test)
     __shared__ u32 s_par[TPB / 32][2];                            // parity of each barrier's next phase
@@ -594,18 +594,32 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
                     const u32 Lc = H->Lc;
                     if ((w & ~31u) + gs < nitems) {
                         V gB = item_start<MODE>(R, min(w + gs, nitems - 1), H, tb, tg);
+                        // two steps of both chains per test of the four probes
+                        u32 t = 0;
 #pragma unroll GIANT_UNROLL
-                        for (u32 t = 0; t < Lc; ++t) {
+                        for (; t + 1 < Lc; t += 2) {
                             const u32 ha = val_hash(RM::bits(gA)), hb = val_hash(RM::bits(gB));
                             const u32 fa = filt[__umulhi(ha, nw)], fb = filt[__umulhi(hb, nw)];
                             const V nA = R.step(gA, f), nB = R.step(gB, f);
-                            const bool hitA = (filter_mask(ha) & ~fa) == 0, hitB = (filter_mask(hb) & ~fb) == 0;
-                            if (__any_sync(0xFFFFFFFFu, hitA | hitB)) {
-                                if (hitA) pass(gA, w, t);
-                                if (hitB) pass(gB, w + gs, t);
+                            const u32 hc = val_hash(RM::bits(nA)), hd = val_hash(RM::bits(nB));
+                            const u32 fc = filt[__umulhi(hc, nw)], fd = filt[__umulhi(hd, nw)];
+                            const V mA = R.step(nA, f), mB = R.step(nB, f);
+                            // the bits each probe misses: none for a pass
+                            const u32 a = filter_mask(ha) & ~fa, b = filter_mask(hb) & ~fb, c2 = filter_mask(hc) & ~fc,
+                                      d = filter_mask(hd) & ~fd;
+                            if (__any_sync(0xFFFFFFFFu, min(min(a, b), min(c2, d)) == 0)) {
+                                if (a == 0) pass(gA, w, t);
+                                if (b == 0) pass(gB, w + gs, t);
+                                if (c2 == 0) pass(nA, w, t + 1);
+                                if (d == 0) pass(nB, w + gs, t + 1);
                             }
-                            gA = nA;
-                            gB = nB;
+                            gA = mA;
+                            gB = mB;
+                        }
+                        if (t < Lc) {
+                            const u32 ha = val_hash(RM::bits(gA)), hb = val_hash(RM::bits(gB));
+                            if ((filter_mask(ha) & ~filt[__umulhi(ha, nw)]) == 0) pass(gA, w, t);
+                            if ((filter_mask(hb) & ~filt[__umulhi(hb, nw)]) == 0) pass(gB, w + gs, t);
                         }
                     } else {
                         for (u32 t = 0; t < Lc; ++t) {

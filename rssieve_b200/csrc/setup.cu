@@ -671,7 +671,9 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
                     while ((r0 = sc.slot[s]) != 0) {
                         if (sc.hv[r0 - 1] == v) {
                             keep = true;
-                            off = (r0 - 1 + 2 * e - j - nmod) % e;
+                            off = r0 - 1 + e - nmod;       // (GL = 32: j = 0)
+                            if constexpr (GL < 32) off = (off + e - j) % e;
+                            else if (off >= e) off -= e;
                             break;
                         }
                         s = (s + 1) & smask;
