@@ -393,7 +393,7 @@ __device__ __forceinline__ u32 choose_class(const JobGeom &gm, u32 nk, u32 Le)
 #pragma unroll
     for (u32 c = 0; c < NCLASS; ++c) {
         const u32 lq = 9 + c;
-        const u32 mg = (Le + (1u << lq) - 1) >> lq;
+        const u32 mg = ((Le - 1) >> lq) + 1;
         const float cost = 1.5f * (float)(1u << lq) + (float)nk * (float)mg;
         if (((gm.classes >> c) & 1u) && cost < best) { best = cost; best_c = c; }
     }
@@ -746,7 +746,7 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
     if (!live || skip) return;
     // baby steps for this prime (the giant-step tables follow in kernel 3), and the
     // targets T = -c * k * b^(nmin + off + e(Q'-1))
-    const u32 cls = choose_class(gm, nk, (job->L + e - 1) / e);
+    const u32 cls = choose_class(gm, nk, (job->L - 1) / e + 1);
     const V wr0 = F::val(X.wr0[cls]);
     for (u32 j = l; j < nk; j += GL) {
         tgt[(size_t)w * KSTRIDE + j] = F::bits(f.mul(F::val(sc.part[j]), wr0));
@@ -812,8 +812,8 @@ __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u
     PrimeHdr &h = hdr[t];
     const F f(h, aux[t]);
     const u32 e = run ? h.e : 1, nk = run ? h.numk : 1, cls = run ? h.cls : 0, gs = 32u << cls, lq = 9 + cls;
-    const u32 Le = (job->L + e - 1) / e;
-    const u32 Mg = (Le + (1u << lq) - 1) >> lq;
+    const u32 Le = (job->L - 1) / e + 1;            // (L - 1 and not L + e - 1: an n-range may be 2^32 - 1 long)
+    const u32 Mg = ((Le - 1) >> lq) + 1;
     u32 G, Lc, nseg, rounds;
     giant_split(gs, nk, Mg, (float)h.p, G, Lc, nseg, rounds);
     const V s = F::val(h.s), S = F::val(aux[t].S[cls]);          // (not a record's when !run: never stored)

@@ -64,3 +64,38 @@ def test_planted_factors_in_every_step_kind(sieve, oracle, p0, kcount, width):
     got = oracle.term_set(sieve.factors())
     # a term may be hit by chance as well: at most width * kcount * primes / p, far below one
     assert want == got
+
+
+def _planted(sieve, oracle, base, kcount, nmin, nmax, p0, p1, seed, q=0):
+    """A job whose only candidates are terms that a prime of [p0, p1) divides, one
+    per sequence: every one of them has to go, and nothing else."""
+    rng = np.random.default_rng(seed)
+    plist = oracle.primes(p0, p1)
+    ks, cs, want = [], [], set()
+    bm = np.zeros((kcount, (nmax - nmin + 32) // 32), dtype=np.uint32)
+    for i in range(kcount):
+        k, c = base % 2, 1 if i % 2 else -1
+        while k % 2 == base % 2:                                # odd terms
+            p, n = int(rng.choice(plist)), (nmin, nmax, int(rng.integers(nmin, nmax + 1)))[i % 3]
+            k = -c * pow(base, -n, p) % p
+        ks.append(k)
+        cs.append(c)
+        bm[i, (n - nmin) >> 5] |= np.uint32(1 << ((n - nmin) & 31))
+        want.add((i, n))
+    sieve.set_baby_steps(q)
+    try:
+        sieve.load(W.seqs_of(W.job_dict(base, ks, cs, nmin, nmax, bm)))
+        cnt = sieve.run(p0, p1)
+        got = oracle.term_set(sieve.factors())
+        left = sieve.bitmap()
+    finally:
+        sieve.set_baby_steps(0)
+    assert cnt["primes"] == len(plist)
+    assert got == want
+    assert not left.any()
+
+
+@pytest.mark.parametrize("nmin", [1, 200, 9_000])      # n-ranges of 2^32 - 1 and a little below: L + e - 1, L + Q' - 1 pass 2^32
+@pytest.mark.parametrize("p0", [(1 << 47) + 1, (1 << 57) + 1])
+def test_n_range_of_32_bits(sieve, oracle, nmin, p0):
+    _planted(sieve, oracle, 2, 3, nmin, (1 << 32) - 1, p0, p0 + 2_000, nmin)
