@@ -99,3 +99,12 @@ def _planted(sieve, oracle, base, kcount, nmin, nmax, p0, p1, seed, q=0):
 @pytest.mark.parametrize("p0", [(1 << 47) + 1, (1 << 57) + 1])
 def test_n_range_of_32_bits(sieve, oracle, nmin, p0):
     _planted(sieve, oracle, 2, 3, nmin, (1 << 32) - 1, p0, p0 + 2_000, nmin)
+
+
+# Sequence counts at every step of the set-up's lanes per prime (4, 8, 16, 32) and of
+# its last, partial round of powers, shared by four primes of a warp once a chunk has
+# about 19000 primes: the window has 25000 or more.
+@pytest.mark.parametrize("kcount", [1, 4, 5, 8, 9, 16, 17, 20, 24, 25, 31, 32, 33, 56, 57, 64, 68, 87, 88, 89, 96, 97, 100])
+@pytest.mark.parametrize("p0", [(1 << 49) + 5, (1 << 59) + 5])
+def test_sequence_counts(sieve, oracle, kcount, p0):
+    _planted(sieve, oracle, 3 if kcount % 2 else 10, kcount, 5_001, 25_000, p0, p0 + 1_100_000, kcount)
