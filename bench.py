@@ -35,11 +35,11 @@ WORKLOAD = ("config2 plain form: 100 seqs k*2^n+-1 (50 +1, 50 -1), k odd U[3,2^3
             "kept w.p. 0.03, p windows from 2^50")
 P_START = 1 << 50
 # DRAM bytes (read + write) per prime of the BSGS kernel, from one ncu capture
-# of a 2^20-wide window at 2^50 at the tuned Q = 8192 (69.36 MB for 30 203
-# primes, FP64 steps and start values): the 2272-byte prime record plus
+# of a 2^20-wide window at 2^50 at the tuned Q = 8192 (68.47 MB for 30 203
+# primes): the 2272-byte prime record, of which nearly all is read, plus
 # claims.  Traffic grows in proportion to primes, so the per-launch figure is
 # this times the primes one launch processes.
-BSGS_DRAM_BYTES_PER_PRIME = 2296.4
+BSGS_DRAM_BYTES_PER_PRIME = 2267.1
 
 
 def reference_params(nmin, nmax):
@@ -534,7 +534,7 @@ def main():
     bsgs_ms_avg = bsgs_ms / max(bsgs_launches, 1)
     # roofline of the BSGS kernel: its executed steps per launch (baby steps and
     # giant steps, one modular product -- or doublings for b^e <= 4 -- and one
-    # table insert or probe each) / average launch time
+    # filter insert or probe each) / average launch time
     achieved = ((tot["giant"] + tot["baby"]) / max(bsgs_launches, 1)) / (bsgs_ms_avg / 1e3) / 1e9
     peak_mult = wide / 11.0                       # products the 32x32->64 multiplier allows
     # below 2^51 the steps' products run on the FP64 pipe: the roofline is then
@@ -616,7 +616,7 @@ def main():
                          "traffic": BSGS_DRAM_BYTES_PER_PRIME * tot["primes"] / max(bsgs_launches, 1),
                          "traffic_unit": "bytes per BSGS launch (ncu per-prime DRAM bytes x primes per launch)",
                          "work_unit": "baby + giant steps of the BSGS kernel (each one modular product or "
-                                      "doublings, plus one table insert or probe)",
+                                      "doublings, plus one filter insert or probe)",
                          "peak_source": ("measured live: rs_fpmul_peak, independent chains of the steps' FP64 product"
                                          if fp_steps else
                                          "measured live: rs_mulmod_peak, independent Montgomery-product chains"),

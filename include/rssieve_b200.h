@@ -74,7 +74,7 @@ typedef struct rs_counters {
     uint64_t baby;              /* baby steps */
     uint64_t giant;             /* giant steps = Montgomery products + probes */
     uint64_t small_order;       /* primes where ord(b^e) < Q */
-    uint64_t candidates;        /* fingerprint matches verified */
+    uint64_t candidates;        /* filter passes checked exactly */
     uint64_t hits;              /* verified solutions with n in [nmin,nmax] (factors + dups) */
     uint64_t factors;           /* terms eliminated */
     uint64_t dups;

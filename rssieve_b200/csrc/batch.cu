@@ -23,22 +23,21 @@
 // any range is unfinished.  The first round runs eagerly (it also sizes the
 // persistent grids); it is then captured as a CUDA graph and replayed.
 //
-// A job's p-range is split at 2^63 into two ranges (Shoup giant steps below,
-// Montgomery above) that share its bitmap and factor list.  Each job's BSGS
+// A job's p-range is split at 2^51 and 2^63 into ranges of one step kind each (FP64
+// below, Shoup, Montgomery above) that share its bitmap and factor list.  Each job's BSGS
 // geometry is the one a single-job run on the device measured for the job's
 // shape (base, sequence count, n-range), else the per-prime cost model's
 // (geom_model_best), unless the caller fixes Q.
 //
 // Capacity is fixed when the batch is created: job slots and range slots (each
-// range slot owns one round's buffers, about 136 MB).  Jobs can be added
+// range slot owns one round's buffers, about 170 MB).  Jobs can be added
 // between rounds -- their tables are written to device memory that the
 // captured round reads -- and a finished job's slots are released for the
 // next one, so the batch also serves a stream of arriving work units.  The
 // six BSGS groups take whatever the set-up put on their lists, so the captured
-// round never changes.  A job's
-// bitmap and factor list come from the batch's own stream-ordered memory pool,
-// which keeps freed blocks mapped and can be grown ahead of time
-// (rs_batch_reserve): admitting or releasing a job neither
+// round never changes.  A job's bitmap and factor list come from the batch's own
+// stream-ordered memory pool, which keeps freed blocks mapped and can be grown
+// ahead of time (rs_batch_reserve): admitting or releasing a job neither
 // synchronises the device nor maps new pages.
 #include <algorithm>
 #include <cstring>

@@ -26,22 +26,27 @@
 // 4-byte load).  It never misses a value; about one probe in 2000 passes for a
 // value that is not there.  Passing probes go on a queue and are checked exactly
 // once the giant steps are done, 16 lanes each: with anchors x_t = s^(16t), t =
-// 0..GS, in an index that then takes the filter's place, gamma = s^j for some j = 16t -
-// l, 0 <= l < 16, exactly when gamma * s^l is an anchor, so lane l forms gamma *
-// s^l and looks it up.  The search is exact for every 64-bit value (the reference's split lo32/hi32
-// table cannot find values whose low 32 bits are zero, giant.cl:46,63).
+// 0..GS, in an index that then takes the filter's place, gamma = s^j for some j =
+// 16t - l, 0 <= l < 16, exactly when gamma * s^l is an anchor, so lane l forms gamma
+// * s^l and looks it up.  The search is exact for every 64-bit value (the reference's
+// split lo32/hi32 table cannot find values whose low 32 bits are zero,
+// giant.cl:46,63).
 //
 // What bounds it: issue.  A random 4-byte shared-memory access of a warp, load or
 // atomic, takes 3.55 cycles of the SM's shared-memory pipe, a 16-byte one 10.2,
 // and the ALU and FP64 pipes take two cycles per warp instruction (measured).
 // A step is about 8 FP64, 8 ALU and 3 IMAD instructions and one such access,
 // 14 to 16 cycles of an SM quarter on each of these resources, and its 22 issue
-// slots come first.  100 sequences, n-range 6*10^6, p near 2^50: 18.3 ns per
-// prime (28.1 with an exact table of 16-byte buckets of fingerprints, whose
-// probes and three-store inserts took 5600 shared-memory cycles per prime
-// against 2200 now, and with one group size for all primes of a job); p near
-// 2^58, 61 sequences: 20.5 (26.8); 68 sequences over an n-range of 10^5: 2.4
-// (4.0).  Three bits per value and three words per value: with two bits a pass
+// slots come first: mixed streams of instructions that each hold their pipe for
+// two cycles issue one in 1.5 cycles at best (measured), and the kernel issues in
+// 65% of all cycles.  100 sequences, n-range 6*10^6, p near 2^50: 13.9 ns per
+// prime for 9200 steps (28.1 for 12100 with an exact table of 16-byte buckets of
+// fingerprints, whose probes and three-store inserts took 5600 shared-memory
+// cycles per prime against 2200 now, and with one group size for all primes of a
+// job); p near 2^58, 61 sequences: 16.1 (26.8); 68 sequences over an n-range of
+// 10^5: 2.2 (4.0).  One test for two steps of both chains (the least of the four
+// probes' missing bits) instead of one each took 14.1 to 13.9 and 17.0 to 16.1 of
+// these.  Three bits per value and three words per value: with two bits a pass
 // comes four times as often and costs more than the third bit's two
 // instructions; the filter fills what two CTAs of 512 threads have of shared
 // memory.  A group of Q'/16 threads per prime instead of the whole CTA keeps 16

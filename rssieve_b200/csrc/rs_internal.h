@@ -87,7 +87,6 @@ constexpr u64 MR_BOUND = 4295098369ULL;     // 65537^2: below it the sieve by al
 // error bits (JobDev-independent, one word per context)
 constexpr u32 ERR_PRIME_OVERFLOW = 1u;      // segment produced more primes than the buffer holds
 constexpr u32 ERR_CAND_OVERFLOW = 2u;
-constexpr u32 ERR_HASH_OVERFLOW = 4u;       // a bucket chain exceeded BSGS_MAXPROBE
 constexpr u32 ERR_FACTOR_OVERFLOW = 8u;     // factor buffer full (cannot happen: sized to the bitmap)
 constexpr u32 ERR_TMA_TIMEOUT = 16u;        // a bulk copy did not complete within the wait bound
 constexpr u32 ERR_SIEVE_TABLE = 32u;        // the sieving-prime table is missing (does not start with 3)
@@ -100,9 +99,9 @@ enum Stat {
     ST_PARITY,            // primes searched over one class of n mod e per sequence (e >= 2; e = 2: parity)
     ST_TARGETS,           // sum over primes of surviving k
     ST_BABY,              // baby steps executed
-    ST_GIANT,             // giant steps executed (one Montgomery product and one lookup each)
+    ST_GIANT,             // giant steps executed (one modular product and one probe each)
     ST_SMALLORDER,        // primes with ord(b^e) < Q
-    ST_CANDIDATES,        // fingerprint matches verified
+    ST_CANDIDATES,        // filter passes checked exactly
     ST_HITS,              // verified solutions p | k*b^n+c with n in range
     ST_FACTORS,           // bitmap claims won
     ST_DUPS,              // solutions whose bitmap bit was already clear

@@ -21,10 +21,11 @@
 // generated by chi(b), of order eo (the reference's filters are the cases
 // d | D of this), and (2) n mod e is fixed, for every divisor e of eo, by the
 // discrete logarithm of h = chi(b)^(eo/e) -- a table of e values.  e is the
-// largest divisor of eo up to 256 (64 for small jobs, JobDev::split).  Both take one power per sequence, z = k^E with
-// E = (p-1)/D * eo/e: the logarithm of (-c)^E / z to the base h exists exactly
-// when (chi(-c)/chi(k))^eo = 1, the groups being cyclic.  Every n the reference finds satisfies both,
-// so the eliminated terms are the same, while each sequence's giant steps
+// largest divisor of eo up to 256 (64 for small jobs, JobDev::split).  Both take
+// one power per sequence, z = k^E with E = (p-1)/D * eo/e: the logarithm of
+// (-c)^E / z to the base h exists exactly when (chi(-c)/chi(k))^eo = 1, the groups
+// being cyclic.  Every n the reference finds satisfies both, so the eliminated
+// terms are the same, while each sequence's giant steps
 // shrink from L/Q to L/(e*Q) (e = 2 is the reference's parity case; at the
 // 2^50 p-range of the 100-sequence job e averages well above 2).
 // Primes dividing b or any k, and primes where no k survives, are skipped for
@@ -518,8 +519,8 @@ __device__ __forceinline__ u32 cls_hash(u64 v, u32 mask)
 
 // The powers of four primes' last sequences together.  With K = 32R + m sequences,
 // 0 < m <= REST_MAX, a warp's last round of lanes would leave 32 - m of them idle
-// (and for odd R it runs beside another, as the second chain of its lanes, where it
-// costs little: shares_rest);
+// (for odd R it runs beside another round, as the second chain of its lanes, where
+// it costs little: shares_rest says no);
 // here m8 = 8*ceil(m/8) lanes take a prime's m sequences, so that m8/8 rounds serve
 // four primes (each lane its own exponent, 1.5 products per bit against 1.375).
 // z = k^E goes to the target row of its record until setup_k_one takes it up.
