@@ -41,13 +41,11 @@ class Unit:
 
 # Relative cost of one prime by the kind of step its p takes in the library:
 # FP64 products below 2^51, Shoup products below 2^63, Montgomery products
-# above.  Measured on a B200 with config-2-style units served one at a time:
-# 4.0e11 model cost units/s below 2^51 against 2.8-3.0e11 for units between
-# 2^52 and 2^61, i.e. a prime there costs 1.38 times as much.  Above 2^63 the
-# steps and the set-up's chains are full Montgomery products; the factor there
-# is the config-4 job's step rate against config 2's (253 against 427 G
-# steps/s in the BSGS kernel), an estimate for whole units.
-STEP_COST = ((1 << 51, 1.0), (1 << 63, 1.38), (1 << 64, 1.7))
+# above.  Measured on a B200, whole windows at 2^50, 2^58 and 1.5*2^63: 100
+# sequences over an n-range of 6*10^6 19.6, 39.7 and 45.0 ns per prime, 20
+# sequences over 2*10^6 7.2, 13.0 and 14.4, i.e. a prime costs 1.8 to 2.0 and
+# 2.0 to 2.3 times as much.
+STEP_COST = ((1 << 51, 1.0), (1 << 63, 1.9), (1 << 64, 2.15))
 
 
 def step_factor(p0):
@@ -59,10 +57,12 @@ def step_factor(p0):
 
 
 def cost_per_prime(q, kcount, L):
-    """Model cost of one prime in baby-step units for Q baby steps (the library's
-    geometry model: Q baby steps plus the giant steps of the surviving targets,
-    each over one class of n modulo the prime's split modulus, about 0.15 L/Q
-    steps and at least one)."""
+    """Model cost of one prime in baby-step units for Q baby steps, to weigh units
+    against one another: Q baby steps plus the giant steps of the surviving
+    targets, each over one class of n modulo the prime's split modulus, about
+    0.15 L/Q steps and at least one.  (100 sequences over an n-range of 6*10^6
+    against 20 over 2*10^6 and 68 over 10^5: 3.0 and 3.5 by the model, 2.7 and 2.9
+    measured.)"""
     m = max(1.0, 0.15 * L / q + 0.5)
     return 1.15 * q + 1.2 * 0.6 * kcount * m
 
