@@ -269,7 +269,10 @@ __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, 
     const u32 b = job->base;
     const u64 bp = (b < p) ? b : b % p;
     if (bp == 0) {                                        // p | b: no term is divisible by p
-        hdr[t].p = 0;
+        PrimeHdr H{};                                     // (kernels 2 and 3 read its job and e)
+        H.job = jb;
+        H.e = 1;
+        hdr[t] = H;
         return;
     }
     const F f(p);
@@ -576,9 +579,9 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
     const u32 gmask = GL == 32 ? 0xFFFFFFFFu : ((1u << (GL & 31)) - 1u) << sub;
     const PrimeAux &X = aux[w];
     const F f(hdr[w], X);
-    const u64 p = hdr[w].p;
-    const u32 K = job->kcount, e = hdr[w].e;
-    const u64 E = X.E;
+    // (without a live record only the loops' ends matter: a skipped one has no X)
+    const u64 p = live ? hdr[w].p : ~0ull, E = live ? X.E : 1;
+    const u32 K = job->kcount, e = live ? hdr[w].e : 1;
     // class table: lane l forms h^(-l) by a multiplicative scan over the GL lanes,
     // then every GL-th value from there by products with h^(-GL)
     constexpr u32 TAB = KScratch<GL>::TAB, CLS_SLOTS = KScratch<GL>::CLS_SLOTS;
@@ -813,7 +816,8 @@ __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u
     PrimeHdr &h = hdr[t];
     const F f(h, aux[t]);
     const u32 e = run ? h.e : 1, nk = run ? h.numk : 1, cls = run ? h.cls : 0, gs = 32u << cls, lq = 9 + cls;
-    const u32 Le = (job->L - 1) / e + 1;            // (L - 1 and not L + e - 1: an n-range may be 2^32 - 1 long)
+    // (L - 1 and not L + e - 1: an n-range may be 2^32 - 1 long; without run job is not the record's)
+    const u32 Le = run ? (job->L - 1) / e + 1 : 1;
     const u32 Mg = ((Le - 1) >> lq) + 1;
     u32 G, Lc, nseg, rounds;
     giant_split(gs, nk, Mg, (float)h.p, G, Lc, nseg, rounds);
@@ -892,7 +896,7 @@ __global__ void __launch_bounds__(128, 8) k_setup_tabs(const JobDev *__restrict_
         const bool live = i < total && hdr[rec].p != 0;
         u32 key = 0xFFFFFFFFu;                             // list of the record: group * NCLASS + class
         const u64 p = hdr[rec].p;
-        const u32 jb = BATCH ? hdr[rec].job : 0;
+        const u32 jb = BATCH && live ? hdr[rec].job : 0;   // (past the end rec 0 may never have been written)
         const bool fp = KIND == FP_PRIMES || (BATCH && p < FP_BOUND);
         if (KIND != INT_PRIMES && __any_sync(0xFFFFFFFFu, live && fp))
             setup_tabs_one<true>(jobs + jb, rec, hdr, aux, tabs, tile, live && fp, nt, nf, ns);

@@ -1,0 +1,64 @@
+"""The batch's set-up: primes without a search (they divide the base, or leave no
+sequence) beside others, range slots without a prime, and its counters.
+
+Every result is compared with the brute-force oracle or with the single-job path:
+whole numbers, equal or not.
+"""
+from contextlib import closing
+
+import numpy as np
+import pytest
+
+from rssieve_b200 import workloads as W
+from tests.conftest import oracle_job
+
+pytestmark = pytest.mark.gpu
+
+
+def _terms(f):
+    return set(zip(f["seq"].tolist(), f["n"].tolist()))
+
+
+def _small_job(base, kcount, seed=0):
+    return W.small_job(300 + base + kcount + seed, kcount=kcount, base=base, nmin=1000, nmax=9000, keep=0.3,
+                       kmax=1 << 24)
+
+
+def _check(oracle, job, p0, p1, fac, bitmap):
+    plist = oracle.primes(p0, p1)
+    ofac, _, obm = oracle.brute(oracle_job(oracle, job), plist, ref_skip=True)
+    assert _terms(fac) == _terms(ofac)
+    assert np.array_equal(bitmap, obm)
+    return len(plist)
+
+
+@pytest.mark.parametrize("kcount", [1, 8, 20, 68])     # a warp per prime; 20 and 68: four primes may share a round
+@pytest.mark.parametrize("base", [3, 6, 10, 15])       # odd primes that divide the base at the start of the range
+def test_primes_dividing_the_base(rs, oracle, sieve, base, kcount):
+    """The range's first records are primes that divide the base: in a batch that
+    has used none of its record slots before, and in the single-job path."""
+    job = _small_job(base, kcount)
+    with closing(rs.Batch(0, max_jobs=2, range_slots=3)) as b:
+        j = b.add(W.seqs_of(job), 3, 60_000)
+        assert b.run(0)
+        n = _check(oracle, job, 3, 60_000, b.factors(j), b.bitmap(j))
+        assert b.job_info(j)[1] == n
+    sieve.load(W.seqs_of(job))
+    assert sieve.run(3, 60_000)["primes"] == n
+    _check(oracle, job, 3, 60_000, sieve.factors(), sieve.bitmap())
+
+
+def test_first_range_slot_without_a_prime(rs, oracle):
+    """Range slot 0 holds no prime in the batch's first round, and a number of
+    primes that is no multiple of 32 in the next slot; then slot 0 is reused."""
+    empty, job, late = _small_job(2, 5), _small_job(3, 20), _small_job(10, 7, seed=1)
+    with closing(rs.Batch(0, max_jobs=4, range_slots=4)) as b:
+        e = b.add(W.seqs_of(empty), 24, 28)
+        j = b.add(W.seqs_of(job), 3, 1_000)
+        assert b.run(0)
+        assert b.job_info(e)[1:] == (0, True) and len(b.factors(e)) == 0
+        _check(oracle, job, 3, 1_000, b.factors(j), b.bitmap(j))
+        b.release(e)
+        k = b.add(W.seqs_of(late), 3, 5_000)
+        assert b.run(0)
+        _check(oracle, late, 3, 5_000, b.factors(k), b.bitmap(k))
