@@ -1043,10 +1043,12 @@ cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const B
                                                        rcap, rec_of);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_setup_k<INT_PRIMES, 32, true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, true, tgt, meta,
-                                                                   stats, gm, geoms, prefix_p, nranges, rec_of);
+    // FP_PRIMES first: it also takes the records without a search from kernel 1 (p = 0 is
+    // below FP_BOUND), and the records that the other launch drops must not be among them
     k_setup_k<FP_PRIMES, 32, true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, true, tgt, meta,
                                                                   stats, gm, geoms, prefix_p, nranges, rec_of);
+    k_setup_k<INT_PRIMES, 32, true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, true, tgt, meta,
+                                                                   stats, gm, geoms, prefix_p, nranges, rec_of);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_setup_tabs<ANY_PRIMES><<<sms * 8, 128, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, stats, lists.list,

@@ -62,3 +62,27 @@ def test_first_range_slot_without_a_prime(rs, oracle):
         k = b.add(W.seqs_of(late), 3, 5_000)
         assert b.run(0)
         _check(oracle, late, 3, 5_000, b.factors(k), b.bitmap(k))
+
+
+# one round and several, one to 100 sequences, primes on both sides of 2^51 (where the
+# set-up's launches part) and of 2^63, and primes that divide the base
+COUNTED = [(1, 2, 3, 40_000), (3, 3, 3, 200_000), (1, 2, (1 << 51) - 100_000, (1 << 51) + 300_000),
+           (20, 3, (1 << 51) - 200_000, (1 << 51) + 200_000), (100, 2, (1 << 58) + 1, (1 << 58) + 100_000),
+           (5, 10, (1 << 63) - 200_000, (1 << 63) + 200_000)]
+
+
+def test_counters_equal_the_single_job_path(rs, sieve):
+    jobs = [(_small_job(base, kcount), p0, p1) for kcount, base, p0, p1 in COUNTED]
+    want = dict.fromkeys(("primes", "skipped", "full", "parity", "targets", "factors", "dups"), 0)
+    for job, p0, p1 in jobs:
+        sieve.load(W.seqs_of(job))
+        cnt = sieve.run(p0, p1)
+        assert cnt["skipped"] + cnt["full"] + cnt["parity"] == cnt["primes"]
+        for key in want:
+            want[key] += cnt[key]
+    with closing(rs.Batch(0, max_jobs=len(jobs), range_slots=2 * len(jobs))) as b:
+        for job, p0, p1 in jobs:
+            assert b.add(W.seqs_of(job), p0, p1) is not None
+        assert b.run(0)
+        got = b.counters()
+    assert {key: got[key] for key in want} == want
