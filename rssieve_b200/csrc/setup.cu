@@ -944,10 +944,13 @@ __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restri
     u32 i = (blockIdx.x * SETUP_TPB + threadIdx.x) / GL;
     if constexpr (GL == 32) {
         // four consecutive primes per warp when the sequences leave a partial round
-        // that they can share, else one
+        // that they can share, else one.  A round of a batch only knows its primes here:
+        // four as in launch_setup_kind when every warp of the grid then still has some
+        // (100 sequences near 2^58, a round of 430 primes: 354 us with four at any
+        // size, 283 with one).
         static_assert(KIND != ANY_PRIMES, "a warp holds primes of one step kind");
         const u32 total = BATCH ? prefix[nr] : count;
-        const u32 per = four ? 4 : 1;
+        const u32 per = four && (!BATCH || total >= 4 * stride) ? 4 : 1;
         for (i *= per; i < total; i += stride * per) {
             const u32 n = min(per, total - i);
             // lane q: prime q (mine: of this launch's kind; a skipped one, p = 0, counts
@@ -960,7 +963,7 @@ __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restri
                 mine = !BATCH || (hdr[rec].p < FP_BOUND) == (KIND == FP_PRIMES);
             }
             const u32 todo = __ballot_sync(0xFFFFFFFFu, mine);
-            if (four && todo) {
+            if (per == 4 && todo) {
                 const u32 j0 = __shfl_sync(0xFFFFFFFFu, jb, 0);
                 rest = shares_rest(jobs[j0].kcount) && __all_sync(0xFFFFFFFFu, l >= n || (mine && jb == j0));
                 if (rest) rest_powers<KIND == FP_PRIMES>(jobs + j0, rec, n, hdr, aux, tgt);

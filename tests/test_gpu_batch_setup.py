@@ -71,8 +71,7 @@ COUNTED = [(1, 2, 3, 40_000), (3, 3, 3, 200_000), (1, 2, (1 << 51) - 100_000, (1
            (5, 10, (1 << 63) - 200_000, (1 << 63) + 200_000)]
 
 
-def test_counters_equal_the_single_job_path(rs, sieve):
-    jobs = [(_small_job(base, kcount), p0, p1) for kcount, base, p0, p1 in COUNTED]
+def _check_counters(rs, sieve, jobs):
     want = dict.fromkeys(("primes", "skipped", "full", "parity", "targets", "factors", "dups"), 0)
     for job, p0, p1 in jobs:
         sieve.load(W.seqs_of(job))
@@ -86,3 +85,18 @@ def test_counters_equal_the_single_job_path(rs, sieve):
         assert b.run(0)
         got = b.counters()
     assert {key: got[key] for key in want} == want
+
+
+def test_counters_equal_the_single_job_path(rs, sieve):
+    _check_counters(rs, sieve, [(_small_job(base, kcount), p0, p1) for kcount, base, p0, p1 in COUNTED])
+
+
+# From 4 * 4 * 8 * 148 = 18944 primes in a round a warp takes four primes, which may
+# share their last, partial round of sequences (20 and 68; 100 has none to share):
+# about 17800 and 20300 primes, and a round of two jobs that a warp's four may straddle.
+@pytest.mark.parametrize("p0,widths", [(10 ** 7, (288_000, 328_000)), (1 << 52, (642_000, 732_000))])
+@pytest.mark.parametrize("kcounts", [(20,), (68,), (100,), (68, 20)])
+def test_primes_per_warp(rs, sieve, kcounts, p0, widths):
+    for w in widths:
+        w = w // len(kcounts)
+        _check_counters(rs, sieve, [(_small_job(3, k), p0 + i * w, p0 + (i + 1) * w) for i, k in enumerate(kcounts)])
