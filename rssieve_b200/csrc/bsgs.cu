@@ -185,7 +185,8 @@ struct Slice {
     u32 order;                   // ord(s) when it is at most Q', else NONE
     u32 abort;                   // a record wait gave up
     u32 nq;                      // filter passes put on the queue
-    u32 pad_[2];
+    u32 w0, w1, t0, t1;          // this pass: giant steps [t0, t1) of the chunks of items [w0, w1)
+    u64 zt;                      // S^t0
     u64 pw[16];                  // s^l, l < 16
 };
 static_assert(sizeof(Slice) % 16 == 0, "slices start on 16-byte boundaries");
@@ -325,32 +326,64 @@ __device__ __forceinline__ void check_pass(const Ring<MODE> &R, Slice *sl, const
     if (n <= args->nmax) claim(*args, H->p, m & 0x7Fu, (u32)n);
 }
 
-// Start value of item w: T_i * S^(g*Lc).
+// Pass seg of a prime whose chunks are longer than a pass should be: `piece` steps of
+// one round's chunks.  Returns the round.
 template <int MODE>
-__device__ __forceinline__ typename Ring<MODE>::V item_start(const Ring<MODE> &R, u32 w, const PrimeHdr *H, const u64 *tb,
-                                                             const u64 *tg)
+__device__ __noinline__ u32 cut_chunk(Slice *sl, const PrimeHdr *H, u32 seg)
+{
+    typedef typename Ring<MODE>::V V;
+    const Ring<MODE> R(*H);
+    const u32 n = (H->Lc + H->piece - 1) / H->piece, r = seg / n, t0 = (seg - r * n) * H->piece;
+    sl->t0 = t0;
+    sl->t1 = min(t0 + H->piece, H->Lc);
+    V z = Ring<MODE>::one(*H), x = Ring<MODE>::val(H->S);
+    for (u32 k = t0; k; k >>= 1) {
+        if (k & 1) z = R.mul(z, x);
+        x = R.mul(x, x);
+    }
+    sl->zt = Ring<MODE>::bits(z);
+    return r;
+}
+// What pass seg of a prime walks (Slice): `rounds` rounds of 2 GS items and their whole
+// chunks, or a part of one round's.  By the group's first thread.
+template <int MODE>
+__device__ __forceinline__ void start_pass(Slice *sl, const PrimeHdr *H, u32 gs, u32 seg)
+{
+    sl->t0 = 0;
+    sl->t1 = H->Lc;
+    if (H->piece < H->Lc) seg = cut_chunk<MODE>(sl, H, seg);
+    const u32 per = H->rounds * 2 * gs;
+    sl->w0 = seg * per;
+    sl->w1 = min((seg + 1) * per, H->numk * H->G);
+}
+
+// Value of item w at the pass's first giant step: T_i * S^(g*Lc + t0).
+template <int MODE>
+__device__ __forceinline__ typename Ring<MODE>::V item_start(const Ring<MODE> &R, u32 w, const Slice *sl, const PrimeHdr *H,
+                                                             const u64 *tb, const u64 *tg)
 {
     typedef typename Ring<MODE>::V V;
     u32 g, i;
     item_of(w, H, g, i);
     V z = Ring<MODE>::val(tb[64 + (g & 31)]);
     if (H->G > 32) z = R.mul(z, Ring<MODE>::val(tb[96 + (g >> 5)]));
+    if (sl->t0) z = R.mul(z, Ring<MODE>::val(sl->zt));
     return R.mul(Ring<MODE>::val(tg[i]), z);
 }
 
 // More filter passes than the queue holds (p not far above Q', where most are
-// true): the giant steps of items [w0, w1) again, one item per thread, each
-// value checked by its own thread.
+// true): the pass's giant steps again, one item per thread, each value checked by
+// its own thread.
 template <int MODE>
-__device__ __noinline__ void giant_unqueued(Slice *sl, const PrimeHdr *H, u32 gs, u32 gt, u32 w0, u32 w1, const u64 *tb,
-                                            const u64 *tg, const BsgsArgs *args, const unsigned short *meta)
+__device__ __noinline__ void giant_unqueued(Slice *sl, const PrimeHdr *H, u32 gs, u32 gt, const u64 *tb, const u64 *tg,
+                                            const BsgsArgs *args, const unsigned short *meta)
 {
     typedef typename Ring<MODE>::V V;
     const Ring<MODE> R(*H);
     const typename Ring<MODE>::Fix f = Ring<MODE>::giant(*H);
-    for (u32 w = w0 + gt; w < w1; w += gs) {
-        V g = item_start<MODE>(R, w, H, tb, tg);
-        for (u32 t = 0; t < H->Lc; ++t, g = R.step(g, f))
+    for (u32 w = sl->w0 + gt; w < sl->w1; w += gs) {
+        V g = item_start<MODE>(R, w, sl, H, tb, tg);
+        for (u32 t = sl->t0; t < sl->t1; ++t, g = R.step(g, f))
             for (u32 l = 0; l < 16; ++l) check_pass<MODE>(R, sl, H, gs, Ring<MODE>::bits(g), w, t, l, args, meta);
     }
 }
@@ -478,7 +511,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
         group_sync(gid, gs);
 
         // one pass of the loop per prime, or per segment seg of a prime with a long
-        // giant phase (every segment fills the filter again)
+        // giant phase (every segment fills the filter again; start_pass says what it walks)
         for (u32 it = 0, seg = 0;;) {
             const u32 buf = it & 1;
             const u32 r = sl->idx[buf];
@@ -507,6 +540,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
             if (gt == 0) {
                 sl->order = NONE;
                 sl->nq = 0;
+                if (!sl->abort) start_pass<MODE>(sl, &sl->hdr[buf], gs, seg);   // (the header is here)
             }
             group_sync(gid, gs);
             if (sl->abort) {
@@ -583,8 +617,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
             const u32 order = sl->order;                          // (the first thread resets it for the next pass)
             if (order == NONE) {
                 // ---- giant steps: items (target i, chunk g), two per thread at a time ----
-                const u32 nitems = H->numk * H->G;
-                const u32 wend = min((seg + 1) * H->rounds * 2 * gs, nitems);
+                const u32 wend = sl->w1, nitems = H->numk * H->G;
                 const typename RM::Fix f = RM::giant(*H);
                 // a filter pass of giant step t of item w goes on the queue (a lane
                 // past the last item repeats it, and its passes are that item's own)
@@ -594,15 +627,15 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
                     const u32 k = atomicAdd(&sl->nq, 1u);
                     if (k < gs / 4) slice_queue(sl, gs)[k] = make_uint4((u32)v, (u32)(v >> 32), w, t);
                 };
-                for (u32 w = seg * H->rounds * 2 * gs + gt; (w & ~31u) < wend; w += 2 * gs) {
-                    V gA = item_start<MODE>(R, min(w, nitems - 1), H, tb, tg);
-                    const u32 Lc = H->Lc;
+                for (u32 w = sl->w0 + gt; (w & ~31u) < wend; w += 2 * gs) {
+                    V gA = item_start<MODE>(R, min(w, nitems - 1), sl, H, tb, tg);
+                    const u32 t1 = sl->t1;
+                    u32 t = sl->t0;
                     if ((w & ~31u) + gs < nitems) {
-                        V gB = item_start<MODE>(R, min(w + gs, nitems - 1), H, tb, tg);
+                        V gB = item_start<MODE>(R, min(w + gs, nitems - 1), sl, H, tb, tg);
                         // two steps of both chains per test of the four probes
-                        u32 t = 0;
 #pragma unroll GIANT_UNROLL
-                        for (; t + 1 < Lc; t += 2) {
+                        for (; t + 1 < t1; t += 2) {
                             const u32 ha = val_hash(RM::bits(gA)), hb = val_hash(RM::bits(gB));
                             const u32 fa = filt[__umulhi(ha, nw)], fb = filt[__umulhi(hb, nw)];
                             const V nA = R.step(gA, f), nB = R.step(gB, f);
@@ -621,13 +654,13 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
                             gA = mA;
                             gB = mB;
                         }
-                        if (t < Lc) {
+                        if (t < t1) {
                             const u32 ha = val_hash(RM::bits(gA)), hb = val_hash(RM::bits(gB));
                             if ((filter_mask(ha) & ~filt[__umulhi(ha, nw)]) == 0) pass(gA, w, t);
                             if ((filter_mask(hb) & ~filt[__umulhi(hb, nw)]) == 0) pass(gB, w + gs, t);
                         }
                     } else {
-                        for (u32 t = 0; t < Lc; ++t) {
+                        for (; t < t1; ++t) {
                             const u32 ha = val_hash(RM::bits(gA));
                             const u32 fa = filt[__umulhi(ha, nw)];
                             const V nA = R.step(gA, f);
@@ -655,8 +688,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
                         check_pass<MODE>(RM(*H), sl, H, gs, ((u64)x.y << 32) | x.x, x.z, x.w, gt & 15, args, mt);
                     }
                 } else {
-                    const u32 per = H->rounds * 2 * gs;
-                    giant_unqueued<MODE>(sl, H, gs, gt, seg * per, min((seg + 1) * per, H->numk * H->G), tb, tg, args, mt);
+                    giant_unqueued<MODE>(sl, H, gs, gt, tb, tg, args, mt);
                 }
                 if (gt == 0) atomicAdd(&s_cands, (unsigned long long)nq);
                 group_sync(gid, gs);

@@ -152,7 +152,7 @@ struct PrimeHdr {        // 128 bytes (a 16-byte multiple: copied by TMA bulk co
     u32 cls;             // class: Q' = 512 << cls, 32 << cls threads
     float rk;            // 1/numk
     u32 nseg, rounds;    // segments of a long giant phase: rounds of 2 * (32 << cls) items each
-    u32 pad_;
+    u32 piece;           // giant steps of a chunk per segment: Lc, or less with a single round
 };
 static_assert(sizeof(PrimeHdr) == 128, "PrimeHdr is copied in 16-byte units");
 

@@ -341,7 +341,7 @@ __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, 
     }
     H.numk = 0; H.e = e; H.G = 0; H.Lc = 0; H.job = jb; H.Mg = 0; H.cls = 0;
     H.smul = small_power(b, e);
-    H.rk = 0; H.nseg = 0; H.rounds = 0; H.pad_ = 0;
+    H.rk = 0; H.nseg = 0; H.rounds = 0; H.piece = 0;
     hdr[t] = H;
     aux[t] = X;
 }
@@ -773,10 +773,15 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
 // `run` steps per chain (48 unless p is small) leaves about a quarter of the
 // queue's room, GS/16 passes; longer giant phases are cut into chunks and
 // segments of that length.  G is at most 1024 (the start tables), and a
-// target's last chunk is never empty.
-__device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float p, u32 &G, u32 &Lc, u32 &nseg, u32 &rounds)
+// target's last chunk is never empty.  A chunk that is longer all the same (Mg
+// above 1024 times the length) is walked in several segments, `piece` steps of
+// one round's chunks in each: one sequence, n-range 2^32, Q' = 1024 near 2^47
+// took 339 us per prime with segments of whole chunks, every queue overflowing.
+__device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float p, u32 &G, u32 &Lc, u32 &nseg, u32 &rounds,
+                                            u32 &piece)
 {
-    const u32 run = (u32)fminf(48.0f, fmaxf(1.0f, 1.0f / (32.0f * (5.0e-4f + 16.0f * (float)gs / p))));
+    const float fill = fmaxf(1.0f, 1.0f / (32.0f * (5.0e-4f + 16.0f * (float)gs / p)));
+    const u32 run = (u32)fminf(48.0f, fill);
     u32 best = 0xFFFFFFFFu, hb = 0;
     for (u32 h = 1; h <= 8; ++h) {
         u32 g = gs * h / nk;
@@ -795,6 +800,10 @@ __device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float p, u32
     const u32 total = (nk * G + 2 * gs - 1) / (2 * gs);   // rounds
     rounds = min(total, max(run / Lc, 1u));
     nseg = (total + rounds - 1) / rounds;
+    // (a round of half the items leaves twice the room)
+    const u32 most = (u32)(nk * G <= gs ? 2.0f * fill : fill), pieces = (Lc + most - 1) / most;
+    piece = (Lc + pieces - 1) / pieces;
+    nseg *= (Lc + piece - 1) / piece;                     // (1 for more rounds than one: then 2*Lc <= run)
 }
 
 // Baby- and giant-step tables of record t (one thread): giant steps per target
@@ -819,8 +828,8 @@ __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u
     // (L - 1 and not L + e - 1: an n-range may be 2^32 - 1 long; without run job is not the record's)
     const u32 Le = run ? (job->L - 1) / e + 1 : 1;
     const u32 Mg = ((Le - 1) >> lq) + 1;
-    u32 G, Lc, nseg, rounds;
-    giant_split(gs, nk, Mg, (float)h.p, G, Lc, nseg, rounds);
+    u32 G, Lc, nseg, rounds, piece;
+    giant_split(gs, nk, Mg, (float)h.p, G, Lc, nseg, rounds, piece);
     const V s = F::val(h.s), S = F::val(aux[t].S[cls]);          // (not a record's when !run: never stored)
     V u8 = f.mul(s, s);
     u8 = f.mul(u8, u8);
@@ -859,6 +868,7 @@ __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u
     h.rk = 1.0f / (float)nk;
     h.nseg = nseg;
     h.rounds = rounds;
+    h.piece = piece;
     h.S = F::bits(S);
     h.u8 = F::bits(u8);
     if constexpr (FP) {
