@@ -173,7 +173,7 @@ constexpr u32 WAIT_BOUND = 1u << 24;   // default try_wait rounds before a copy 
 constexpr u32 NONE = 0xFFFFFFFFu;
 
 // ---- a group's slice of the CTA's dynamic shared memory ----
-// Slice | anchors start[GS + 1] (+1 pad) | filter words | queue of GS/4 filter
+// Slice | anchors start[GS + 1] (+1 pad) | filter words | queue of GS/2 filter
 // passes.  The index of the anchors takes the filter's place once the giant
 // steps are done.
 // The rare paths are __noinline__ functions that take the slice and a few
@@ -198,7 +198,7 @@ static_assert(INDEX_PT <= FILTER_WPT, "the index lies in the filter's words");
 __device__ __forceinline__ uint4 *slice_queue(Slice *s, u32 gs) { return reinterpret_cast<uint4 *>(slice_filter(s, gs) + FILTER_WPT * gs); }
 __host__ __device__ constexpr size_t slice_bytes(u32 gs)
 {
-    return sizeof(Slice) + (gs + 2) * 8 + (size_t)FILTER_WPT * gs * 4 + gs / 4 * 16;
+    return sizeof(Slice) + (gs + 2) * 8 + (size_t)FILTER_WPT * gs * 4 + gs / 2 * 16;
 }
 static_assert(slice_bytes(32) % 16 == 0, "slices start on 16-byte boundaries");
 // the slices of TPB/gs groups take the most room for gs = 32
@@ -209,6 +209,14 @@ extern __shared__ __align__(128) unsigned char smem_raw[];
 __shared__ unsigned long long s_cands, s_dups, s_facs;   // per-CTA totals
 __shared__ unsigned long long s_baby, s_giant, s_small;
 
+// One more for each of the warp's lanes here together, by one atomic (a 64-bit add in
+// shared memory by every lane to the same word: 38 cycles of an SM per claim).
+__device__ __forceinline__ void count(unsigned long long *total)
+{
+    const u32 here = __activemask();
+    if ((threadIdx.x & 31) == (u32)__ffs((int)here) - 1) atomicAdd(total, (unsigned long long)__popc(here));
+}
+
 // First claimer of term (seq, n) clears its bitmap bit and appends the factor.
 __device__ __forceinline__ void claim(const BsgsArgs &a, u64 p, u32 seq, u32 n)
 {
@@ -218,7 +226,7 @@ __device__ __forceinline__ void claim(const BsgsArgs &a, u64 p, u32 seq, u32 n)
     const u32 old = atomicAnd(w, ~mask);
     if (old & mask) {
         const u32 f = atomicAdd(a.factor_ctr, 1u);
-        atomicAdd(&s_facs, 1ull);
+        count(&s_facs);
         if (f < a.factor_cap) {
             FactorRec r;
             r.p = p; r.n = n; r.seq = seq;
@@ -227,7 +235,7 @@ __device__ __forceinline__ void claim(const BsgsArgs &a, u64 p, u32 seq, u32 n)
             atomicOr(a.err, ERR_FACTOR_OVERFLOW);
         }
     } else {
-        atomicAdd(&s_dups, 1ull);
+        count(&s_dups);
     }
 }
 
@@ -306,22 +314,26 @@ __device__ __forceinline__ void item_of(u32 w, const PrimeHdr *H, u32 &g, u32 &i
     i = w - g * H->numk;
 }
 
-// Lane l < 16's share of a filter pass's exact check: if gamma * s^l is anchor t,
-// gamma = s^j with j = 16t - l, and for 0 <= j < Q' the step (item w, giant step
-// t of its chunk) claims n = nmin + off + e*((q+1)Q'-1-j).
+// One sixteenth of a filter pass's exact check: if gamma * s^l is anchor t, gamma =
+// s^j with j = 16t - l.  Returns j when it lies in [0, Q'), else NONE.
 template <int MODE>
-__device__ __forceinline__ void check_pass(const Ring<MODE> &R, Slice *sl, const PrimeHdr *H, u32 gs, u64 gamma, u32 w,
-                                           u32 t, u32 l, const BsgsArgs *args, const unsigned short *meta)
+__device__ __forceinline__ u32 log_at(const Ring<MODE> &R, Slice *sl, u32 gs, u64 gamma, u32 l)
 {
     const u32 a = anchor_find(slice_filter(sl, gs), slice_start(sl), gs,
                               Ring<MODE>::bits(R.mul(Ring<MODE>::val(gamma), Ring<MODE>::val(sl->pw[l]))));
-    if (a == NONE) return;
-    const int Q = 16 * (int)gs, j = 16 * (int)a - (int)l;
-    if (j < 0 || j >= Q) return;
+    const u32 j = 16 * a - l;                              // (negative: past the end as well)
+    return (a != NONE && j < 16 * gs) ? j : NONE;
+}
+
+// Claims the term of item w's giant step t (of its chunk), whose value is s^j: n =
+// nmin + off + e*((q+1)Q'-1-j).
+__device__ __forceinline__ void claim_step(const PrimeHdr *H, u32 gs, u32 j, u32 w, u32 t, const BsgsArgs *args,
+                                           const unsigned short *meta)
+{
     u32 g, i;
     item_of(w, H, g, i);
     const u32 m = meta[i];
-    const u64 u = (u64)(g * H->Lc + t + 1) * (u32)Q - 1 - (u32)j;
+    const u64 u = (u64)(g * H->Lc + t + 1) * (16 * gs) - 1 - j;
     const u64 n = (u64)args->nmin + (m >> 7) + (u64)H->e * u;
     if (n <= args->nmax) claim(*args, H->p, m & 0x7Fu, (u32)n);
 }
@@ -383,8 +395,11 @@ __device__ __noinline__ void giant_unqueued(Slice *sl, const PrimeHdr *H, u32 gs
     const typename Ring<MODE>::Fix f = Ring<MODE>::giant(*H);
     for (u32 w = sl->w0 + gt; w < sl->w1; w += gs) {
         V g = item_start<MODE>(R, w, sl, H, tb, tg);
-        for (u32 t = sl->t0; t < sl->t1; ++t, g = R.step(g, f))
-            for (u32 l = 0; l < 16; ++l) check_pass<MODE>(R, sl, H, gs, Ring<MODE>::bits(g), w, t, l, args, meta);
+        for (u32 t = sl->t0; t < sl->t1; ++t, g = R.step(g, f)) {
+            u32 j = NONE;                                  // (claimed past the loop: by all lanes of a warp together)
+            for (u32 l = 0; l < 16 && j == NONE; ++l) j = log_at<MODE>(R, sl, gs, Ring<MODE>::bits(g), l);
+            if (j != NONE) claim_step(H, gs, j, w, t, args, meta);
+        }
     }
 }
 
@@ -625,7 +640,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
                     if (w >= nitems) return;
                     const u64 v = RM::bits(g);
                     const u32 k = atomicAdd(&sl->nq, 1u);
-                    if (k < gs / 4) slice_queue(sl, gs)[k] = make_uint4((u32)v, (u32)(v >> 32), w, t);
+                    if (k < gs / 2) slice_queue(sl, gs)[k] = make_uint4((u32)v, (u32)(v >> 32), w, t);
                 };
                 for (u32 w = sl->w0 + gt; (w & ~31u) < wend; w += 2 * gs) {
                     V gA = item_start<MODE>(R, min(w, nitems - 1), sl, H, tb, tg);
@@ -682,10 +697,11 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
                 build_index<MODE>(sl, H, gid, gs, gt);
                 const BsgsArgs *args = BATCH ? job_args + H->job : &s_args;
                 const unsigned short *mt = meta + (size_t)r * KSTRIDE;
-                if (nq <= gs / 4) {
+                if (nq <= gs / 2) {
                     for (u32 k = gt >> 4; k < nq; k += gs >> 4) {
                         const uint4 x = slice_queue(sl, gs)[k];
-                        check_pass<MODE>(RM(*H), sl, H, gs, ((u64)x.y << 32) | x.x, x.z, x.w, gt & 15, args, mt);
+                        const u32 j = log_at<MODE>(RM(*H), sl, gs, ((u64)x.y << 32) | x.x, gt & 15);
+                        if (j != NONE) claim_step(H, gs, j, x.z, x.w, args, mt);
                     }
                 } else {
                     giant_unqueued<MODE>(sl, H, gs, gt, tb, tg, args, mt);

@@ -769,18 +769,20 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
 // an odd h counting half a round more (an item's start values cost about three
 // steps, and an odd half round runs one chain per thread instead of two).  A
 // segment is checked for filter passes at its end: the filter passes one value
-// in 2000 that is not there and Q'/p of all values are there, so a segment of
-// `run` steps per chain (48 unless p is small) leaves about a quarter of the
-// queue's room, GS/16 passes; longer giant phases are cut into chunks and
-// segments of that length.  G is at most 1024 (the start tables), and a
-// target's last chunk is never empty.  A chunk that is longer all the same (Mg
-// above 1024 times the length) is walked in several segments, `piece` steps of
-// one round's chunks in each: one sequence, n-range 2^32, Q' = 1024 near 2^47
+// in 2000 that is not there, and Q'/E of all values are there (they and the s^j lie
+// in the group of order E, PrimeAux), so a segment of `run` steps per chain (48
+// unless E is small) fills at most a quarter of the queue, GS/8 passes (with Q'/p
+// for the share that is there, queues overflowed up to p of 10^8: 100 sequences,
+// n-range 6*10^6, p from 2*10^6 to 8*10^6, 124 ns per prime, now 75); longer giant
+// phases are cut into chunks and segments of that length.  G is at most 1024 (the
+// start tables), and a target's last chunk is never empty.  A chunk that is longer all
+// the same (Mg above 1024 times the length) is walked in several segments, `piece`
+// steps of one round's chunks in each: one sequence, n-range 2^32, Q' = 1024 near 2^47
 // took 339 us per prime with segments of whole chunks, every queue overflowing.
-__device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float p, u32 &G, u32 &Lc, u32 &nseg, u32 &rounds,
+__device__ __forceinline__ void giant_split(u32 gs, u32 nk, u32 Mg, float E, u32 &G, u32 &Lc, u32 &nseg, u32 &rounds,
                                             u32 &piece)
 {
-    const float fill = fmaxf(1.0f, 1.0f / (32.0f * (5.0e-4f + 16.0f * (float)gs / p)));
+    const float fill = fmaxf(1.0f, 1.0f / (16.0f * (5.0e-4f + 16.0f * (float)gs / E)));
     const u32 run = (u32)fminf(48.0f, fill);
     u32 best = 0xFFFFFFFFu, hb = 0;
     for (u32 h = 1; h <= 8; ++h) {
@@ -829,7 +831,7 @@ __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u
     const u32 Le = run ? (job->L - 1) / e + 1 : 1;
     const u32 Mg = ((Le - 1) >> lq) + 1;
     u32 G, Lc, nseg, rounds, piece;
-    giant_split(gs, nk, Mg, (float)h.p, G, Lc, nseg, rounds, piece);
+    giant_split(gs, nk, Mg, (float)aux[t].E, G, Lc, nseg, rounds, piece);
     const V s = F::val(h.s), S = F::val(aux[t].S[cls]);          // (not a record's when !run: never stored)
     V u8 = f.mul(s, s);
     u8 = f.mul(u8, u8);
