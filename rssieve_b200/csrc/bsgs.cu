@@ -262,12 +262,13 @@ __device__ __noinline__ void build_index(Slice *sl, const PrimeHdr *H, u32 gid, 
     }
     group_sync(gid, gs);
     // anchors t = gt, and by the first thread the one past the end, s^Q'; at most
-    // GS + 1 entries, so the walks end
+    // GS + 1 entries, so the walks end.  Of equal ones (ord(s) <= Q') one is enough:
+    // all of them, in one run of slots, made every walk as long as the run.
     for (u32 t = gt; t < gs + 1; t += gs) {
         const u64 v = (t == gs) ? H->S : start[t];
         if (t == gs) start[gs] = v;
         u32 k = __umulhi(val_hash(v), INDEX_PT * gs);
-        while (atomicCAS(&idx[k], 0u, t + 1) != 0u) k = (k + 1) & (INDEX_PT * gs - 1);
+        for (u32 e; (e = atomicCAS(&idx[k], 0u, t + 1)) != 0u && start[e - 1] != v;) k = (k + 1) & (INDEX_PT * gs - 1);
     }
     group_sync(gid, gs);
 }
@@ -403,27 +404,41 @@ __device__ __noinline__ void giant_unqueued(Slice *sl, const PrimeHdr *H, u32 gs
     }
 }
 
-// ord(s) <= Q': each target is looked up once; every n in range with the same
-// residue mod e*ord is claimed (giant.cl:146-168).  Warps of the group take
-// targets in turn.  Called by whole warps.
+// ord(s) <= Q': each target is looked up once, warps of the group taking targets in
+// turn, and every n in range with the same residue mod e*ord is claimed
+// (giant.cl:146-168): blocks of 32 claims of all targets, dealt to the warps in turn,
+// as there may be fewer targets than warps, of 10^5 claims each (100 sequences, n-range
+// 6*10^6, the primes from 100 to 1000: 17.4 ms with a warp per target, 13.3 so).  The
+// targets' first u lie in the filter's words past the index.  Called by the whole group.
 template <int MODE>
-__device__ __noinline__ void small_order_search(Slice *sl, const PrimeHdr *H, const BsgsArgs *args, u32 gs, u32 gt,
+__device__ __noinline__ void small_order_search(Slice *sl, const PrimeHdr *H, const BsgsArgs *args, u32 gid, u32 gs, u32 gt,
                                                 const u64 *__restrict__ tgt, const unsigned short *__restrict__ meta)
 {
+    static_assert((FILTER_WPT - INDEX_PT) * 32 >= KMAX, "room for the targets' first u");
     const Ring<MODE> R(*H);
-    const u32 lane = gt & 31;
+    const u32 lane = gt & 31, warps = gs >> 5, numk = H->numk;
     const u32 Q = 16 * gs, order = sl->order;
-    for (u32 i = gt >> 5; i < H->numk; i += gs >> 5) {
+    u32 *first = slice_filter(sl, gs) + INDEX_PT * gs;
+    for (u32 i = gt >> 5; i < numk; i += warps) {
         const int j = warp_find<MODE>(R, sl, gs, Ring<MODE>::val(tgt[i]));
-        if (j == NO_LOG) continue;
-        if (lane == 0) atomicAdd(&s_cands, 1ull);
-        const u32 u0 = (u32)((int)(Q - 1 + order) - j) % order;
-        const u32 m = meta[i];
-        for (u64 u = u0 + (u64)lane * order;; u += 32ull * order) {
-            const u64 n = (u64)args->nmin + (m >> 7) + (u64)H->e * u;
-            if (n > args->nmax) break;
-            claim(*args, H->p, m & 0x7Fu, (u32)n);
+        if (lane == 0) {
+            first[i] = (j == NO_LOG) ? NONE : (u32)((int)(Q - 1 + order) - j) % order;
+            if (j != NO_LOG) atomicAdd(&s_cands, 1ull);
         }
+    }
+    group_sync(gid, gs);
+    // u < ceil(L/e), blocks of 32*order of them
+    const u64 span = 32ull * order;
+    const u32 blocks = (u32)((args->nmax - args->nmin) / H->e / span) + 1;
+    for (u32 i = 0, k = gt >> 5;; k += warps) {
+        while (i < numk && (first[i] == NONE || k >= blocks)) {
+            if (first[i] != NONE) k -= blocks;
+            ++i;
+        }
+        if (i >= numk) return;
+        const u32 m = meta[i];
+        const u64 n = (u64)args->nmin + (m >> 7) + (u64)H->e * (first[i] + lane * order + k * span);
+        if (n <= args->nmax) claim(*args, H->p, m & 0x7Fu, (u32)n);
     }
 }
 
@@ -686,7 +701,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
                 }
             } else {
                 build_index<MODE>(sl, H, gid, gs, gt);
-                small_order_search<MODE>(sl, H, BATCH ? job_args + H->job : &s_args, gs, gt, tg,
+                small_order_search<MODE>(sl, H, BATCH ? job_args + H->job : &s_args, gid, gs, gt, tg,
                                          meta + (size_t)r * KSTRIDE);
             }
             if (claimer) sl->claim = ahead;

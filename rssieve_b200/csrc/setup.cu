@@ -390,7 +390,13 @@ __global__ void __launch_bounds__(128, 8) k_setup_prime(const JobDev *__restrict
 // gm.classes that minimises 1.5 Q' + nk*ceil(Le/Q') with Q' = 512 << c, baby
 // steps, the work of the 32 << c threads that does not depend on their steps
 // (clearing the filter, start values; about eight steps each) and giant steps.
-__device__ __forceinline__ u32 choose_class(const JobGeom &gm, u32 nk, u32 Le)
+// Where solutions are many (`claims` of them expected, as ord(s) divides E), each
+// also costs a group's 32 << c threads a claim, about 16 steps' time, and with Q' < E
+// an exact check as well, 64; with Q' >= E ord(s) is found among the baby steps and
+// there are no giant steps.  (By giant steps alone, 100 sequences, n-range 6*10^6:
+// p from 100 to 1000 75 ms, now 13; from 10^6 to 2*10^6 10.2, now 7.8.)
+template <bool CLAIMS>
+__device__ __forceinline__ u32 best_class(const JobGeom &gm, u32 nk, u32 Le, u64 E, float claims)
 {
     u32 best_c = 0;
     float best = 3.0e38f;
@@ -398,10 +404,20 @@ __device__ __forceinline__ u32 choose_class(const JobGeom &gm, u32 nk, u32 Le)
     for (u32 c = 0; c < NCLASS; ++c) {
         const u32 lq = 9 + c;
         const u32 mg = ((Le - 1) >> lq) + 1;
-        const float cost = 1.5f * (float)(1u << lq) + (float)nk * (float)mg;
+        float cost = (float)nk * (float)mg;
+        if (CLAIMS) cost = E > (1u << lq) ? cost + 64.0f * claims / (float)(1u << c) : 16.0f * claims / (float)(1u << c);
+        cost += 1.5f * (float)(1u << lq);
         if (((gm.classes >> c) & 1u) && cost < best) { best = cost; best_c = c; }
     }
     return best_c;
+}
+__device__ __noinline__ u32 class_of_many(const JobGeom gm, u32 nk, u32 Le, u64 E)
+{
+    return best_class<true>(gm, nk, Le, E, (float)nk * (float)Le / (float)E);
+}
+__device__ __forceinline__ u32 choose_class(const JobGeom &gm, u32 nk, u32 Le, u64 E)
+{
+    return (u64)nk * Le < E ? best_class<false>(gm, nk, Le, E, 0.0f) : class_of_many(gm, nk, Le, E);
 }
 
 // a[r] = x[r]^ex for r < R, the chains interleaved.  UNIFORM: ex (>= 1) is the
@@ -750,7 +766,7 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
     if (!live || skip) return;
     // baby steps for this prime (the giant-step tables follow in kernel 3), and the
     // targets T = -c * k * b^(nmin + off + e(Q'-1))
-    const u32 cls = choose_class(gm, nk, (job->L - 1) / e + 1);
+    const u32 cls = choose_class(gm, nk, (job->L - 1) / e + 1, E);
     const V wr0 = F::val(X.wr0[cls]);
     for (u32 j = l; j < nk; j += GL) {
         tgt[(size_t)w * KSTRIDE + j] = F::bits(f.mul(F::val(sc.part[j]), wr0));
@@ -773,7 +789,7 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
 // in the group of order E, PrimeAux), so a segment of `run` steps per chain (48
 // unless E is small) fills at most a quarter of the queue, GS/8 passes (with Q'/p
 // for the share that is there, queues overflowed up to p of 10^8: 100 sequences,
-// n-range 6*10^6, p from 2*10^6 to 8*10^6, 124 ns per prime, now 75); longer giant
+// n-range 6*10^6, p from 2*10^6 to 8*10^6, 124 ns per prime, now 65); longer giant
 // phases are cut into chunks and segments of that length.  G is at most 1024 (the
 // start tables), and a target's last chunk is never empty.  A chunk that is longer all
 // the same (Mg above 1024 times the length) is walked in several segments, `piece`

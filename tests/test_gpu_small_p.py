@@ -63,3 +63,16 @@ def test_small_order_at_large_p(sieve, oracle, base, p, kcount):
     job = W.job_dict(base, ks, cs, nmin, nmin + width - 1, W.random_bitmap(kcount, nmin, nmin + width - 1, 0.5, 3))
     cnt = _against_brute(sieve, oracle, job, p - 1, p + 1, 0)
     assert cnt["small_order"] == 1 and cnt["hits"] > 0
+
+
+def test_claims_of_small_orders_fill_the_group(sieve):
+    """100 sequences, n-range 6*10^6, the primes from 100 to 1000: 10^8 solutions and
+    more, each an atomic on the bitmap.  With the chip full these take 0.04 ns each; 143
+    primes, some with many more than others, leave part of it idle.  The bound is five
+    times that (32 threads for a prime of up to 10^6 solutions: 0.43)."""
+    job = W.small_job(77, kcount=100, base=2, nmin=4_000_000, nmax=9_999_999, keep=0.03, kmax=1 << 32)
+    sieve.load(W.seqs_of(job))
+    sieve.run(100, 1_000)
+    cnt = sieve.run(100, 1_000)
+    assert cnt["hits"] > 10 ** 8
+    assert sieve.last_timing()["bsgs_ms_avg"] * 1e6 < 0.2 * cnt["hits"]
