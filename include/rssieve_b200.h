@@ -206,8 +206,8 @@ int rs_last_timing(rs_ctx *ctx, double *bsgs_ms, double *total_kernel_ms, uint32
  * p-range. */
 typedef struct rs_batch rs_batch;
 /* max_jobs job slots and range_slots range slots (0: 64 each).  Each range slot
- * holds one round's buffers (about 136 MB); a job takes one range slot, or two
- * when its p-range straddles 2^63. */
+ * holds one round's buffers (158 MB); a job takes one range slot for each part of
+ * its p-range below 2^51, from there to 2^63 and above, so one to three. */
 int rs_batch_create(int device, uint32_t max_jobs, uint32_t range_slots, rs_batch **out);
 void rs_batch_destroy(rs_batch *b);
 /* A caller stream (cudaStream_t as void*, not the legacy NULL stream); only

@@ -30,7 +30,7 @@
 // (geom_model_best), unless the caller fixes Q.
 //
 // Capacity is fixed when the batch is created: job slots and range slots (each
-// range slot owns one round's buffers, about 170 MB).  Jobs can be added
+// range slot owns one round's buffers, 158 MB).  Jobs can be added
 // between rounds -- their tables are written to device memory that the
 // captured round reads -- and a finished job's slots are released for the
 // next one, so the batch also serves a stream of arriving work units.  The
@@ -157,9 +157,9 @@ extern "C" void rs_batch_destroy(rs_batch *b)
     }
     if (b->fork) cudaEventDestroy(b->fork);
     void *ptrs[] = {b->d_sp, b->d_jobs, b->d_geoms, b->d_args, b->d_fctrs, b->d_ranges, b->d_wins, b->d_ctrs,
-                    b->d_range_primes, b->d_cands, b->d_primes, b->d_hdr, b->d_aux, b->d_tabs, b->d_tgt, b->d_meta,
+                    b->d_range_primes, b->d_primes, b->d_hdr, b->d_aux, b->d_tabs, b->d_tgt, b->d_meta,
                     b->d_err, b->d_stats, b->d_unfinished, b->d_win, b->d_prefix_c, b->d_prefix_p,
-                    b->lists.list, b->lists.ctl, b->d_mid, b->d_mid_r, b->d_mid_ctr, b->d_rec_of};
+                    b->lists.list, b->lists.ctl, b->d_mid_ctr, b->d_rec_of};
     for (void *p : ptrs) cudaFree(p);
     if (b->h_pin) cudaFreeHost(b->h_pin);
     if (b->h_win_pin) cudaFreeHost(b->h_win_pin);
@@ -210,18 +210,17 @@ extern "C" int rs_batch_create(int device, uint32_t max_jobs, uint32_t range_slo
         !alloc((void **)&b->d_args, J * sizeof(BsgsArgs)) || !alloc((void **)&b->d_fctrs, J * 4) ||
         !alloc((void **)&b->d_ranges, R * sizeof(BatchRange)) || !alloc((void **)&b->d_wins, R * sizeof(BatchWin)) ||
         !alloc((void **)&b->d_ctrs, (size_t)R * BR_CTRS * 4) || !alloc((void **)&b->d_range_primes, R * 8) ||
-        !alloc((void **)&b->d_cands, (size_t)R * CCAP * 8) || !alloc((void **)&b->d_primes, (size_t)R * RCAP * 8) ||
-        !alloc((void **)&b->d_mid, (size_t)R * CCAP * 8) || !alloc((void **)&b->d_mid_r, (size_t)R * CCAP * 4) ||
+        !alloc((void **)&b->d_primes, (size_t)R * RCAP * 8) ||
         !alloc((void **)&b->d_mid_ctr, 4) || !alloc((void **)&b->d_rec_of, (size_t)R * RCAP * 4) ||
         !alloc((void **)&b->d_hdr, (size_t)R * RCAP * sizeof(PrimeHdr)) ||
-        !alloc(&b->d_aux, (size_t)R * RCAP * setup_aux_bytes()) ||
+        !alloc(&b->d_aux, (size_t)R * RCAP * SETUP_AUX) ||
         !alloc((void **)&b->d_tabs, (size_t)R * RCAP * TABS * 8) ||
         !alloc((void **)&b->d_tgt, (size_t)R * RCAP * KSTRIDE * 8) ||
         !alloc((void **)&b->d_meta, (size_t)R * RCAP * KSTRIDE * 2) || !alloc((void **)&b->d_win, R * 4) ||
         !alloc((void **)&b->d_prefix_c, (R + 1) * 4) || !alloc((void **)&b->d_prefix_p, (R + 1) * 4) ||
         cudaMallocHost(&b->h_pin, 16) != cudaSuccess || cudaMallocHost(&b->h_win_pin, R * 4) != cudaSuccess) {
         rs_set_error("cannot allocate a batch of %u range slots (about %zu MB)", R,
-                     (size_t)R * RCAP * (sizeof(PrimeHdr) + TABS * 8 + KSTRIDE * 10 + 24 + 8 + 16 + 24 + 4) >> 20);
+                     (size_t)R * RCAP * (sizeof(PrimeHdr) + TABS * 8 + KSTRIDE * 10 + SETUP_AUX + 8 + 4 + 4) >> 20);
         return fail(RS_ENOMEM);
     }
     if (cudaMemcpy(b->d_sp, sp.data(), sp.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -250,9 +249,12 @@ extern "C" int rs_batch_create(int device, uint32_t max_jobs, uint32_t range_slo
         if (cudaMemPoolSetAttribute(b->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
             return fail(RS_ECUDA);
     }
-    b->lists.stride = R * RCAP;
-    if (!alloc((void **)&b->lists.list, (size_t)NGROUP * NCLASS * R * RCAP * 4) ||
-        !alloc((void **)&b->lists.ctl, (size_t)NGROUP * 2 * NCLASS * 4)) {
+    // the generator's lists in the set-up's scratch (SETUP_AUX)
+    static_assert((size_t)CCAP * (8 + 8 + 4) <= (size_t)RCAP * SETUP_AUX, "survivors and probable primes fit the scratch");
+    b->d_cands = (u64 *)b->d_aux;
+    b->d_mid = b->d_cands + (size_t)R * CCAP;
+    b->d_mid_r = (u32 *)(b->d_mid + (size_t)R * CCAP);
+    if (!alloc((void **)&b->lists.list, (size_t)R * RCAP * 4) || !alloc((void **)&b->lists.ctl, NGROUP * LIST_CTL * 4)) {
         rs_set_error("cannot allocate the BSGS group lists");
         return fail(RS_ENOMEM);
     }
@@ -490,7 +492,7 @@ static int batch_round(rs_batch *b)
     BCU(launch_mr_batch2(b->d_cands, CCAP, b->d_primes, RCAP, b->d_ctrs, R, b->d_prefix_c, b->d_mid, b->d_mid_r,
                          R * CCAP, b->d_mid_ctr, b->d_err, b->sms, st));
     BCU(launch_batch_prefix_all(b->d_ranges, R, 1, RCAP, b->d_ctrs, b->d_prefix_p, st));
-    BCU(cudaMemsetAsync(b->lists.ctl, 0, (size_t)NGROUP * 2 * NCLASS * 4, st));
+    BCU(cudaMemsetAsync(b->lists.ctl, 0, NGROUP * LIST_CTL * 4, st));
     BCU(launch_setup_batch(b->d_jobs, b->d_geoms, b->d_ranges, b->d_primes, RCAP, b->d_prefix_p, R, b->d_hdr,
                            b->d_aux, b->d_tabs, b->d_tgt, b->d_meta, b->lists, b->d_stats, b->d_rec_of, b->sms, st));
     BsgsArgs a;
@@ -503,8 +505,7 @@ static int batch_round(rs_batch *b)
     BCU(cudaEventRecord(b->fork, st));
     for (int g = 0; g < NGROUP; ++g) {
         BCU(cudaStreamWaitEvent(b->side[g], b->fork, 0));
-        const BsgsLists L = {b->lists.list + (size_t)g * NCLASS * b->lists.stride, b->lists.stride,
-                             b->lists.ctl + g * 2 * NCLASS};
+        const BsgsLists L = {b->lists.list, 0, b->lists.ctl + g * LIST_CTL};
         BCU(launch_bsgs_batch(a, b->d_args, b->d_hdr, b->d_tabs, b->d_tgt, b->d_meta, L, g, b->sms, b->side[g]));
         BCU(cudaEventRecord(b->join[g], b->side[g]));
         BCU(cudaStreamWaitEvent(st, b->join[g], 0));

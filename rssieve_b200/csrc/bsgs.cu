@@ -461,7 +461,7 @@ __device__ __noinline__ void order_check(Slice *sl, const PrimeHdr *H, u32 j0, u
 }
 
 // The primes of one launch, sorted by class into lists of record indices
-// (setup.cu): count[c] primes of class c at lists + c*stride.  CTAs of TPB
+// (setup.cu, BsgsLists): count[c] primes of class c at lists + c*stride.  CTAs of TPB
 // threads work through the classes from the largest down; a class of GS
 // threads per prime runs TPB/GS groups side by side, each claiming the next
 // prime of the class when it finishes one.  taken[c] starts at zero.
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(TPB, 1024 / TPB)
         u64 *start = slice_start(sl);
         u32 *filt = slice_filter(sl, gs);
         const u32 nw = FILTER_WPT * gs;
-        const u32 *list = lists + (size_t)c * stride;
+        const u32 *list = lists + (BATCH ? count[3 * NCLASS + c] : c * stride);
         auto fetch = [&](u32 buf, u32 r) {                        // group's first thread only
             mbar_expect_tx(&s_bar[w0][buf], (u32)sizeof(PrimeHdr));
             bulk_load(&sl->hdr[buf], hdr + r, (u32)sizeof(PrimeHdr), &s_bar[w0][buf]);

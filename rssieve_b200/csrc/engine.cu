@@ -133,7 +133,6 @@ extern "C" void rs_ctx_destroy(rs_ctx *c)
     cudaFree(c->d_primes);
     cudaFree(c->d_ctrs);
     cudaFree(c->d_hdr);
-    cudaFree(c->d_aux);
     cudaFree(c->d_tabs);
     cudaFree(c->d_tgt);
     cudaFree(c->d_meta);
@@ -172,14 +171,12 @@ extern "C" int rs_ctx_create(int device, rs_ctx **out)
     c->prime_cap = 1u << 24;
     c->chunk_cap = 1u << 17;
     c->lists.stride = c->chunk_cap;
-    const size_t aux_bytes = (size_t)c->chunk_cap * setup_aux_bytes(), list_bytes = (size_t)NCLASS * c->chunk_cap * 4;
     if (cudaMalloc(&c->d_sp, sp.size() * 4) != cudaSuccess ||
         cudaMalloc(&c->d_cands, (size_t)c->cand_cap * 8) != cudaSuccess ||
         cudaMalloc(&c->d_mid, (size_t)c->cand_cap * 8) != cudaSuccess ||
         cudaMalloc(&c->d_primes, (size_t)c->prime_cap * 8) != cudaSuccess ||
         cudaMalloc(&c->d_ctrs, BLOCK_BYTES) != cudaSuccess ||
         cudaMalloc(&c->d_hdr, (size_t)c->chunk_cap * sizeof(PrimeHdr)) != cudaSuccess ||
-        cudaMalloc(&c->d_aux, aux_bytes + list_bytes + 2 * NCLASS * 4) != cudaSuccess ||
         cudaMalloc(&c->d_tabs, (size_t)c->chunk_cap * TABS * 8) != cudaSuccess ||
         cudaMalloc(&c->d_tgt, (size_t)c->chunk_cap * KSTRIDE * 8) != cudaSuccess ||
         cudaMalloc(&c->d_meta, (size_t)c->chunk_cap * KSTRIDE * 2) != cudaSuccess ||
@@ -191,7 +188,12 @@ extern "C" int rs_ctx_create(int device, rs_ctx **out)
     if (cudaMemcpy(c->d_sp, sp.data(), sp.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(c->d_ctrs, 0, BLOCK_BYTES) != cudaSuccess)
         return fail(RS_ECUDA);
-    // (behind the scratch: as allocations of their own they took 1 ms of a context's 8)
+    // the set-up's scratch and the class lists in the memory of the probable primes, which
+    // nothing reads once a segment's primes are there (as allocations of their own they
+    // took 1 ms of a context's 8)
+    const size_t aux_bytes = (size_t)c->chunk_cap * SETUP_AUX;
+    if (aux_bytes + ((size_t)NCLASS * c->chunk_cap + 2 * NCLASS) * 4 > (size_t)c->cand_cap * 8) return fail(RS_ENOMEM);
+    c->d_aux = c->d_mid;
     c->lists.list = reinterpret_cast<u32 *>((char *)c->d_aux + aux_bytes);
     c->lists.ctl = c->lists.list + (size_t)NCLASS * c->chunk_cap;
     c->d_err = c->d_ctrs + CTR_ERR;

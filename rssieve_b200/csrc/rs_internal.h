@@ -205,12 +205,19 @@ inline JobGeom job_geom(int g)
     return G;
 }
 // One BSGS launch's primes, sorted by class: ctl[c] record indices of class c
-// at list + c*stride; ctl[NCLASS + c] counts those taken (zero at the start).
+// at list + c*stride (a batch's group: at list + ctl[3*NCLASS + c]); ctl[NCLASS + c]
+// counts those taken.  A batch's groups share one list, so that it needs one entry per
+// record and not one per record, group and class: ctl[2*NCLASS + c] counts the class
+// before the list is written, which gives the starts.  All of ctl is zero at the start.
 struct BsgsLists {
     u32 *list;
     u32 stride;
     u32 *ctl;
 };
+constexpr u32 LIST_CTL = 4 * NCLASS;        // u32 of ctl per group
+// Set-up scratch of one prime.  Nothing of it is read once the set-up is done, and the
+// prime generator's lists are not read once it begins: they share memory.
+constexpr size_t SETUP_AUX = 32 + 16 * NCLASS;
 
 // Index i of work spread over nr ranges with prefix sums prefix[0..nr]:
 // the range k with prefix[k] <= i < prefix[k+1] (i < prefix[nr]).
@@ -236,7 +243,6 @@ cudaError_t launch_mr2(const u64 *cands, const u32 *ctrs, u32 cand_cap, u64 *pri
 cudaError_t launch_setup(const JobDev *job, u32 kcount, const u64 *primes, u32 first, u32 count, u64 pmax, PrimeHdr *hdr,
                          void *aux, u64 *tabs, u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats,
                          int geom, int sms, cudaStream_t st);
-size_t setup_aux_bytes();
 // every prime of the launch lies in [pmin, pmax), entirely below or entirely at or above 2^63
 cudaError_t launch_bsgs(const BsgsArgs &a, const PrimeHdr *hdr, const u64 *tabs, const u64 *tgt,
                         const unsigned short *meta, const BsgsLists &lists, u64 pmin, u64 pmax, int geom, int sms,
@@ -261,8 +267,8 @@ cudaError_t launch_mr_batch2(const u64 *cands, u32 ccap, u64 *primes, u32 rcap, 
                              const u32 *prefix_c, u64 *mid, u32 *mid_r, u32 mid_cap, u32 *mid_ctr, u32 *err, int sms,
                              cudaStream_t st);
 // set-up of the primes of all ranges (prefix_p: prefix sums of their counts;
-// rec_of: room for one record index per prime, nranges * rcap); group g's lists
-// are lists.list + g*NCLASS*stride with lists.ctl + 2*NCLASS*g, zero at the start
+// rec_of and lists.list: room for one record index per prime, nranges * rcap); group
+// g's part of lists.ctl starts at LIST_CTL*g
 cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const BatchRange *ranges, const u64 *primes,
                                u32 rcap, const u32 *prefix_p, u32 nranges, PrimeHdr *hdr, void *aux, u64 *tabs,
                                u64 *tgt, unsigned short *meta, const BsgsLists &lists, u64 *stats, u32 *rec_of, int sms,

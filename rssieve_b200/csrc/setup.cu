@@ -68,6 +68,7 @@ struct PrimeAux {        // kernel 1 -> kernels 2 and 3; residues in the step ki
     u64 wr0[NCLASS];     // per class, Q'_c = 512 << c: b^(nmin + e(Q'_c - 1))
     u64 S[NCLASS];       //   and s^Q'_c
 };
+static_assert(sizeof(PrimeAux) == SETUP_AUX, "the engine and the batch allocate it");
 
 // ---- arithmetic of the set-up: plain residues in doubles below FP_BOUND, else
 // Montgomery residues ----
@@ -386,6 +387,12 @@ __global__ void __launch_bounds__(128, 8) k_setup_prime(const JobDev *__restrict
     }
 }
 
+// A batch's BSGS group of prime p of a job of geometry gm.
+__device__ __forceinline__ u32 list_group(const JobGeom &gm, u64 p)
+{
+    return gm.group + (p < FP_BOUND ? 2u : (p >> 63) ? 0u : 1u);
+}
+
 // Class for a prime with nk targets of Le giant-step units each: the c among
 // gm.classes that minimises 1.5 Q' + nk*ceil(Le/Q') with Q' = 512 << c, baby
 // steps, the work of the 32 << c threads that does not depend on their steps
@@ -581,9 +588,10 @@ __device__ __forceinline__ void rest_powers(const JobDev *__restrict__ job, u32 
 // of them) of a warp; live: the record exists and is not skipped.  GL = 32: up to
 // 128 sequences, four rounds of lanes (rest: the last, partial round's powers are in
 // the record's target row); GL < 32: at most GL sequences, 32/GL primes side by side
-// in a warp.  Called by the whole warp.
+// in a warp.  Called by the whole warp.  Returns the prime's class, or NCLASS when it
+// is skipped.
 template <bool FP, u32 GL>
-__device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 w, u32 l, bool live,
+__device__ __forceinline__ u32 setup_k_one(const JobDev *__restrict__ job, u32 w, u32 l, bool live,
                                             PrimeHdr *__restrict__ hdr, const PrimeAux *__restrict__ aux,
                                             u64 *tgt, unsigned short *__restrict__ meta,
                                             u64 *__restrict__ stats, const JobGeom &gm, bool rest, KScratch<GL> &sc)
@@ -763,7 +771,7 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
         atomicAdd(&stats[ST_SKIPPED], 1ull);
     }
     __syncwarp();                                          // the compacted parts are written
-    if (!live || skip) return;
+    if (!live || skip) return NCLASS;
     // baby steps for this prime (the giant-step tables follow in kernel 3), and the
     // targets T = -c * k * b^(nmin + off + e(Q'-1))
     const u32 cls = choose_class(gm, nk, (job->L - 1) / e + 1, E);
@@ -776,6 +784,7 @@ __device__ __forceinline__ void setup_k_one(const JobDev *__restrict__ job, u32 
         hdr[w].numk = nk;
         hdr[w].cls = cls;
     }
+    return cls;
 }
 
 // Giant phase of nk targets with Mg giant steps each, over a group of gs
@@ -900,7 +909,8 @@ __device__ __forceinline__ void setup_tabs_one(const JobDev *__restrict__ job, u
 }
 
 // Kernel 3: one thread per prime (indexing as kernel 1); then the record's index
-// goes on the list of its class (ANY_PRIMES: of its job's group and step kind).
+// goes on the list of its class (ANY_PRIMES: of its job's group and step kind, with the
+// lists' starts from kernel 2's counts).
 template <int KIND>
 __global__ void __launch_bounds__(128, 8) k_setup_tabs(const JobDev *__restrict__ jobs, PrimeHdr *__restrict__ hdr,
                                                     const PrimeAux *__restrict__ aux, u32 count,
@@ -916,6 +926,17 @@ __global__ void __launch_bounds__(128, 8) k_setup_tabs(const JobDev *__restrict_
     const u32 total = BATCH ? prefix[nr] : count;
     __shared__ u64 s_tile[128 / 32][32][33];
     u64 (*tile)[33] = s_tile[threadIdx.x >> 5];
+    __shared__ u32 s_first[BATCH ? NGROUP * NCLASS : 1];
+    if constexpr (BATCH) {
+        const u32 k = threadIdx.x;
+        if (k < NGROUP * NCLASS) {
+            u32 first = 0;
+            for (u32 l = 0; l < k; ++l) first += list_ctl[l / NCLASS * LIST_CTL + 2 * NCLASS + l % NCLASS];
+            s_first[k] = first;
+            if (blockIdx.x == 0) list_ctl[k / NCLASS * LIST_CTL + 3 * NCLASS + k % NCLASS] = first;
+        }
+        __syncthreads();
+    }
     u32 nt = 0, nf = 0, ns = 0;
     // i0 is uniform over the warp, so that the list claims below stay whole
     for (u32 i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < total; i0 += stride) {
@@ -931,15 +952,14 @@ __global__ void __launch_bounds__(128, 8) k_setup_tabs(const JobDev *__restrict_
         if (KIND != FP_PRIMES && __any_sync(0xFFFFFFFFu, live && !fp))
             setup_tabs_one<false>(jobs + jb, rec, hdr, aux, tabs, tile, live && !fp, nt, nf, ns);
         if (live) {
-            const u32 g = BATCH ? geoms[jb].group + (p < FP_BOUND ? 2u : (p >> 63) ? 0u : 1u) : 0u;
-            key = g * NCLASS + hdr[rec].cls;
+            key = (BATCH ? list_group(geoms[jb], p) : 0u) * NCLASS + hdr[rec].cls;
         }
         const u32 same = __match_any_sync(0xFFFFFFFFu, key);
         const u32 lead = __ffs((int)same) - 1;
         u32 base = 0;
-        if (live && lane == lead) base = atomicAdd(&list_ctl[(key / NCLASS) * 2 * NCLASS + key % NCLASS], __popc(same));
+        if (live && lane == lead) base = atomicAdd(&list_ctl[key / NCLASS * LIST_CTL + key % NCLASS], __popc(same));
         base = __shfl_sync(0xFFFFFFFFu, base, lead);
-        if (live) lists[(size_t)key * list_stride + base + __popc(same & ((1u << lane) - 1))] = rec;
+        if (live) lists[(BATCH ? s_first[key] : key * list_stride) + base + __popc(same & ((1u << lane) - 1))] = rec;
     }
     // one atomic per warp and counter
     nt = __reduce_add_sync(0xFFFFFFFFu, nt);
@@ -963,7 +983,7 @@ __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restri
                                                        u64 *__restrict__ stats, JobGeom gm,
                                                        const JobGeom *__restrict__ geoms,
                                                        const u32 *__restrict__ prefix, u32 nr,
-                                                       const u32 *__restrict__ rec_of)
+                                                       const u32 *__restrict__ rec_of, u32 *list_ctl)
 {
     __shared__ KScratch<GL> s_sc[SETUP_TPB / GL];
     const u32 l = threadIdx.x & (GL - 1);
@@ -1004,8 +1024,10 @@ __global__ void __launch_bounds__(SETUP_TPB, 4) k_setup_k(const JobDev *__restri
                     if (l == 0) atomicAdd(&stats[ST_SKIPPED], 1ull);
                     continue;
                 }
-                setup_k_one<KIND == FP_PRIMES, GL>(jobs + j, w, l, true, hdr, aux, tgt, meta, stats, BATCH ? geoms[j] : gm,
-                                                   rest, sc);
+                const u32 cls = setup_k_one<KIND == FP_PRIMES, GL>(jobs + j, w, l, true, hdr, aux, tgt, meta, stats,
+                                                                   BATCH ? geoms[j] : gm, rest, sc);
+                if (BATCH && l == 0 && cls < NCLASS)       // the length of the list that kernel 3 puts it on
+                    atomicAdd(&list_ctl[list_group(geoms[j], hdr[w].p) * LIST_CTL + 2 * NCLASS + cls], 1u);
             }
         }
     } else {
@@ -1036,7 +1058,7 @@ static cudaError_t launch_setup_kind(const JobDev *job, u32 kcount, const u64 *p
         const bool four = GL == 32 && shares_rest(kcount) && count >= 4u * 4 * 8 * (u32)sms;
         const u32 ppb = SETUP_TPB / GL * (four ? 4 : 1);   // primes per block
         k_setup_k<KIND, GL><<<(count + ppb - 1) / ppb, SETUP_TPB, 0, st>>>(job, hdr, aux, count, four, tgt, meta, stats,
-                                                                          gm, nullptr, nullptr, 0, nullptr);
+                                                                          gm, nullptr, nullptr, 0, nullptr, nullptr);
     };
     if (kcount <= 4) go(std::integral_constant<u32, 4>{});
     else if (kcount <= 8) go(std::integral_constant<u32, 8>{});
@@ -1077,16 +1099,14 @@ cudaError_t launch_setup_batch(const JobDev *jobs, const JobGeom *geoms, const B
     // FP_PRIMES first: it also takes the records without a search from kernel 1 (p = 0 is
     // below FP_BOUND), and the records that the other launch drops must not be among them
     k_setup_k<FP_PRIMES, 32, true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, true, tgt, meta,
-                                                                  stats, gm, geoms, prefix_p, nranges, rec_of);
+                                                                  stats, gm, geoms, prefix_p, nranges, rec_of, lists.ctl);
     k_setup_k<INT_PRIMES, 32, true><<<sms * 4, SETUP_TPB, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, true, tgt, meta,
-                                                                   stats, gm, geoms, prefix_p, nranges, rec_of);
+                                                                   stats, gm, geoms, prefix_p, nranges, rec_of, lists.ctl);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_setup_tabs<ANY_PRIMES><<<sms * 8, 128, 0, st>>>(jobs, hdr, (const PrimeAux *)aux, 0, tabs, stats, lists.list,
                                                       lists.stride, lists.ctl, geoms, prefix_p, nranges, rec_of);
     return cudaGetLastError();
 }
-
-size_t setup_aux_bytes() { return sizeof(PrimeAux); }
 
 }  // namespace rs

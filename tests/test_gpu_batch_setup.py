@@ -100,3 +100,17 @@ def test_primes_per_warp(rs, sieve, kcounts, p0, widths):
     for w in widths:
         w = w // len(kcounts)
         _check_counters(rs, sieve, [(_small_job(3, k), p0 + i * w, p0 + (i + 1) * w) for i, k in enumerate(kcounts)])
+
+
+def test_memory_of_a_range_slot(rs):
+    """A range slot holds 2^16 primes' records and scratch: 2420 bytes each or less, so
+    that a batch of 1150 slots fits 180 GB."""
+    import torch
+    free = []
+    for slots in (4, 36):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        with closing(rs.Batch(0, max_jobs=2, range_slots=slots)):
+            free.append(before - torch.cuda.mem_get_info()[0])
+    # (2 MB granules: one or two per buffer, whatever the number of slots)
+    assert (free[1] - free[0]) / 32 <= 2420 * 65536 + (1 << 20)
