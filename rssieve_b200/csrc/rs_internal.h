@@ -121,9 +121,14 @@ struct JobDev {
 // A larger split modulus e means fewer giant steps and a longer class table per
 // prime.  With a warp per prime (more than 16 sequences) 256 always pays: 100
 // sequences over 6*10^6, 26.0 -> 21.8 ns per prime against 64; 68 over 10^5, 8.5
-// -> 8.4.  With a few lanes per prime the table weighs more: one sequence over
-// 10^7, 4.24 -> 4.07; 8 over 2*10^5, 3.74 -> 3.92, so small searches keep 64.
-constexpr u32 split_limit(u32 kcount, u32 L) { return kcount > 16 || (u64)kcount * L > 4000000 ? 256u : 64u; }
+// -> 8.4.  With 4 to 16 lanes per prime the table weighs more, and small searches keep
+// 64: in sequences * n-range both take the same time at 6*10^6 for one sequence, 8*10^6
+// for 4, 10^7 for 8 and 1.4*10^7 for 16 (p of 2^40 to 2^63; within 2% for all step
+// kinds), at 2*10^6 64 is ahead by 3 to 8%, at 2*10^7 256 by 2 to 7%.
+constexpr u32 split_limit(u32 kcount, u32 L)
+{
+    return kcount > 16 || (u64)kcount * L > 6000000 + 500000 * kcount ? 256u : 64u;
+}
 
 // Below FP_BOUND = 2^51 the BSGS steps run on the FP64 pipe (fp_mulfix in
 // mont.cuh): residues are exact integers in doubles, and a product by a fixed

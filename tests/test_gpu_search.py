@@ -108,3 +108,13 @@ def test_n_range_of_32_bits(sieve, oracle, nmin, p0):
 @pytest.mark.parametrize("p0", [(1 << 49) + 5, (1 << 59) + 5])
 def test_sequence_counts(sieve, oracle, kcount, p0):
     _planted(sieve, oracle, 3 if kcount % 2 else 10, kcount, 5_001, 25_000, p0, p0 + 1_100_000, kcount)
+
+
+# The split modulus goes up to 256 from sequences * n-range of 6.5*10^6 (one sequence),
+# 8*10^6 (4), 10^7 (8) and 1.4*10^7 (16) on: n-ranges at the line and one past it.
+@pytest.mark.parametrize("kcount", [1, 4, 8, 16])
+@pytest.mark.parametrize("past", [0, 1])
+def test_split_limit_of_few_sequences(sieve, oracle, kcount, past):
+    width = (6_000_000 + 500_000 * kcount) // kcount + past
+    for p0 in ((1 << 44) + 1, (1 << 56) + 1):
+        _planted(sieve, oracle, 2, kcount, 1_001, 1_000 + width, p0, p0 + 20_000, 31 + kcount)
