@@ -394,8 +394,6 @@ static int batch_add_job(rs_batch *b, const rs_seqs *s, const BJob *src, uint64_
         R.p_end = hi;
         R.job = jid;
         R.active = 1;
-        R.mode = (hi <= FP_BOUND) ? 2 : (hi <= TOP) ? 1 : 0;
-        R.geom = (u8)J.geom;
         b->h_ranges[r] = R;
         b->range_used[r] = 1;
         b->range_done[r] = 0;

@@ -71,8 +71,6 @@ __device__ __forceinline__ u32 filter_mask(u32 h)
     return (1u << (h & 31)) | (1u << ((h >> 5) & 31)) | (1u << ((h >> 10) & 31));
 }
 
-// y -> y*s: doubling/quadrupling for b = 2 (the common case), additions for
-// b^e <= 16, a Montgomery product otherwise (smul is uniform per prime)
 // 2x mod p for p < 2^63 (2x cannot wrap): one compare, one predicated subtract
 __device__ __forceinline__ u64 dbl63(u64 x, u64 p)
 {

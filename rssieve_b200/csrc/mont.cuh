@@ -160,7 +160,6 @@ RS_DEV u64 madd(u64 a, u64 b, u64 p)
 }
 
 RS_DEV u64 msub(u64 a, u64 b, u64 p) { return (a >= b) ? a - b : a - b + p; }
-RS_DEV u64 mneg(u64 a, u64 p) { return a ? p - a : 0; }
 
 // p^-1 mod 2^64 by Newton iteration: p*p == 1 mod 8 gives 3 correct bits,
 // each step doubles them (3, 6, 12, 24, 48, 96).
@@ -220,26 +219,6 @@ RS_DEV u64 mpow(u64 x, u64 e, const Mont &M)
         if ((e >> bit) & 1) a = mmul(a, x, M.p, M.q);
     }
     return a;
-}
-
-// x * b mod p for a small integer multiplier b in [1, 16] by doubling and
-// adding (no multiply); the reference does the same for b = 2, 3, 5
-// (common.cl:74-85).  Larger b use mmul with the Montgomery form of b.
-RS_DEV u64 mul_small(u64 x, u32 b, u64 p)
-{
-    u64 acc = x;
-    int top = 31 - __clz(b);
-    for (int i = top - 1; i >= 0; --i) {
-        acc = madd(acc, acc, p);
-        if ((b >> i) & 1) acc = madd(acc, x, p);
-    }
-    return acc;
-}
-
-// Multiplication by the base: mul_small when b <= 16, else Montgomery.
-RS_DEV u64 mul_base(u64 x, u32 b, u64 bm, const Mont &M)
-{
-    return (b <= 16) ? mul_small(x, b, M.p) : mmul(x, bm, M.p, M.q);
 }
 
 // Jacobi symbol (a/n) for odd n > 0 and 0 <= a < n: binary algorithm

@@ -132,9 +132,9 @@ constexpr u32 split_limit(u32 kcount, u32 L)
 
 // Below FP_BOUND = 2^51 the BSGS steps run on the FP64 pipe (fp_mulfix in
 // mont.cuh): residues are exact integers in doubles, and a product by a fixed
-// multiplier w takes its quotient from the double w/p.
+// multiplier w takes its quotient from the double w/p.  The set-up's residues and
+// products are of the same kind.
 constexpr u64 FP_BOUND = 1ull << 51;
-// The set-up runs on the FP64 pipe below FP_BOUND as well.
 
 // A prime's record header.  Residues are held by step kind: below FP_BOUND each is
 // a plain one, as the bits of the double that holds it; from there on residues are
@@ -151,7 +151,7 @@ struct PrimeHdr {        // 128 bytes (a 16-byte multiple: copied by TMA bulk co
     u32 numk;            // surviving targets
     u32 e;               // split modulus, 1..256
     u32 G, Lc;           // giant phase: G chunks of Lc giant steps per target
-    u32 smul;            // b^e as an integer when it is at most 16, else 0 (2 and 4: baby steps by doublings)
+    u32 smul;            // 2 or 4 when b^e is (baby steps by doublings), else 0
     u32 job;             // job index within a batch (0 for a single job)
     u32 Mg;              // giant steps per target: ceil(ceil(L/e)/Q')
     u32 cls;             // class: Q' = 512 << cls, 32 << cls threads
@@ -189,9 +189,7 @@ struct BatchRange {      // device state of one range slot
     u64 p_cur, p_end;    // next window start, end of the range
     u32 job;             // job slot it belongs to
     u8 active;           // slot in use
-    u8 mode;             // BSGS step kind: 2 p_end <= 2^51 (FP64), 1 p_end <= 2^63 (Shoup), 0 p >= 2^63
-    u8 geom;             // BSGS geometry index of its job
-    u8 pad_;
+    u8 pad_[3];
 };
 // per-range counters of a round: [0] sieve survivors, [1] primes, [2] pad, [3] pad
 constexpr int BR_CTRS = 4;

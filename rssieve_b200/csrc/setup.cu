@@ -119,10 +119,9 @@ struct Field<false> {
     template <bool LAZY> __device__ __forceinline__ V pend(V a) const { return LAZY ? mred(a, M.p) : a; }
 };
 
-// x^e, every lane its own e (0 or more): two bits of e at a time, the digit's
+// x^e, every lane its own e (1 or more): two bits of e at a time, the digit's
 // power (1, x, x^2, x^3) chosen by selects, so lanes do not diverge on their
-// bits: 1.5 products per bit.  Out of line: one copy keeps the kernels small
-// enough for the instruction cache.
+// bits: 1.5 products per bit.
 template <bool FP, bool LAZY>
 __device__ __forceinline__ typename Field<FP>::V power_as(const Field<FP> &F, typename Field<FP>::V x, u64 e)
 {
@@ -141,6 +140,8 @@ __device__ __forceinline__ typename Field<FP>::V power_as(const Field<FP> &F, ty
     }
     return F.template pend<LAZY>(a);
 }
+// The same for e of 0 or more.  Out of line: one copy keeps the kernels small enough
+// for the instruction cache.
 template <bool FP>
 __device__ __noinline__ typename Field<FP>::V power(const Field<FP> F, typename Field<FP>::V x, u64 e)
 {
@@ -248,15 +249,11 @@ __device__ __forceinline__ u32 split_modulus(u64 eo, u32 most)
     }
 }
 
-// b^e as an integer when it is at most 16 (baby steps by additions), else 0.
-__device__ __forceinline__ u32 small_power(u32 b, u32 e)
+// b^e when it is 2 or 4 (baby steps by doublings), else 0.
+__device__ __forceinline__ u32 doubling_power(u32 b, u32 e)
 {
-    u64 v = 1;
-    for (u32 i = 0; i < e; ++i) {
-        v *= b;
-        if (v > 16) return 0;
-    }
-    return (u32)v;
+    if (e == 1) return b == 2 || b == 4 ? b : 0;
+    return e == 2 && b == 2 ? 4 : 0;
 }
 
 // Per-prime constants of prime p into record t, with the powers that depend on
@@ -341,7 +338,7 @@ __device__ __forceinline__ void setup_prime_one(const JobDev *__restrict__ job, 
         }
     }
     H.numk = 0; H.e = e; H.G = 0; H.Lc = 0; H.job = jb; H.Mg = 0; H.cls = 0;
-    H.smul = small_power(b, e);
+    H.smul = doubling_power(b, e);
     H.rk = 0; H.nseg = 0; H.rounds = 0; H.piece = 0;
     hdr[t] = H;
     aux[t] = X;
@@ -511,8 +508,8 @@ __device__ __forceinline__ void power_chains_as(const Field<FP> &F, typename Fie
     for (int r = 0; r < R; ++r) a[r] = F.template pend<LAZY>(a[r]);
 }
 // (Two chains per lane: four would not fit 64 registers.  Issue and the FP64 pipe
-// bound the FP64 form: 100 sequences near 2^50 take 5.2 ns per prime at 73% issue,
-// FP64 58% busy; 7.8 with an exponentiation per sequence to D alone, a second one
+// bound the FP64 form: 100 sequences near 2^50, a launch of 30000 primes, take 5.1 ns
+// per prime at 71% issue, FP64 62% busy (4.7 in launches of 120000); 7.8 with an exponentiation per sequence to D alone, a second one
 // for the rest of the order, and Montgomery conversions around both.)
 template <bool FP, int R, bool UNIFORM>
 __device__ __forceinline__ void power_chains(const Field<FP> &F, typename Field<FP>::V (&a)[2],
@@ -523,10 +520,10 @@ __device__ __forceinline__ void power_chains(const Field<FP> &F, typename Field<
 }
 
 // Shared memory of a sub-warp of GL lanes in kernel 2: the values h^(-r), r <
-// min(e, TAB) (all of them for GL = 32; the others look a class up in several
-// turns, which with 64 entries cost GL = 32 a third of the kernel), the class lookup over them (open addressing, r + 1 in a 16-bit
-// slot, 0: empty), powers of b, and the targets' parts until the baby-step count
-// is known.
+// min(e, TAB) (all of them for GL = 32; the others look a class up in several turns,
+// which with 64 entries cost GL = 32 a third of the kernel), the class lookup over
+// them (open addressing, r + 1 in a 16-bit slot, 0: empty), powers of b, and the
+// targets' parts until the baby-step count is known.
 template <u32 GL>
 struct KScratch {
     static constexpr u32 KM = GL == 32 ? 128 : GL;       // sequences

@@ -4,7 +4,7 @@
 // (kernels/getsegprimes.cl:128-182, kernels/addsmallprimes.cl:8-27, driven by
 // cl_sieve.cpp:1303-1320).  The reference emits base-2 strong probable primes
 // after removing multiples of 2..113; here each CTA runs a segmented
-// Eratosthenes sieve over 2^17 odd numbers in shared memory with every odd
+// Eratosthenes sieve over 2^13 to 2^17 odd numbers in shared memory with every odd
 // prime below 2^16, compacts the survivors with warp ballots/popc, and a
 // second kernel proves the survivors at or above 65537^2 prime with the
 // Baillie-PSW test (a base-2 strong probable-prime test, then a strong Lucas
@@ -360,17 +360,6 @@ __device__ __forceinline__ bool base2_test(u64 n)
     return (n < FP_BOUND) ? sprp2_fp(n, (n - 1) >> t, t) : sprp2(n, mont_init(n), (n - 1) >> t, t);
 }
 
-// Deterministic primality of a sieve survivor below 2^64 (Baillie-PSW): a
-// strong probable prime to base 2 that also passes the strong Lucas test with
-// Selfridge's parameters.  No composite below 2^64 passes both: J. Feitsma and
-// W. Galway enumerated every base-2 Fermat pseudoprime below 2^64 (published
-// 2009-2010, about 118.9 million numbers), and J. Gilchrist checked that none of
-// them is a strong Lucas probable prime with these parameters, i.e. there is no
-// Baillie-PSW pseudoprime below 2^64 (reported 2009, on Feitsma's list; it is
-// the verification that makes BPSW a deterministic test in that range).  About
-// 3.5 Miller-Rabin rounds of work per prime instead of the seven bases of
-// is_prime_mr, which remains the answer when no Lucas parameter is found.
-
 // Appends v of the lanes with keep set to list[*ctr ...] with one atomic per
 // warp (ballot compaction); flags err and drops the warp's values when the
 // list is full.  All 32 lanes call it.
@@ -390,6 +379,17 @@ __device__ __forceinline__ void warp_push(bool keep, u64 v, u64 *__restrict__ li
     if (keep) list[basepos + __popc(mask & ((1u << lane) - 1))] = v;
 }
 
+// Deterministic primality of a sieve survivor below 2^64 (Baillie-PSW): a
+// strong probable prime to base 2 that also passes the strong Lucas test with
+// Selfridge's parameters.  No composite below 2^64 passes both: J. Feitsma and
+// W. Galway enumerated every base-2 Fermat pseudoprime below 2^64 (published
+// 2009-2010, about 118.9 million numbers), and J. Gilchrist checked that none of
+// them is a strong Lucas probable prime with these parameters, i.e. there is no
+// Baillie-PSW pseudoprime below 2^64 (reported 2009, on Feitsma's list; it is
+// the verification that makes BPSW a deterministic test in that range).  About
+// 3.5 Miller-Rabin rounds of work per prime instead of the seven bases of
+// is_prime_mr, which remains the answer when no Lucas parameter is found.
+//
 // The test runs in two passes, so that the Lucas ladder runs on full warps.
 // About 57% of the survivors of a sieve by the primes below 2^16 are prime at
 // p near 2^50 (Mertens: 1/ln p over e^-gamma/ln 2^16), and the base-2 test
