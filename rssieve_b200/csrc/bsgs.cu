@@ -39,13 +39,13 @@
 // 14 to 16 cycles of an SM quarter on each of these resources, and its 22 issue
 // slots come first: mixed streams of instructions that each hold their pipe for
 // two cycles issue one in 1.5 cycles at best (measured), and the kernel issues in
-// 65% of all cycles.  100 sequences, n-range 6*10^6, p near 2^50: 13.9 ns per
+// 65% of all cycles.  100 sequences, n-range 6*10^6, p near 2^50: 13.7 ns per
 // prime for 9200 steps (28.1 for 12100 with an exact table of 16-byte buckets of
 // fingerprints, whose probes and three-store inserts took 5600 shared-memory
 // cycles per prime against 2200 now, and with one group size for all primes of a
-// job); p near 2^58, 61 sequences: 16.1 (26.8); 68 sequences over an n-range of
-// 10^5: 2.2 (4.0).  One test for two steps of both chains (the least of the four
-// probes' missing bits) instead of one each took 14.1 to 13.9 and 17.0 to 16.1 of
+// job); p near 2^58, 61 sequences: 15.8 (26.8); 68 sequences over an n-range of
+// 10^5: 2.1 (4.0).  One test for two steps of both chains (the least of the four
+// probes' missing bits) instead of one each took 14.1 to 13.9 and 17.0 to 16.1 (then) of
 // these.  Three bits per value and three words per value: with two bits a pass
 // comes four times as often and costs more than the third bit's two
 // instructions; the filter fills what two CTAs of 512 threads have of shared
